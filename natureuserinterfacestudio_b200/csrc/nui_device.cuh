@@ -15,6 +15,10 @@ constexpr int kMaxRadius = 7;
 constexpr int kIcpTerms = 29;  // 21 JtJ + 6 Jtr + r^2 + count  (icp.cl:122-160)
 constexpr int kTile = 16;      // pixel tile of the depth bound used by integration culling
 constexpr int kPreBlockX = 32, kPreBlockY = 8;  // k_preprocess block: 32 x 16 pixels, two a thread
+// Shared memory a warp stages its rows in: two arrays of 32 x 4 floats, the second 16 banks
+// on, so that the 32 lanes reading the eight components of four rows hit 32 banks.
+constexpr int kIcpHalf = 144;                       // floats from the first array to the second
+constexpr int kIcpStageBytes = (kIcpHalf + 128) * 4;  // per warp (also holds its 64 sums)
 constexpr int kFastWarps = 4;  // warps per block of the tolerance-mode integration
 constexpr int kFastWarpSmem = 64 * 32 * 4 + 64 * 32 * 4;  // its shared memory per warp (bytes)
 
@@ -62,6 +66,28 @@ struct TrackState {
   // tolerance-mode integration: tiles listed by the cull; blocks of the integration done
   // (both zero between integrations)
   unsigned int fast_count, fast_done;
+};
+
+// The tracker state the host step reads and writes: kept in block 0's shared memory for
+// the whole ICP kernel (so that the single thread's step makes no global-memory round
+// trips), copied in at the start and back at the end.
+struct IcpLm {
+  float R[9], t[3], Rg[9], tg[3];
+  double good[27];
+  float lambda, err_old, error, count;
+  int level_done, status, iterations_run;
+  unsigned icp_iters[kMaxLevels];
+};
+
+// Level 0 of one session spread over many blocks (k_icp_finest): the blocks' sums (depth in
+// 0..28, photometric in 32..60), the tracker state from iteration to iteration, and the
+// blocks that have finished the current one (zero between launches).
+constexpr int kIcpWideBlocks = 320;  // blocks a session, at most
+constexpr int kIcpWideSessions = 4;  // sessions a launch, at most
+struct IcpFinest {
+  double part[kIcpWideBlocks][64];
+  IcpLm lm;
+  unsigned done;
 };
 
 // What one session does in the current tick (host-written, read by every kernel).

@@ -5,10 +5,10 @@
 // transform it by the running estimate, project into the previous camera with
 // full-resolution intrinsics, bilinearly sample the world reference normal and vertex
 // (icp.cl:192-220; a tap NaN -> no match), and if |q - p| < distThres form the row
-// [n x p, n | n.(q - p)].  Each thread accumulates the 29 products of its pixels in FP64
-// (exact products of the FP32 row values, fused multiply-adds);
-// blocks reduce them with warp shuffles and shared memory; the cluster's first block adds
-// the blocks' sums (distributed shared memory, fixed order) and runs the host step of
+// [n x p, n | n.(q - p)].  A warp adds the outer products of its pixels' rows in FP64 on the
+// tensor path (exact products of the FP32 row values); blocks add their warps' sums, the
+// cluster's first block the blocks' (distributed shared memory, fixed order), and it runs the
+// host step of
 // NuiKinfuOpenCLDepthTracker::IterativeClosestPoint (NuiKinfuOpenCLDepthTracker.cpp:324-496):
 // Levenberg-Marquardt accept/reject, FP64 determinant check and Cholesky solve, ZYX Euler
 // increment composed in FP64.  The next iteration reads the updated estimate.
@@ -18,18 +18,17 @@
 
 namespace nui {
 
-constexpr int kIcpThreads = 256;  // pixels per thread: the template parameter PPT (tuned)
-
-// Bilinear sample with holes; taps whose linear index falls past the map read as holes.
+// Bilinear sample with holes; taps whose linear index falls past the map read as holes (the
+// last tap has the largest index).  A hole is NaN in a component and makes that component of
+// the sample NaN whatever its weight, so the caller tests the sample instead of the taps.
 __device__ __forceinline__ float3 bilinear_holes(const float4* __restrict__ src, float px, float py, int W,
                                                  int N) {
   const int ix = (int)floorf(px), iy = (int)floorf(py);
   const float dx = px - (float)ix, dy = py - (float)iy;
-  const int ia = ix + iy * W, ib = (ix + 1) + iy * W, ic = ix + (iy + 1) * W, id = (ix + 1) + (iy + 1) * W;
-  if (id >= N || ic >= N || ib >= N) return f3(qnan(), qnan(), qnan());
-  const float3 a = xyz(__ldg(src + ia)), b = xyz(__ldg(src + ib)), c = xyz(__ldg(src + ic)),
-               d = xyz(__ldg(src + id));
-  if (isnan3(a) || isnan3(b) || isnan3(c) || isnan3(d)) return f3(qnan(), qnan(), qnan());
+  const int ia = ix + iy * W;
+  if (ia + W + 1 >= N) return f3(qnan(), qnan(), qnan());
+  const float3 a = xyz(__ldg(src + ia)), b = xyz(__ldg(src + ia + 1)), c = xyz(__ldg(src + ia + W)),
+               d = xyz(__ldg(src + ia + W + 1));
   const float ex = 1.0f - dx, ey = 1.0f - dy;
   float3 r;
   r.x = a.x * ex * ey + b.x * dx * ey + c.x * ex * dy + d.x * dx * dy;
@@ -38,6 +37,16 @@ __device__ __forceinline__ float3 bilinear_holes(const float4* __restrict__ src,
   return r;
 }
 
+// a / b rounded to nearest, given r = 1 / b rounded to nearest (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): a
+// quotient within one ulp plus its exactly computed remainder times r rounds correctly.  The
+// first remainder step brings a r within one ulp, the second rounds.  Exact while nothing
+// under- or overflows: b in 2^-40 .. 2^40, a zero or in 2^-80 .. 2^80 in magnitude.
+__device__ __forceinline__ float div_shared(float a, float b, float r) {
+  float q = a * r;
+  q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
 // ---------------------------------------------------------------- photometric rows
 // One model point of the colour tracker's term (color_icp_block_kernel, colorIcp.cl:
 // 119-178, in the tracker's convention), at the finest level: the world point m of the
@@ -47,9 +56,25 @@ __device__ __forceinline__ float3 bilinear_holes(const float4* __restrict__ src,
 // image; the residual is the colour difference (units of 1/255) and its derivative in
 // each ICP parameter x_k is  grad(I) . d(proj)/dp . dp/dx_k  with dp/dx_k = R^T (e_k x m)
 // for the rotations and -R^T e_k for the translations (the depth ICP's update
-// R <- Rinc^-1 R, t <- Rinc^-1 t + tinc).  Colours count with alpha 255.  c receives the
-// upper triangle of [D | -diff]^T [D | -diff] by rows (21 + 6), |diff|^2 and 1.
-__device__ __forceinline__ bool color_row(const SessionDesc& s, int i, const float* R, const float3 t, float* c) {
+// R <- Rinc^-1 R, t <- Rinc^-1 t + tinc).  Colours count with alpha 255.  The point's terms
+// are the upper triangle of [D | -diff]^T [D | -diff] by rows (21 + 6) and |diff|^2.
+struct ColorRow {
+  float3 D[6], nd;  // derivatives per parameter and -diff, a value per colour channel
+  // adds the 28 terms -- the upper triangle of [D | nd] by rows (21 + 6), then |diff|^2 --
+  // and a count to the sums
+  __device__ __forceinline__ void add_to(double (&acc)[29]) const {
+    int q = 0;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+#pragma unroll
+      for (int b = a; b < 6; ++b) acc[q++] += (double)dot3(D[a], D[b]);
+      acc[q++] += (double)dot3(D[a], nd);
+    }
+    acc[27] += (double)dot3(nd, nd);
+    acc[28] += 1.0;
+  }
+};
+__device__ __forceinline__ bool color_row(const SessionDesc& s, int i, const float* R, const float3 t, ColorRow& row) {
   const float3 m = xyz(__ldg(s.vref + i));
   if (isnan3(m)) return false;
   const uchar4 mc = __ldg(s.cprev + i);
@@ -69,31 +94,33 @@ __device__ __forceinline__ bool color_row(const SessionDesc& s, int i, const flo
   const float3 diff = mul3(f3((float)co.x - (float)mc.x, (float)co.y - (float)mc.y, (float)co.z - (float)mc.z), k255);
   const float3 g1 = mul3(f3((float)(signed char)gx.x, (float)(signed char)gx.y, (float)(signed char)gx.z), k255);
   const float3 g2 = mul3(f3((float)(signed char)gy.x, (float)(signed char)gy.y, (float)(signed char)gy.z), k255);
-  float3 D[6];
   const float zz = p.z * p.z;
+  // D[k] = jx g1 + jy g2 with (jx, jy) = f (p.z dp - dp.z p) / zz for
+  // dp = (dot3(c0, w), dot3(c1, w), dot3(c2, w)), w = e_k x m (k < 3) or -e_k, without the
+  // terms of w's zeros
+  auto derive = [&](auto quotient) {
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const float3 w = k == 0 ? f3(0.f, -m.z, m.y)
-                   : k == 1 ? f3(m.z, 0.f, -m.x)
-                   : k == 2 ? f3(-m.y, m.x, 0.f)
-                   : k == 3 ? f3(-1.f, 0.f, 0.f)
-                   : k == 4 ? f3(0.f, -1.f, 0.f)
-                            : f3(0.f, 0.f, -1.f);
-    const float3 dp = f3(dot3(c0, w), dot3(c1, w), dot3(c2, w));
-    const float jx = fx * ((p.z * dp.x - dp.z * p.x) / zz);
-    const float jy = fy * ((p.z * dp.y - dp.z * p.y) / zz);
-    D[k] = f3(jx * g1.x + jy * g2.x, jx * g1.y + jy * g2.y, jx * g1.z + jy * g2.z);
+    for (int k = 0; k < 6; ++k) {
+      const float3 dp = k == 0 ? f3(c0.y * -m.z + c0.z * m.y, c1.y * -m.z + c1.z * m.y, c2.y * -m.z + c2.z * m.y)
+                      : k == 1 ? f3(c0.x * m.z + c0.z * -m.x, c1.x * m.z + c1.z * -m.x, c2.x * m.z + c2.z * -m.x)
+                      : k == 2 ? f3(c0.x * -m.y + c0.y * m.x, c1.x * -m.y + c1.y * m.x, c2.x * -m.y + c2.y * m.x)
+                      : k == 3 ? f3(-c0.x, -c1.x, -c2.x)
+                      : k == 4 ? f3(-c0.y, -c1.y, -c2.y)
+                               : f3(-c0.z, -c1.z, -c2.z);
+      const float jx = fx * quotient(p.z * dp.x - dp.z * p.x), jy = fy * quotient(p.z * dp.y - dp.z * p.y);
+      row.D[k] = f3(jx * g1.x + jy * g2.x, jx * g1.y + jy * g2.y, jx * g1.z + jy * g2.z);
+    }
+  };
+  // the twelve quotients by zz share its reciprocal for points between a micrometre and 10^6 m
+  // away along every axis that counts: the numerators are then far inside div_shared's range
+  const float far = fmaxf(fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(m.x), fabsf(m.y))), fmaxf(fabsf(m.z), p.z));
+  if (zz > 1e-12f && far < 1e6f) {
+    const float rzz = 1.0f / zz;
+    derive([&](float a) { return div_shared(a, zz, rzz); });
+  } else {
+    derive([&](float a) { return a / zz; });
   }
-  const float3 nd = f3(-diff.x, -diff.y, -diff.z);
-  int sh = 0;
-#pragma unroll
-  for (int a = 0; a < 6; ++a) {
-#pragma unroll
-    for (int b = a; b < 6; ++b) c[sh++] = dot3(D[a], D[b]);
-    c[sh++] = dot3(D[a], nd);
-  }
-  c[27] = dot3(diff, diff);
-  c[28] = 1.0f;
+  row.nd = f3(-diff.x, -diff.y, -diff.z);
   return true;
 }
 
@@ -208,31 +235,24 @@ __device__ __forceinline__ void euler_zyx(double sa, double ca, double sb, doubl
     }
 }
 
-// The tracker state the host step reads and writes: kept in block 0's shared memory for
-// the whole ICP kernel (so that the single thread's step makes no global-memory round
-// trips), copied in at the start and back at the end.
-struct IcpLm {
-  float R[9], t[3], Rg[9], tg[3];
-  double good[27];
-  float lambda, err_old, error, count;
-  int level_done, status, iterations_run;
-  unsigned icp_iters[kMaxLevels];
-};
-
-// Copies the fields (d <- s); T, U: TrackState or IcpLm.
+// Copies the fields (d <- s), a field element a thread (called by the block's threads, the
+// first 27 of which copy); T, U: TrackState or IcpLm.
 template <class T, class U>
 __device__ __forceinline__ void lm_copy(T* d, const U* s) {
-  for (int k = 0; k < 9; ++k) d->R[k] = s->R[k], d->Rg[k] = s->Rg[k];
-  for (int k = 0; k < 3; ++k) d->t[k] = s->t[k], d->tg[k] = s->tg[k];
-  for (int k = 0; k < 27; ++k) d->good[k] = s->good[k];
-  d->lambda = s->lambda;
-  d->err_old = s->err_old;
-  d->error = s->error;
-  d->count = s->count;
-  d->level_done = s->level_done;
-  d->status = s->status;
-  d->iterations_run = s->iterations_run;
-  for (int k = 0; k < kMaxLevels; ++k) d->icp_iters[k] = s->icp_iters[k];
+  const int k = threadIdx.x;
+  if (k < 9) d->R[k] = s->R[k], d->Rg[k] = s->Rg[k];
+  if (k < 3) d->t[k] = s->t[k], d->tg[k] = s->tg[k];
+  if (k < 27) d->good[k] = s->good[k];
+  if (k < kMaxLevels) d->icp_iters[k] = s->icp_iters[k];
+  if (k == 0) {
+    d->lambda = s->lambda;
+    d->err_old = s->err_old;
+    d->error = s->error;
+    d->count = s->count;
+    d->level_done = s->level_done;
+    d->status = s->status;
+    d->iterations_run = s->iterations_run;
+  }
 }
 
 // The LM step on the reduced sums (NuiKinfuOpenCLDepthTracker.cpp:324-496), spread over
@@ -241,13 +261,14 @@ __device__ __forceinline__ void lm_copy(T* d, const U* s) {
 // the determinant on two threads of different warps at once, the increments' sines and
 // cosines on three threads, the composition on one.  Every value comes from the same FP64
 // operations in the same order as a one-thread step; only their latencies overlap (one
-// thread took ~8 us per iteration, while the cluster's other blocks waited).  All threads
-// of the block call it.
+// thread took ~8 us per iteration, while the cluster's other blocks waited).  The block's
+// first two warps call it and its barriers are theirs alone (a block has up to 32 warps).
 struct IcpStepScratch {
   double A[6][6], b[6], x[6], det, sc[6];
   float cnt;
   int go, solved;
 };
+__device__ __forceinline__ void icp_step_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
 __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const double* sums, int iter,
                                               unsigned min_count) {
   const int tid = threadIdx.x;
@@ -283,7 +304,7 @@ __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const d
       for (int k = 0; k < 27; ++k) ts->good[k] = sums[k];
     }
   }
-  __syncthreads();
+  icp_step_sync();
   if (!w.go) return;
   if (tid < 27) {  // sum sh = (i, j) of the upper triangle of [J|r] by rows, over the count
     int i = 0, j = tid;
@@ -298,7 +319,7 @@ __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const d
       w.A[j][i] = v;
     }
   }
-  __syncthreads();
+  icp_step_sync();
   // a singular system (|det| < 1e-15 or NaN) or a failed factorisation loses tracking; the
   // determinant's elimination works on a copy
   if (tid == 0) {
@@ -320,7 +341,7 @@ __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const d
       for (int c = 0; c < 6; ++c) A[r][c] = w.A[r][c];
     w.det = det6(A);
   }
-  __syncthreads();
+  icp_step_sync();
   if (tid == 0) {
     if (!w.solved || !(fabs(w.det) >= 1e-15)) {
       ts->status = 3;
@@ -333,7 +354,7 @@ __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const d
       }
     }
   }
-  __syncthreads();
+  icp_step_sync();
   if (!w.go) return;
   if (tid < 3) {  // sin and cos of the increment's angles (alpha, beta, gamma)
     double sn, cs;
@@ -341,7 +362,7 @@ __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const d
     w.sc[2 * tid] = sn;
     w.sc[2 * tid + 1] = cs;
   }
-  __syncthreads();
+  icp_step_sync();
   if (tid == 0) {
     double Ri[9];
     euler_zyx(w.sc[0], w.sc[1], w.sc[2], w.sc[3], w.sc[4], w.sc[5], Ri);
@@ -369,88 +390,186 @@ __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const d
   }
 }
 
-// The 29 sums of the depth rows of one block of pixels (kIcpThreads x PPT consecutive
-// pixels of the level, index `vb`), added to this thread's FP64 accumulators.  sR / tc: the
-// running estimate; sp: the previous camera pose (the reference maps' frame).
-template <int PPT>
-__device__ __forceinline__ void icp_depth_rows(const SessionDesc& s, int level, int vb, const float* sR, float3 tc,
-                                               const DevXform& sp, double (&acc)[kIcpTerms]) {
+// One product of the FP64 tensor path: D (8 x 8) += A (8 x 4) B (4 x 8).  Lane l holds
+// A[l / 4][l % 4], B[l % 4][l / 4] and D[l / 4][2 (l % 4) + {0, 1}], so a lane's value of
+// component l / 4 of row l % 4 serves as both operands of a sum of outer products.
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
+// What a depth pass reads for every pixel: held in registers through the pass (the barriers
+// of the staging would have it loaded again for each pixel).
+struct IcpView {
+  const float4 *nref, *vref;
+  float fx, fy, cx, cy;      // full-resolution intrinsics
+  float fxi, fyi, cxl, cyl;  // the level's, as level_vertex forms them
+  float fW, fH, thr;
+  int W, N;
+  __device__ __forceinline__ IcpView(const SessionDesc& s, int level)
+      : nref(s.nref), vref(s.vref), fx(s.cam.fx), fy(s.cam.fy), cx(s.cam.cx), cy(s.cam.cy),
+        fxi((float)(1 << level) * s.cam.fx_inv), fyi((float)(1 << level) * s.cam.fy_inv),
+        cxl(s.cam.cx / (float)(1 << level)), cyl(s.cam.cy / (float)(1 << level)), fW((float)s.W), fH((float)s.H),
+        thr(s.dist_thr), W(s.W), N(s.W * s.H) {}
+};
+// The running estimate and the previous camera pose (the reference maps' frame), a row and
+// its translation a float4: R | t, and R_inv | t.
+struct IcpPoses {
+  float4 cur[3], prev[3];
+};
+// Fills three rows from a matrix and a translation (a row's column a thread, 12 threads).
+__device__ __forceinline__ void icp_pose_rows(float4* rows, const float* R, const float* t) {
+  const int k = threadIdx.x >> 2, c = threadIdx.x & 3;
+  if (threadIdx.x < 12) reinterpret_cast<float*>(rows)[threadIdx.x] = c < 3 ? R[3 * k + c] : t[k];
+}
+__device__ __forceinline__ float dot_row(float4 r, float3 v) { return dot3(f3(r.x, r.y, r.z), v); }
+
+// The row of one pixel (level pixel (x, y) at depth dep): false without a match, else
+// [n x p, n | n.(q - p), 1].
+__device__ __forceinline__ bool icp_depth_row(const IcpView& c, int x, int y, float dep, const IcpPoses& P,
+                                              float4& ra, float4& rb) {
+  if (isnan(dep)) return false;
+  const float3 v = f3(dep * (((float)x - c.cxl) * c.fxi), dep * (((float)y - c.cyl) * c.fyi), dep);  // level_vertex
+  const float4 r0 = P.cur[0], r1 = P.cur[1], r2 = P.cur[2];
+  const float3 pv = f3(dot_row(r0, v) + r0.w, dot_row(r1, v) + r1.w, dot_row(r2, v) + r2.w);
+  const float4 q0 = P.prev[0], q1 = P.prev[1], q2 = P.prev[2];
+  const float3 pd = f3(pv.x - q0.w, pv.y - q1.w, pv.z - q2.w);
+  const float3 pp = f3(dot_row(q0, pd), dot_row(q1, pd), dot_row(q2, pd));
+  const float u = pp.x * c.fx / pp.z + c.cx;
+  const float vv = pp.y * c.fy / pp.z + c.cy;
+  if (!(u >= 0.0f && u < c.fW && vv >= 0.0f && vv < c.fH)) return false;
+  // both maps sampled at once (their eight loads in flight together), then tested: a hole
+  // of either makes the distance or the residual NaN
+  const float3 rn = bilinear_holes(c.nref, u, vv, c.W, c.N);
+  const float3 rv = bilinear_holes(c.vref, u, vv, c.W, c.N);
+  const float3 diff = sub3(rv, pv);
+  const float dist = sqrtf(dot3(diff, diff)), res = dot3(rn, diff);
+  if (!(dist < c.thr) || isnan(res)) return false;
+  const float3 r = cross3(rn, pv);
+  ra = make_float4(r.x, r.y, r.z, rn.x);
+  rb = make_float4(rn.y, rn.z, res, 1.0f);
+  return true;
+}
+
+// The depth rows of the level's pixels that fall to this block (runs of blockDim.x x per
+// pixels: runs rank, rank + C, ...), their outer products added to the warp's 8 x 8 FP64
+// sums (d0, d1: this lane's two of them).  The 29 sums of a pixel are the upper triangle of
+// the outer product of [row, 1]: JtJ, Jtr, r^2 and the count.  The rows' FP32 values are
+// widened, so every product is exact and only the sums round.
+//
+// The pass waits on its eight map gathers.  The sums of a warp take two doubles a lane instead
+// of 29 a thread (58 registers), which lets 1024 threads of 64 registers share an SM instead of
+// 512 of 128, so twice the warps wait at once (track at 640 x 480: 337 -> 281 us; 39 sessions:
+// 164 -> 147 M warp instructions a launch).
+__device__ __forceinline__ void icp_depth_pass(const SessionDesc& s, int level, int per, int rank, int C,
+                                               const IcpPoses& P, float* stage, double& d0, double& d1) {
+  const IcpView view(s, level);
   const int w = s.W >> level, n = w * (s.H >> level);
   const float* __restrict__ Dl = s.dlev[level];
-  const float fx = s.cam.fx, fy = s.cam.fy, cx = s.cam.cx, cy = s.cam.cy;
-  const int RW = s.W, RN = s.W * s.H;
-  const float fW = (float)s.W, fH = (float)s.H;
-  const float3 tp = f3(sp.t[0], sp.t[1], sp.t[2]);
-  const int base = vb * kIcpThreads * PPT;
-  // the depths of all the thread's pixels in flight at once, consumed from the front
-  float dq[PPT];
+  const int T = (int)blockDim.x, lane = threadIdx.x & 31;
+  const int c = lane >> 2, src = (lane & 3) * 4 + (c < 4 ? c : kIcpHalf + c - 4);
+  float4* const sa = reinterpret_cast<float4*>(stage) + lane;
+  float4* const sb = reinterpret_cast<float4*>(stage + kIcpHalf) + lane;
+  // the next pixel's depth is in flight while the current one's row forms; a pixel's column
+  // and row advance with its index, by T within a run and by the rest of the other blocks'
+  // runs after it
+  const int jump = T * ((C - 1) * per + 1), ty = T / w, tx = T - ty * w, jy = jump / w, jx = jump - jy * w;
+  int base = rank * T * per, k = 0;
+  int i = base + (int)threadIdx.x, y = i / w, x = i - y * w;
+  float dn = i < n ? __ldg(Dl + i) : qnan();
+  while (base < n) {
+    const int cx = x, cy = y;
+    const float dep = dn;
+    const bool step = ++k < per;
+    if (!step) {
+      k = 0;
+      base += C * T * per;
+    }
+    i += step ? T : jump;
+    x += step ? tx : jx;
+    y += step ? ty : jy;
+    if (x >= w) x -= w, ++y;
+    dn = i < n ? __ldg(Dl + i) : qnan();
+    float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb = ra;
+    const bool ok = icp_depth_row(view, cx, cy, dep, P, ra, rb);
+    if (!__any_sync(0xffffffffu, ok)) continue;
+    *sa = ra;
+    *sb = rb;
+    __syncwarp();
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    const int i = base + k * kIcpThreads + threadIdx.x;
-    dq[k] = i < n ? __ldg(Dl + i) : qnan();
-  }
-#pragma unroll 1
-  for (int k = 0; k < PPT; ++k) {
-    const float dep = dq[0];
-#pragma unroll
-    for (int j = 0; j + 1 < PPT; ++j) dq[j] = dq[j + 1];
-    if (isnan(dep)) continue;
-    const int i = base + k * kIcpThreads + threadIdx.x;
-    const int py = i / w;
-    const float3 v = level_vertex(s.cam, level, i - py * w, py, dep);
-    const float3 pv = add3(rot_rows(sR, v), tc);
-    const float3 pp = rot_rows(sp.R_inv, sub3(pv, tp));
-    const float u = pp.x * fx / pp.z + cx;
-    const float vv = pp.y * fy / pp.z + cy;
-    if (!(u >= 0.0f && u < fW && vv >= 0.0f && vv < fH)) continue;
-    // both maps sampled at once (their eight loads in flight together), then tested
-    const float3 rn = bilinear_holes(s.nref, u, vv, RW, RN);
-    const float3 rv = bilinear_holes(s.vref, u, vv, RW, RN);
-    if (isnan3(rn) || isnan3(rv)) continue;
-    const float3 diff = sub3(rv, pv);
-    const float dist = sqrtf(dot3(diff, diff));
-    if (!(dist < s.dist_thr)) continue;
-    const float3 r0 = cross3(rn, pv);
-    // the row's seven FP32 values widened once; each product is exact in FP64 and enters
-    // its sum with one rounding (fused multiply-add)
-    const double c7[7] = {(double)r0.x, (double)r0.y, (double)r0.z, (double)rn.x, (double)rn.y, (double)rn.z,
-                          (double)dot3(rn, diff)};
-    int sh = 0;
-#pragma unroll
-    for (int a = 0; a < 6; ++a)
-#pragma unroll
-      for (int b = a; b < 7; ++b, ++sh) acc[sh] = fma(c7[a], c7[b], acc[sh]);
-    acc[27] = fma(c7[6], c7[6], acc[27]);
-    acc[28] += 1.0;
+    for (int g = 0; g < 8; ++g) {
+      const double x = (double)stage[16 * g + src];
+      dmma(d0, d1, x, x);
+    }
+    __syncwarp();
   }
 }
 
-// The photometric rows of one block of full-resolution model points (colour tracking).
-template <int PPT>
-__device__ __forceinline__ void icp_color_rows(const SessionDesc& s, int vb, const float* sR, float3 tc,
+// The photometric rows of the model points that fall to this block, their 28 FP32 terms and
+// the count added to this thread's FP64 sums.
+__device__ __forceinline__ void icp_color_pass(const SessionDesc& s, int per, int rank, int C, const IcpPoses& P,
                                                double (&acc)[kIcpTerms]) {
-  const int cbase = vb * kIcpThreads * PPT, NM = s.W * s.H;
+  const int NM = s.W * s.H, T = (int)blockDim.x;
+  const float4 r0 = P.cur[0], r1 = P.cur[1], r2 = P.cur[2];
+  const float R[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
+  const float3 tc = f3(r0.w, r1.w, r2.w);
 #pragma unroll 1
-  for (int k = 0; k < PPT; ++k) {
-    const int i = cbase + k * kIcpThreads + threadIdx.x;
-    if (i >= NM) break;
-    float c[kIcpTerms];
-    if (!color_row(s, i, sR, tc, c)) continue;
-#pragma unroll
-    for (int q = 0; q < kIcpTerms - 1; ++q) acc[q] += (double)c[q];
-    acc[28] += 1.0;
-  }
+  for (int base = rank * T * per; base < NM; base += C * T * per)
+#pragma unroll 1
+    for (int k = 0; k < per; ++k) {
+      const int i = base + k * T + (int)threadIdx.x;
+      ColorRow row;
+      if (i >= NM || !color_row(s, i, R, tc, row)) continue;
+      row.add_to(acc);
+    }
 }
 
-// Block sum of the threads' accumulators (a reduce-scatter over the 32 lanes of a warp,
-// terms padded to 32 -- at each of five steps a lane keeps half of its values, sends the
-// other half to its partner and adds what it receives, so lane k ends with the warp's sum
-// of term k after 31 exchanges instead of 29 x 5 -- then the warps in shared memory, in a
-// fixed order).  Threads 0..28 receive term threadIdx.x; all threads must call it.
-__device__ __forceinline__ double icp_block_sum(const double (&acc)[kIcpTerms]) {
-  constexpr int kWarps = kIcpThreads / 32;
-  __shared__ double wsum[kWarps][32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Term t of the 29 among a warp's 64 sums: (i, j) of the upper triangle of [row, 1] by rows,
+// at 8 i + j; then r^2 (6, 6) and the count (7, 7).
+__device__ __forceinline__ int icp_term_at(int t) {
+  if (t >= 27) return t == 27 ? 54 : 63;
+  int i = 0, j = t;
+  while (j >= 7 - i) j -= 7 - i, ++i;
+  return 8 * i + i + j;
+}
+
+// Block sums from the warps' sums, each warp's left in its part of the staging memory: term
+// threadIdx.x (< kIcpTerms) at index `at` of every warp's 64 doubles, added in warp order.
+// All threads must call it.
+__device__ __forceinline__ double icp_warps_sum(const float* stage0, int at) {
+  __syncthreads();
+  double D = 0.0;
+  if (threadIdx.x < kIcpTerms)
+    for (int wi = 0; wi < (int)(blockDim.x >> 5); ++wi)
+      D += reinterpret_cast<const double*>(stage0 + wi * (kIcpStageBytes / 4))[at];
+  __syncthreads();  // the staging memory is used again
+  return D;
+}
+
+// The block's sums of one pass: term threadIdx.x (< kIcpTerms) of the depth rows, and with
+// photo of the photometric rows too.  All threads must call it.
+__device__ __forceinline__ double icp_depth_sums(const SessionDesc& s, int level, int per, int rank, int C,
+                                                 const IcpPoses& P, float* stage0, int at) {
+  float* const stage = stage0 + (threadIdx.x >> 5) * (kIcpStageBytes / 4);  // this warp's
+  double* const wsum = reinterpret_cast<double*>(stage);
+  const int lane = threadIdx.x & 31;
+  double d0 = 0.0, d1 = 0.0;
+  icp_depth_pass(s, level, per, rank, C, P, stage, d0, d1);
+  wsum[2 * lane] = d0;
+  wsum[2 * lane + 1] = d1;
+  return icp_warps_sum(stage0, at);
+}
+// (a warp's sums by a reduce-scatter over its lanes, terms padded to 32: at each of five
+// steps a lane keeps half of its values, sends the other half to its partner and adds what it
+// receives, so lane k ends with the warp's sum of term k after 31 exchanges)
+__device__ __forceinline__ double icp_color_sums(const SessionDesc& s, int per, int rank, int C, const IcpPoses& P,
+                                                 float* stage0) {
+  double acc[kIcpTerms];
+#pragma unroll
+  for (int k = 0; k < kIcpTerms; ++k) acc[k] = 0.0;
+  icp_color_pass(s, per, rank, C, P, acc);
+  const int lane = threadIdx.x & 31;
   double v[32];
 #pragma unroll
   for (int k = 0; k < 32; ++k) v[k] = k < kIcpTerms ? acc[k] : 0.0;
@@ -464,83 +583,66 @@ __device__ __forceinline__ double icp_block_sum(const double (&acc)[kIcpTerms]) 
       v[j] = keep + __shfl_xor_sync(0xffffffffu, send, half);
     }
   }
-  wsum[warp][lane] = v[0];
-  __syncthreads();
-  double D = 0.0;
-  if (threadIdx.x < kIcpTerms)
-    for (int wi = 0; wi < kWarps; ++wi) D += wsum[wi][threadIdx.x];
-  __syncthreads();  // wsum is reused by the next call
-  return D;
+  reinterpret_cast<double*>(stage0 + (threadIdx.x >> 5) * (kIcpStageBytes / 4))[lane] = v[0];
+  return icp_warps_sum(stage0, threadIdx.x);
 }
 
 // All ICP iterations of every level of one frame, one thread-block cluster per session
 // (NuiKinfuOpenCLDepthTracker::IterativeClosestPoint, NuiKinfuOpenCLDepthTracker.cpp:240-504).
-// The C blocks of a cluster (C = 2, 4, 8 or 16, a launch attribute: the ICP tuning's
-// blocks per session) share the level's pixels (pixel blocks b = rank, rank + C, ...);
-// every iteration each block reduces its FP64 sums into its own
-// shared memory, a cluster barrier makes them visible, block 0 adds the blocks' sums in
-// rank order through distributed shared memory and runs the host step (LM accept/reject,
-// FP64 Cholesky, pose update) on one thread, and a second barrier publishes the new
-// estimate, which every block reads from block 0's shared memory.  The hardware schedules
-// a cluster's blocks together and its barriers need no polling; every block takes the same
-// exits at the same points, since each decision comes from block 0's published state.
-// One launch per tick replaces one launch per iteration, and sessions whose levels stop
-// early leave their SMs to the others.
-template <int PPT>
-__global__ void __launch_bounds__(kIcpThreads, 2)
-    k_icp_cluster(const SessionDesc* __restrict__ descs, int fam) {
+// The C blocks of a cluster (C = 2..16, a launch attribute: the ICP tuning's blocks per
+// session) share the level's pixels (runs of blockDim.x x per pixels); every iteration each
+// block reduces its FP64 sums into its own shared memory, a cluster barrier makes them
+// visible, block 0 adds the blocks' sums in rank order through distributed shared memory and
+// runs the host step (LM accept/reject, FP64 Cholesky, pose update), and a second barrier
+// publishes the new estimate, which every block reads from block 0's shared memory.  The
+// hardware schedules a cluster's blocks together and its barriers need no polling; every
+// block takes the same exits at the same points, since each decision comes from block 0's
+// published state.  One launch per tick replaces one launch per iteration, and sessions
+// whose levels stop early leave their SMs to the others.
+//
+// The block size is the launch's (256, 512 or 1024 threads, see launch_track): the same code
+// with kIcpStageBytes of dynamic shared memory a warp.  Launches without a colour-tracked
+// session take the variant without the photometric rows (64 registers, up to 1024 threads);
+// the rows' 29 FP64 sums a thread need 128 (up to 512).
+template <bool COLOR>
+__global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
+    k_icp_cluster(const SessionDesc* __restrict__ descs, int fam, int ppt, int wide) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const SessionDesc& s = descs[blockIdx.y];
   if (s.kind != kTrackFrame || !in_family(s, fam)) return;  // the same for every block of the cluster
   TrackState* ts = s.ts;
   const int rank = (int)cluster.block_rank(), C = (int)cluster.num_blocks();
-  __shared__ float sR[9], st[3];
-  __shared__ DevXform sp;
+  extern __shared__ __align__(16) float icp_stage[];
+  __shared__ IcpPoses P;
   __shared__ double part[2][32];  // this block's depth / photometric sums
-  __shared__ float bR[9], bt[3];  // block 0: the estimate after the host step
-  __shared__ int bflags[2];       // block 0: status, level_done
   __shared__ double sums[kIcpTerms];
   __shared__ IcpLm lm;  // block 0: the tracker state during the kernel
   __shared__ IcpStepScratch hw;  // block 0: the LM step's intermediate values
-  if (threadIdx.x < 9) sR[threadIdx.x] = ts->R[threadIdx.x];
-  if (threadIdx.x < 3) st[threadIdx.x] = ts->t[threadIdx.x];
-  if (threadIdx.x < 21) reinterpret_cast<float*>(&sp)[threadIdx.x] = reinterpret_cast<const float*>(&ts->xf)[threadIdx.x];
+  icp_pose_rows(P.cur, ts->R, ts->t);
+  icp_pose_rows(P.prev, ts->xf.R_inv, ts->xf.t);
   const int status0 = ts->status;
-  if (rank == 0 && threadIdx.x == 0) lm_copy(&lm, ts);
+  if (rank == 0) lm_copy(&lm, ts);
   // every block has read the initial state before block 0 writes any of it
   cluster.sync();
   if (status0 != 0) return;
-  for (int level = s.levels - 1; level >= 0; --level) {
-    const int n = (s.W >> level) * (s.H >> level);
-    // the coarser levels in blocks of one pixel a thread: their few pixel blocks would
-    // otherwise fall unevenly on the cluster's blocks (19 blocks of 1024 pixels for 16 at
-    // 160 x 120), and a pass waits for its slowest block
-    const int per_block = kIcpThreads * (level == 0 ? PPT : 1);
-    const int nblocks = (n + per_block - 1) / per_block;
-    const bool photo = s.photo_w > 0.f && level == 0;
-    const int ncb = photo ? (s.W * s.H + per_block - 1) / per_block : 0;
+  const int at = icp_term_at(threadIdx.x);
+  const int last = wide && (s.photo_w > 0.f || wide == 2) ? 1 : 0;  // k_icp_finest runs level 0 of a colour-tracked session
+  for (int level = s.levels - 1; level >= last; --level) {
+    // runs no longer than leave every block one: a level's few runs would otherwise fall
+    // unevenly on the cluster's blocks (19 runs of 1024 pixels for 16 at 160 x 120), and a
+    // pass waits for its slowest block
+    const int per = max(1, min(ppt, (s.W >> level) * (s.H >> level) / (C * (int)blockDim.x)));
+    const bool photo = COLOR && s.photo_w > 0.f && level == 0;
     for (int iter = 0; iter < s.iters[level]; ++iter) {
-      const float3 tc = f3(st[0], st[1], st[2]);
-      double acc[kIcpTerms];
-#pragma unroll
-      for (int k = 0; k < kIcpTerms; ++k) acc[k] = 0.0;
-      if (level == 0) {
-        for (int vb = rank; vb < nblocks; vb += C) icp_depth_rows<PPT>(s, level, vb, sR, tc, sp, acc);
-      } else {
-        for (int vb = rank; vb < nblocks; vb += C) icp_depth_rows<1>(s, level, vb, sR, tc, sp, acc);
-      }
-      double D = icp_block_sum(acc);
+      double D = icp_depth_sums(s, level, per, rank, C, P, icp_stage, at);
       if (threadIdx.x < kIcpTerms) part[0][threadIdx.x] = D;
       if (photo) {
-#pragma unroll
-        for (int k = 0; k < kIcpTerms; ++k) acc[k] = 0.0;
-        for (int vb = rank; vb < ncb; vb += C) icp_color_rows<PPT>(s, vb, sR, tc, acc);
-        D = icp_block_sum(acc);
+        D = icp_color_sums(s, per, rank, C, P, icp_stage);
         if (threadIdx.x < kIcpTerms) part[1][threadIdx.x] = D;
       }
       cluster.sync();  // every block's sums are visible to block 0
-      if (rank == 0) {
+      if (rank == 0 && threadIdx.x < 64) {
         if (threadIdx.x < kIcpTerms) {
           // the blocks' sums in rank order; the photometric normal equations and residual
           // enter weighted, the count stays the depth count
@@ -553,45 +655,112 @@ __global__ void __launch_bounds__(kIcpThreads, 2)
           if (photo && threadIdx.x < kIcpTerms - 1) a += (double)s.photo_w * c;
           sums[threadIdx.x] = a;
         }
-        __syncthreads();
+        icp_step_sync();
         if (threadIdx.x == 0) lm.icp_iters[level] += 1u;
         icp_host_step(&lm, hw, sums, iter, s.icp_min_count[level]);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          for (int k = 0; k < 9; ++k) bR[k] = lm.R[k];
-          for (int k = 0; k < 3; ++k) bt[k] = lm.t[k];
-          bflags[0] = lm.status;
-          bflags[1] = lm.level_done;
-        }
       }
       cluster.sync();  // block 0's new estimate is visible to every block
-      int flags[2];
-      {
-        const float* r0 = cluster.map_shared_rank(&bR[0], 0);
-        const float* t0 = cluster.map_shared_rank(&bt[0], 0);
-        const int* f0 = cluster.map_shared_rank(&bflags[0], 0);
-        if (threadIdx.x < 9) sR[threadIdx.x] = r0[threadIdx.x];
-        if (threadIdx.x < 3) st[threadIdx.x] = t0[threadIdx.x];
-        flags[0] = f0[0];
-        flags[1] = f0[1];
-      }
+      // (block 0 writes its state again only behind the next iteration's first barrier)
+      const IcpLm* lm0 = cluster.map_shared_rank(&lm, 0);
+      icp_pose_rows(P.cur, lm0->R, lm0->t);
+      const int flags[2] = {lm0->status, lm0->level_done};
       __syncthreads();
       if (flags[0] != 0) {  // tracking lost: every block leaves together
-        if (rank == 0 && threadIdx.x == 0) lm_copy(ts, &lm);
+        if (rank == 0) lm_copy(ts, &lm);
         cluster.sync();     // (block 0's shared memory stays alive until all have read it)
         return;
       }
       if (flags[1]) break;
     }
   }
-  if (rank == 0 && threadIdx.x == 0) lm_copy(ts, &lm);
+  if (rank == 0) lm_copy(ts, &lm);
   cluster.sync();  // no block leaves while another may still read block 0's shared memory
 }
 
-template __global__ void k_icp_cluster<2>(const SessionDesc*, int);
-template __global__ void k_icp_cluster<4>(const SessionDesc*, int);
-template __global__ void k_icp_cluster<8>(const SessionDesc*, int);
-template __global__ void k_icp_cluster<16>(const SessionDesc*, int);
+// One iteration of the finest level of a small batch's sessions, over as many blocks a session
+// as the device holds: a cluster is at most 16 blocks, on which an iteration of a
+// colour-tracked 640 x 480 session took 125 us, of which the LM step is 5 (locate on a voxel
+// hash with colour, ten such iterations: 2.2 ms with the clusters alone, 0.91 ms so).  Each
+// block leaves its sums in the session's part of `work`; the last block to finish (a counter,
+// no block waits for another) adds them in block order and runs the LM step on the state in
+// `work`, which the next iteration's launch reads.  The launches follow one another by
+// programmatic dependence: a launch's blocks come up while the previous one drains and wait
+// for its results.  An iteration after the level's end returns at once.
+template <bool COLOR>
+__global__ void __launch_bounds__(256, COLOR ? 2 : 4)
+    k_icp_finest(const SessionDesc* __restrict__ descs, int fam, int ppt, int iter, int wide,
+                 IcpFinest* __restrict__ work) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  const SessionDesc& s = descs[blockIdx.y];
+  if (s.kind != kTrackFrame || !in_family(s, fam) || !(s.photo_w > 0.f || wide == 2) || iter >= s.iters[0]) return;
+  TrackState* ts = s.ts;
+  IcpFinest& f = work[blockIdx.y];
+  // the first iteration starts from the coarser levels' estimate
+  if (iter == 0 ? ts->status != 0 : (f.lm.status != 0 || f.lm.level_done != 0)) return;
+  extern __shared__ __align__(16) float icp_stage[];
+  __shared__ IcpPoses P;
+  __shared__ double sums[kIcpTerms];
+  __shared__ IcpLm lm;
+  __shared__ IcpStepScratch hw;
+  __shared__ int is_last;
+  icp_pose_rows(P.cur, iter == 0 ? ts->R : f.lm.R, iter == 0 ? ts->t : f.lm.t);
+  icp_pose_rows(P.prev, ts->xf.R_inv, ts->xf.t);
+  __syncthreads();
+  const int B = (int)gridDim.x;
+  const double D = icp_depth_sums(s, 0, ppt, blockIdx.x, B, P, icp_stage, icp_term_at(threadIdx.x));
+  const bool photo = COLOR && s.photo_w > 0.f;
+  const double E = photo ? icp_color_sums(s, ppt, blockIdx.x, B, P, icp_stage) : 0.0;
+  if (threadIdx.x < kIcpTerms) {
+    f.part[blockIdx.x][threadIdx.x] = D;
+    f.part[blockIdx.x][32 + threadIdx.x] = E;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) is_last = atomicAdd(&f.done, 1u) == (unsigned)B - 1u;
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  // the blocks' sums: thread t of a warp adds terms t and 32 + t of an eighth of the blocks,
+  // then the eighths in order
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = (B + 7) / 8;
+  double a = 0.0, c = 0.0;
+#pragma unroll 4
+  for (int b = warp * per; b < min(B, (warp + 1) * per); ++b) {
+    a += __ldcg(&f.part[b][lane]);
+    c += __ldcg(&f.part[b][32 + lane]);
+  }
+  double* const w = reinterpret_cast<double*>(icp_stage);
+  w[64 * warp + lane] = a;
+  w[64 * warp + 32 + lane] = c;
+  if (iter == 0) {
+    lm_copy(&lm, ts);
+  } else {
+    for (int k = threadIdx.x; k < (int)(sizeof(IcpLm) / 4); k += blockDim.x)
+      reinterpret_cast<int*>(&lm)[k] = reinterpret_cast<const int*>(&f.lm)[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < kIcpTerms) {
+    a = c = 0.0;
+    for (int b = 0; b < 8; ++b) a += w[64 * b + threadIdx.x], c += w[64 * b + 32 + threadIdx.x];
+    // the photometric normal equations and residual enter weighted, the count stays the
+    // depth count
+    sums[threadIdx.x] = photo && threadIdx.x < kIcpTerms - 1 ? a + (double)s.photo_w * c : a;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) lm.icp_iters[0] += 1u;
+  if (threadIdx.x < 64) icp_host_step(&lm, hw, sums, iter, s.icp_min_count[0]);
+  __syncthreads();
+  for (int k = threadIdx.x; k < (int)(sizeof(IcpLm) / 4); k += blockDim.x)
+    reinterpret_cast<int*>(&f.lm)[k] = reinterpret_cast<const int*>(&lm)[k];
+  if (threadIdx.x == 0) f.done = 0u;
+  if (lm.status != 0 || lm.level_done || iter + 1 == s.iters[0]) lm_copy(ts, &lm);
+}
+
+template __global__ void k_icp_cluster<false>(const SessionDesc*, int, int, int);
+template __global__ void k_icp_cluster<true>(const SessionDesc*, int, int, int);
+template __global__ void k_icp_finest<false>(const SessionDesc*, int, int, int, int, IcpFinest*);
+template __global__ void k_icp_finest<true>(const SessionDesc*, int, int, int, int, IcpFinest*);
 
 // After the last ICP launch (or on frame 0): publish the pose, decide the integration
 // gate (NuiKinfuTrackingEngine.cpp:115-127) and reset the estimate for the next frame.

@@ -31,8 +31,10 @@ __global__ void k_preprocess(const SessionDesc*);
 __global__ void k_pyramid(const SessionDesc*, int);
 __global__ void k_feedback(const SessionDesc*);
 __global__ void k_vertex_map(const SessionDesc*, int, float4*);
-template <int PPT>
-__global__ void k_icp_cluster(const SessionDesc*, int);
+template <bool COLOR>
+__global__ void k_icp_cluster(const SessionDesc*, int, int, int);
+template <bool COLOR>
+__global__ void k_icp_finest(const SessionDesc*, int, int, int, int, IcpFinest*);
 __global__ void k_track_finalize(const SessionDesc*, int, int);
 __global__ void k_ztab(const SessionDesc*);
 __global__ void k_color_level(const SessionDesc*, int);
@@ -227,6 +229,7 @@ struct nui_ctx {
   // scratch descriptor for kernel-level calls
   SessionDesc* d_kdesc = nullptr;
   TrackState* d_kts = nullptr;
+  IcpFinest* d_finest = nullptr;  // level-0 ICP over the whole device: 2 x kIcpWideSessions (a set a stream)
   unsigned long long* d_count = nullptr;  // counter of the point-cloud fetch
   struct Graph {
     cudaGraphExec_t exec;
@@ -671,23 +674,29 @@ void launch_shift(const BatchPlan& p, const SessionDesc* d, cudaStream_t st) {
   k_shift_dirty<<<dim3(kShiftBlocks, dense_n(p)), 256, 0, st>>>(d);
 }
 
-// The ICP kernel over n sessions, one cluster of cl blocks each (cl = 16 is beyond the
-// portable cluster size and needs the kernel's opt-in, given once per kernel).
-void launch_icp_cluster(void (*kern)(const SessionDesc*, int), const SessionDesc* d, int n, int cl, int fam,
-                        cudaStream_t st) {
-  {
-    static std::mutex mu;
-    static std::vector<const void*> opted;
-    std::lock_guard<std::mutex> lock(mu);
-    if (std::find(opted.begin(), opted.end(), (const void*)kern) == opted.end()) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      opted.push_back((const void*)kern);
-    }
-  }
+// The ICP kernel over n sessions, one cluster of cl blocks each (cl > 8 is beyond the
+// portable cluster size and needs the kernel's opt-in).
+//
+// Block size: the clusters of up to eight sessions may fill their SMs (a block an SM, a cluster
+// a GPC); those of more share them.  Small images keep four pixels or more of the finest level
+// a thread, where a wider block only has more warps to reduce.  The colour variant holds twice
+// the registers, so half the threads.  Measured, one 640 x 480 session (the whole step-wise
+// track): 292 us with 1024 threads, 313 with 512, 381 with 256; 64 sessions (39 dense, 25
+// voxel-hash with colour; six ticks): 47.5 ms with 512 / 256, 49.5 with 512 / 512, 48.0 with
+// 256 / 256.
+void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool color, int fam, int wide, cudaStream_t st) {
+  static std::once_flag opt_in;
+  std::call_once(opt_in, [] {
+    cudaFuncSetAttribute(k_icp_cluster<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(k_icp_cluster<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  });
+  const int cl = p.tune.icp_cluster_blocks;
+  int threads = (n <= 8 ? 1024 : 512) / (color ? 2 : 1);
+  while (threads > 256 && (long)p.maxW * p.maxH < 4L * cl * threads) threads /= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cl, n);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = 0;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = (size_t)(threads / 32) * kIcpStageBytes;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -696,25 +705,52 @@ void launch_icp_cluster(void (*kern)(const SessionDesc*, int), const SessionDesc
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, d, fam);
+  cudaLaunchKernelEx(&cfg, color ? k_icp_cluster<true> : k_icp_cluster<false>, d, fam, p.tune.icp_pixels_per_thread, wide);
+}
+
+// Whether level 0 leaves the clusters for launches over the whole device (k_icp_finest, one an
+// iteration): 1 for the colour-tracked sessions, 2 for all, 0 for none.  A cluster holds at
+// most 16 SMs, but a launch costs ~2 us even when the level has ended, so the images must be
+// large enough; a photometric row costs twice a depth row and its level tends to run all its
+// iterations.  Measured, one session, without and with: locate on a voxel hash with colour at
+// 640 x 480 2.2 -> 0.91 ms, colour track at 352 x 208 628 -> 407 us, depth track at 640 x 480
+// 296 -> 286 us (no gain at 320 x 240).
+int icp_wide(const BatchPlan& p, int n, bool color) {
+  const long px = (long)p.maxW * p.maxH;
+  if (n > kIcpWideSessions) return 0;
+  return px >= 1 << 18 ? 2 : color && px >= 1 << 14 ? 1 : 0;
+}
+
+// One iteration of level 0 of the colour-tracked sessions over the whole device.
+void launch_icp_finest(const BatchPlan& p, const SessionDesc* d, int n, bool color, int fam, int iter, int wide, IcpFinest* work,
+                       cudaStream_t st) {
+  const int per = 4;  // pixels a thread and run: 300 blocks of four an SM at 640 x 480
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min(cdiv((long)p.maxW * p.maxH, 256 * per), (unsigned)kIcpWideBlocks), n);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = 8 * kIcpStageBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = iter > 0 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, color ? k_icp_finest<true> : k_icp_finest<false>, d, fam, per, iter, wide, work);
 }
 
 // Colour pyramid (if any session tracks with colour), the ICP iterations of every level,
 // the integration gate and the published pose, for the sessions of family fam among the n
 // descriptors at d.
 void launch_track(const BatchPlan& p, const SessionDesc* d, int n, cudaStream_t st, float* d_pose, int* d_status,
-                  bool color, int fam = kFamAll, bool tick = true) {
+                  bool color, IcpFinest* work, int fam = kFamAll, bool tick = true) {
   if (n <= 0) return;
   const unsigned npix = cdiv((long)p.maxW * p.maxH, 256);
   if (color) k_color_grad<<<dim3(npix, n, 1), 256, 0, st>>>(d, fam);  // finest level
   // every level and iteration of every session in one launch: a cluster of
   // icp_cluster_blocks blocks per session
-  const int ppt = p.tune.icp_pixels_per_thread;
-  const int cl = p.tune.icp_cluster_blocks;
-  if (ppt == 2) launch_icp_cluster(k_icp_cluster<2>, d, n, cl, fam, st);
-  else if (ppt == 8) launch_icp_cluster(k_icp_cluster<8>, d, n, cl, fam, st);
-  else if (ppt == 16) launch_icp_cluster(k_icp_cluster<16>, d, n, cl, fam, st);
-  else launch_icp_cluster(k_icp_cluster<4>, d, n, cl, fam, st);
+  const int wide = icp_wide(p, n, color);
+  launch_icp_cluster(p, d, n, color, fam, wide, st);
+  for (int i = 0; wide && i < p.maxIters[0]; ++i) launch_icp_finest(p, d, n, color, fam, i, wide, work, st);
   k_track_finalize<<<n, 32, 0, st>>>(d, tick ? 1 : 0, fam);
   k_publish<<<cdiv(n, 64), 64, 0, st>>>(d, n, d_pose, d_status, fam);
   if (color) k_color_keep<<<dim3(cdiv(((long)p.maxW * p.maxH + 3) / 4, 256), n), 256, 0, st>>>(d, fam);
@@ -750,14 +786,15 @@ void enqueue_tick(nui_ctx* ctx, const BatchPlan& p, const SessionDesc* d, float*
     cudaStreamWaitEvent(hs, ctx->fork_ev, 0);
     if (ev) cudaEventRecord(ctx->ev[9], hs);
     if (ranged) {
-      launch_track(p, d + p.denseHead, p.n - p.denseHead, hs, d_pose, d_status, (p.colorIcp & 2) != 0);
-      launch_track(p, d, p.denseHead, st, d_pose, d_status, (p.colorIcp & 1) != 0);
+      launch_track(p, d + p.denseHead, p.n - p.denseHead, hs, d_pose, d_status, (p.colorIcp & 2) != 0,
+                   ctx->d_finest + kIcpWideSessions);
+      launch_track(p, d, p.denseHead, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_finest);
     } else {
-      launch_track(p, d, p.n, hs, d_pose, d_status, (p.colorIcp & 2) != 0, kFamHash);
-      launch_track(p, d, p.n, st, d_pose, d_status, (p.colorIcp & 1) != 0, kFamDense);
+      launch_track(p, d, p.n, hs, d_pose, d_status, (p.colorIcp & 2) != 0, ctx->d_finest + kIcpWideSessions, kFamHash);
+      launch_track(p, d, p.n, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_finest, kFamDense);
     }
   } else {
-    launch_track(p, d, p.n, st, d_pose, d_status, p.colorIcp != 0);
+    launch_track(p, d, p.n, st, d_pose, d_status, p.colorIcp != 0, ctx->d_finest);
   }
   mark(3);
   if (ev) ctx->side_timed = fork;
@@ -822,6 +859,15 @@ nui_status ensure_cap(nui_ctx* ctx, int n) {
   return NUI_OK;
 }
 
+// The workspace of k_icp_finest, once a tick of the context may need it.
+nui_status ensure_finest(nui_ctx* ctx, const BatchPlan& p) {
+  if (ctx->d_finest || !icp_wide(p, std::min(p.n, kIcpWideSessions), p.colorIcp != 0)) return NUI_OK;
+  const size_t bytes = sizeof(IcpFinest) * 2 * kIcpWideSessions;
+  NUI_CUDA(counted_pool_alloc((void**)&ctx->d_finest, bytes, ctx->pool, ctx->stream));
+  NUI_CUDA(cudaMemsetAsync(ctx->d_finest, 0, bytes, ctx->stream));
+  return NUI_OK;
+}
+
 nui_status finish_timing(nui_ctx* ctx) {
   if (!ctx->timing) return NUI_OK;
   NUI_CUDA(cudaEventSynchronize(ctx->ev[6]));
@@ -881,6 +927,7 @@ nui_status tick_launch(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
   }
   if (floor) plan_merge(p, *floor);
   p.tune = ctx->tune;
+  if ((st = ensure_finest(ctx, p)) != NUI_OK) return st;
   NUI_CUDA(cudaMemcpyAsync(ctx->d_descs, hd, sizeof(SessionDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
   if (use_graph && !ctx->timing) {
     auto it = ctx->graphs.find(p);
@@ -1131,6 +1178,7 @@ NUI_API nui_status nui_ctx_destroy(nui_ctx* c) {
   cudaFreeHost(c->h_status);
   cudaFree(c->d_kdesc);
   cudaFree(c->d_kts);
+  if (c->d_finest) cudaFreeAsync(c->d_finest, c->stream);
   cudaFree(c->d_count);
   cudaStreamDestroy(c->own);
   cudaStreamDestroy(c->side);
@@ -1824,7 +1872,9 @@ nui_status run_stage(nui_session* s, int what) {
     for (int l = 1; l < p.maxLevels; ++l)
       k_pyramid<<<dim3(cdiv((long)(p.maxW >> l) * (p.maxH >> l), 256), 1), 256, 0, st>>>(dd, l);
   } else if (what == 1) {
-    launch_track(p, dd, p.n, st, ctx->d_pose, ctx->d_status, p.colorIcp != 0, kFamAll, false);
+    const nui_status fs = ensure_finest(ctx, p);
+    if (fs != NUI_OK) return fs;
+    launch_track(p, dd, p.n, st, ctx->d_pose, ctx->d_status, p.colorIcp != 0, ctx->d_finest, kFamAll, false);
   } else if (what == 2) {
     k_ztab<<<1, 32, 0, st>>>(dd);
     launch_shift(p, dd, st);

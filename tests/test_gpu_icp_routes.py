@@ -1,0 +1,75 @@
+"""The launch routes of the ICP: one session over the whole device (k_icp_finest at level 0),
+clusters with and without the photometric rows, block sizes by image size -- the same poses by
+every route, at the edges of the rules -- and the shared-reciprocal quotients of the
+photometric rows against the division they replace."""
+import random
+from fractions import Fraction
+
+import numpy as np
+import pytest
+
+from natureuserinterfacestudio_b200 import _lib as L
+from oracle import oracle as O
+
+from _util import cfg_for, frames, rot_angle
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,color", [(512, 512, False), (508, 512, False), (516, 508, False), (128, 128, True),
+                                       (124, 128, True), (132, 124, True), (64, 48, False)])
+def test_one_session_and_many_agree(gpu_ctx, W, H, color):
+    """n = 1 (the whole-device route from 2^18 pixels, 2^14 with colour) against the same
+    stream nine times in a batch (clusters only): the routes regroup FP64 sums, so poses agree
+    within the 1e-5 that the ICP shapes are held to; depth poses agree with the oracle's."""
+    cfg = cfg_for(W=W, H=H, res=(64, 64, 64), color=color, trunc=0.1)
+    cfg.photometric_weight = 0.1 if color else 0.0
+    seq = frames(4, W=W, H=H, seed=5, color=color)
+    one = L.Session(gpu_ctx, cfg)
+    many = [L.Session(gpu_ctx, cfg) for _ in range(9)]
+    eng = None if color else O.Engine(cfg)
+    for d, c, _, _ in seq:
+        ok, p = one.process(d, c)
+        st, q = gpu_ctx.batch_tick(many, [d] * 9, [c] * 9 if color else None)
+        assert np.all((st == 0) == ok)  # (the smallest image loses tracking, by every route)
+        assert np.array_equal(q, np.repeat(q[:1], 9, axis=0))
+        assert rot_angle(p[:9].reshape(3, 3), q[0, :9].reshape(3, 3)) < 1e-5
+        assert np.max(np.abs(p[9:] - q[0, 9:])) < 1e-5
+        if eng is not None:
+            assert bool(eng.frame(d)) == ok
+            R, t = eng.pose()
+            assert rot_angle(p[:9].reshape(3, 3), R) < 1e-4 and np.max(np.abs(p[9:] - t)) < 1e-4
+    for s in [one] + many:
+        s.close()
+
+
+def _f32(x):
+    """The float32 nearest to a rational (ties to even), as a Fraction; normal range."""
+    if x == 0:
+        return Fraction(0)
+    s, x, e = (-1, -x, 0) if x < 0 else (1, x, 0)
+    while x >= 1 << 24:
+        x, e = x / 2, e + 1
+    while x < 1 << 23:
+        x, e = x * 2, e - 1
+    n, r = divmod(x.numerator, x.denominator)
+    r = Fraction(r, x.denominator)
+    n += 1 if r > Fraction(1, 2) or (r == Fraction(1, 2) and n & 1) else 0
+    return s * n * Fraction(2) ** e
+
+
+def test_shared_reciprocal_quotient_is_the_division():
+    """div_shared's steps in exact arithmetic with one rounding each, against the rounded
+    quotient: random and extreme mantissas over the range it is used in."""
+    rng = random.Random(7)
+
+    def value(lo, hi):
+        m = rng.choice([rng.randrange(1 << 23, 1 << 24), (1 << 24) - 1 - rng.randrange(4), (1 << 23) + rng.randrange(4)])
+        return Fraction(m) * Fraction(2) ** (rng.randint(lo, hi) - 23)
+
+    for _ in range(3000):
+        a, b = value(-60, 59) * rng.choice([-1, 1]), value(-40, 39)
+        r = _f32(1 / b)
+        q = _f32(a * r)
+        for _ in range(2):
+            q = _f32(q + _f32(a - q * b) * r)
+        assert q == _f32(a / b), (a, b)
