@@ -19,6 +19,7 @@ constexpr int kPreBlockX = 32, kPreBlockY = 8;  // k_preprocess block: 32 x 16 p
 // on, so that the 32 lanes reading the eight components of four rows hit 32 banks.
 constexpr int kIcpHalf = 144;                       // floats from the first array to the second
 constexpr int kIcpStageBytes = (kIcpHalf + 128) * 4;  // per warp (also holds its 64 sums)
+constexpr int kSummaryBricks = 32;  // bricks a block of k_brick_summary looks at
 constexpr int kFastWarps = 4;  // warps per block of the tolerance-mode integration
 constexpr int kFastWarpSmem = 64 * 32 * 4 + 64 * 32 * 4;  // its shared memory per warp (bytes)
 

@@ -220,10 +220,13 @@ __global__ void __launch_bounds__(kTsdfThreads, 4) k_integrate(const SessionDesc
   if ((int)(threadIdx.x & 31) == __ffs(mask) - 1 && t) atomicAdd(&s.ts->touched, (unsigned long long)t);
 }
 
-// Re-classifies the bricks integration touched.  A block looks at 1024 bricks: it first
-// compacts the dirty ones into a shared list, then each warp classifies listed bricks,
+// Re-classifies the bricks integration touched.  A block looks at kSummaryBricks bricks: it
+// first compacts the dirty ones into a shared list, then each warp classifies listed bricks,
 // every lane reading 16 of a brick's 512 voxels (8 consecutive x per row, so each row is
-// one contiguous run).
+// one contiguous run).  A warp's bricks follow one another, ~1 us each, so the time is that of
+// the block with most of them: 1024 bricks a block (32 blocks at 256^3) took 141 us an
+// integration of a 640 x 480 frame, 128 took 74, 32 take 28 (512^3, every brick dirty: 706 us,
+// 293, 259).
 template <int FMT>
 __global__ void __launch_bounds__(256) k_brick_summary(const SessionDesc* __restrict__ descs, int force) {
   const SessionDesc& s = descs[blockIdx.y];
@@ -231,13 +234,13 @@ __global__ void __launch_bounds__(256) k_brick_summary(const SessionDesc* __rest
   if (!force && (s.kind < 0 || !s.ts->integrate)) return;
   const int bx = (s.res[0] + 7) >> 3, by = (s.res[1] + 7) >> 3, bz = (s.res[2] + 7) >> 3;
   const long nb = (long)bx * by * bz;
-  const long b0 = (long)blockIdx.x * 1024;
+  const long b0 = (long)blockIdx.x * kSummaryBricks;
   if (b0 >= nb) return;
-  __shared__ int list[1024];
+  __shared__ int list[kSummaryBricks];
   __shared__ int count;
   if (threadIdx.x == 0) count = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < 1024; i += blockDim.x) {
+  for (int i = threadIdx.x; i < kSummaryBricks; i += blockDim.x) {
     const long b = b0 + i;
     if (b < nb && s.occ[b] == kBrickDirty) list[atomicAdd(&count, 1)] = i;
   }
@@ -282,8 +285,10 @@ __global__ void __launch_bounds__(256) k_brick_summary(const SessionDesc* __rest
 }
 
 // Re-classifies the super-bricks whose bricks k_brick_summary changed, then the 128^3
-// regions holding them: one block of 64 threads per region, one thread per super-brick.
-__global__ void __launch_bounds__(64) k_super_summary(const SessionDesc* __restrict__ descs, int force) {
+// regions holding them: one block of 1024 threads per region, sixteen a super-brick, a row of
+// four bricks each (one thread a super-brick took 64 dependent-latency loads: 11.7 us a launch,
+// now 5).
+__global__ void __launch_bounds__(1024) k_super_summary(const SessionDesc* __restrict__ descs, int force) {
   const SessionDesc& s = descs[blockIdx.y];
   if (s.fmt < 0 || !s.occ2) return;
   if (!force && (s.kind < 0 || !s.ts->integrate)) return;
@@ -292,27 +297,33 @@ __global__ void __launch_bounds__(64) k_super_summary(const SessionDesc* __restr
   const int h = blockIdx.x;
   if (h >= hx * hy * hz) return;
   const int HX = h % hx, HY = (h / hx) % hy, HZ = h / (hx * hy);
-  const int X = 4 * HX + (threadIdx.x & 3), Y = 4 * HY + ((threadIdx.x >> 2) & 3), Z = 4 * HZ + (threadIdx.x >> 4);
+  const int sb = threadIdx.x >> 4, row = threadIdx.x & 15;  // super-brick of the region, row of it
+  const int X = 4 * HX + (sb & 3), Y = 4 * HY + ((sb >> 2) & 3), Z = 4 * HZ + (sb >> 4);
   const bool live = X < sx && Y < sy && Z < sz;
   const size_t i = (size_t)X + (size_t)sx * (Y + (size_t)sy * Z);
-  uint8_t st = kSuperEmpty;
-  bool changed = false;
-  if (live) {
-    st = s.occ2[i];
-    if (st == kSuperDirty) {
-      changed = true;
-      const int bx = (s.res[0] + 7) >> 3, by = (s.res[1] + 7) >> 3, bz = (s.res[2] + 7) >> 3;
-      bool all_empty = true, mixed = false;
-      for (int c = 4 * Z; c < min(4 * Z + 4, bz); ++c)
-        for (int b = 4 * Y; b < min(4 * Y + 4, by); ++b)
-          for (int a = 4 * X; a < min(4 * X + 4, bx); ++a) {
-            const uint8_t bs = s.occ[a + (size_t)bx * (b + (size_t)by * c)];
-            if (bs != kBrickEmpty) all_empty = false;
-            if (bs == kBrickMixed || bs == kBrickDirty) mixed = true;
-          }
-      st = mixed ? kSuperMixed : all_empty ? kSuperEmpty : kSuperSkip;
-      s.occ2[i] = st;
+  uint8_t st = live ? s.occ2[i] : (uint8_t)kSuperEmpty;
+  const bool changed = st == kSuperDirty;
+  bool nonempty = false, mixed = false;
+  if (changed) {
+    const int bx = (s.res[0] + 7) >> 3, by = (s.res[1] + 7) >> 3, bz = (s.res[2] + 7) >> 3;
+    const int b = 4 * Y + (row & 3), c = 4 * Z + (row >> 2);
+    if (b < by && c < bz) {
+      const uint8_t* p = s.occ + 4 * X + (size_t)bx * (b + (size_t)by * c);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+        if (4 * X + a < bx) {
+          const uint8_t bs = p[a];
+          nonempty |= bs != kBrickEmpty;
+          mixed |= bs == kBrickMixed || bs == kBrickDirty;
+        }
     }
+  }
+  // the sixteen lanes of a super-brick
+  const unsigned half = (threadIdx.x & 16) ? 0xffff0000u : 0xffffu;
+  const bool any_ne = __ballot_sync(0xffffffffu, nonempty) & half, any_mx = __ballot_sync(0xffffffffu, mixed) & half;
+  if (changed) {
+    st = any_mx ? kSuperMixed : any_ne ? kSuperSkip : kSuperEmpty;
+    if (row == 0) s.occ2[i] = st;
   }
   const bool any_changed = __syncthreads_or(changed);
   if (!any_changed) return;

@@ -553,7 +553,7 @@ void launch_summary(const BatchPlan& p, const SessionDesc* d, cudaStream_t st, i
   // the tolerance-mode integration re-classifies the bricks it updates itself: bricks of
   // those formats are left dirty only by a shift (or an import, which forces the pass)
   if (F >= NUI_TSDF_F16_U8 && !force && !(p.shiftFmtMask & (1 << F))) return;
-  k_brick_summary<F><<<dim3(cdiv(p.maxBricks[F], 1024), dense_n(p)), 256, 0, st>>>(d, force);
+  k_brick_summary<F><<<dim3(cdiv(p.maxBricks[F], kSummaryBricks), dense_n(p)), 256, 0, st>>>(d, force);
 }
 // Brick re-classification after integration, then the super-bricks it touched.
 void launch_summaries(const BatchPlan& p, const SessionDesc* d, cudaStream_t st, int force) {
@@ -561,7 +561,7 @@ void launch_summaries(const BatchPlan& p, const SessionDesc* d, cudaStream_t st,
   launch_summary<1>(p, d, st, force);
   launch_summary<2>(p, d, st, force);
   launch_summary<3>(p, d, st, force);
-  if (p.fmtMask) k_super_summary<<<dim3((unsigned)p.maxHyper, dense_n(p)), 64, 0, st>>>(d, force);
+  if (p.fmtMask) k_super_summary<<<dim3((unsigned)p.maxHyper, dense_n(p)), 1024, 0, st>>>(d, force);
 }
 // Blocks of the raycasts: 2 x 2 warps, each a tw x (32 / tw) pixel tile.
 unsigned ray_blocks(const BatchPlan& p, int tw) { return cdiv(p.maxW, 2 * tw) * cdiv(p.maxH, 2 * (32 / tw)); }
