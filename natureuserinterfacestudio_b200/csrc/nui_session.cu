@@ -238,6 +238,7 @@ struct nui_ctx {
   std::map<BatchPlan, Graph> graphs;
   int last_kernels = 0;  // kernels of the last graphed tick
   nui_tuning tune = {18, 4, 8, 8, 12};
+  std::atomic<bool> mc_tables{false}, hash_mc_tables{false};  // the case tables are on the device
   cudaMemPool_t pool = nullptr;  // session state (stream-ordered; freed memory stays here)
 };
 
@@ -2259,7 +2260,8 @@ nui_status nui_hash_mesh_impl(nui_session* s, float* pos, float* col, uint64_t c
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
   NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, st));
-  hash_mc_upload_tables(st, NUI_MC_TRI_PACKED);
+  if (!s->ctx->hash_mc_tables) hash_mc_upload_tables(st, NUI_MC_TRI_PACKED);
+  s->ctx->hash_mc_tables = true;
   DevBuf cnt, off, dp, dc;
   NUI_CUDA(counted_malloc(&cnt.p, (size_t)nvis * 4));
   NUI_CUDA(counted_malloc(&off.p, ((size_t)nvis + 1) * 8));
@@ -2293,41 +2295,53 @@ nui_status nui_hash_mesh_impl(nui_session* s, float* pos, float* col, uint64_t c
 namespace nui {
 void mc_upload_tables(cudaStream_t st);
 template <int F>
-__global__ void k_mc_count(const SessionDesc*, unsigned int*, unsigned long long*, uint8_t*);
+__global__ void k_mc_count(const SessionDesc*, int, unsigned int*, unsigned long long*, uint8_t*);
 __global__ void k_mc_scan(unsigned long long*, int);
 template <int F>
-__global__ void k_mc_emit(const SessionDesc*, const unsigned int*, const unsigned long long*, float*, float*,
+__global__ void k_mc_emit(const SessionDesc*, int, const unsigned int*, const unsigned long long*, float*, float*,
                           unsigned long long);
 }  // namespace nui
 
 namespace {
+constexpr size_t kNoAllocBlocks = 4096;  // count blocks + 1 bound of the meshing without allocation
+// Columns a block takes: the fewest that keep the blocks within the scratch of the meshing
+// without allocation, so that a block's chunks spread over its warps and the blocks over the
+// SMs (the kernels at 256^3 FP32: 393 us with 128 columns, 205 with 32; 512^3 FP16 + u8:
+// 1.22 ms with 128, 0.83 with 64).
+int mc_cols(const nui_session_cfg& c) {
+  int cols = 32;
+  while (cols < 128 && (size_t)cdiv(c.res[0] - 1, cols) * (c.res[1] - 1) + 1 > kNoAllocBlocks) cols *= 2;
+  return cols;
+}
+unsigned mc_blocks(const nui_session_cfg& c) { return cdiv(c.res[0] - 1, mc_cols(c)) * (unsigned)(c.res[1] - 1); }
 template <int F>
-void mc_count(nui_session* s, unsigned nb, unsigned* cc, unsigned long long* bt, uint8_t* cases) {
-  k_mc_count<F><<<nb, 128, 0, s->ctx->stream>>>(s->d_desc1, cc, bt, cases);
+void mc_count(nui_session* s, unsigned* cc, unsigned long long* bt, uint8_t* cases) {
+  k_mc_count<F><<<mc_blocks(s->cfg), 256, 0, s->ctx->stream>>>(s->d_desc1, mc_cols(s->cfg), cc, bt, cases);
 }
 template <int F>
-void mc_emit(nui_session* s, unsigned nb, const unsigned* cc, const unsigned long long* bt, float* p, float* c,
+void mc_emit(nui_session* s, const unsigned* cc, const unsigned long long* bt, float* p, float* c,
              unsigned long long cap) {
-  k_mc_emit<F><<<nb, 128, 0, s->ctx->stream>>>(s->d_desc1, cc, bt, p, c, cap);
+  const int cols = mc_cols(s->cfg), chunks = (s->cfg.res[2] - 1 + 31) / 32;
+  k_mc_emit<F><<<mc_blocks(s->cfg), 256, (size_t)cols * chunks * 8, s->ctx->stream>>>(s->d_desc1, cols, cc, bt, p, c,
+                                                                                      cap);
 }
 // Count pass + block scan; returns the total vertex count.
-nui_status mc_prepare(nui_session* s, DevBuf& cc, DevBuf& bt, unsigned& nb, uint8_t* d_cases,
-                      unsigned long long& total) {
+nui_status mc_prepare(nui_session* s, DevBuf& cc, DevBuf& bt, uint8_t* d_cases, unsigned long long& total) {
   const nui_session_cfg& c = s->cfg;
   cudaStream_t st = s->ctx->stream;
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
   NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, st));
-  mc_upload_tables(st);
-  const unsigned tilesX = cdiv(c.res[0] - 1, 128);
-  nb = tilesX * (unsigned)(c.res[1] - 1);
+  if (!s->ctx->mc_tables) mc_upload_tables(st);
+  s->ctx->mc_tables = true;
+  const unsigned nb = mc_blocks(c);
   NUI_CUDA(counted_malloc(&cc.p, sizeof(unsigned) * (size_t)(c.res[0] - 1) * (c.res[1] - 1)));
   NUI_CUDA(counted_malloc(&bt.p, sizeof(unsigned long long) * (nb + 1)));
   switch (c.tsdf_format) {
-    case 0: mc_count<0>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
-    case 1: mc_count<1>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
-    case 2: mc_count<2>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
-    case 3: mc_count<3>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
+    case 0: mc_count<0>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
+    case 1: mc_count<1>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
+    case 2: mc_count<2>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
+    case 3: mc_count<3>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, d_cases); break;
   }
   k_mc_scan<<<1, 1024, 0, st>>>((unsigned long long*)bt.p, (int)nb);
   NUI_CUDA(cudaGetLastError());
@@ -2341,9 +2355,8 @@ extern "C" NUI_API nui_status nui_mesh(nui_session* s, float* pos, float* col, u
   if (!s || !nverts) return fail(NUI_ERR_INVALID_ARG, "null argument");
   if (s->hash) return nui_hash_mesh_impl(s, pos, col, cap, nverts);
   DevBuf cc, bt, dp, dc;
-  unsigned nb = 0;
   unsigned long long total = 0;
-  nui_status st = mc_prepare(s, cc, bt, nb, nullptr, total);
+  nui_status st = mc_prepare(s, cc, bt, nullptr, total);
   if (st != NUI_OK) return st;
   *nverts = total;
   const unsigned long long k = total < cap ? total : cap;
@@ -2351,10 +2364,10 @@ extern "C" NUI_API nui_status nui_mesh(nui_session* s, float* pos, float* col, u
     if (pos) NUI_CUDA(counted_malloc(&dp.p, k * 3 * sizeof(float)));
     if (col) NUI_CUDA(counted_malloc(&dc.p, k * 4 * sizeof(float)));
     switch (s->cfg.tsdf_format) {
-      case 0: mc_emit<0>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
-      case 1: mc_emit<1>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
-      case 2: mc_emit<2>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
-      case 3: mc_emit<3>(s, nb, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
+      case 0: mc_emit<0>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
+      case 1: mc_emit<1>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
+      case 2: mc_emit<2>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
+      case 3: mc_emit<3>(s, (unsigned*)cc.p, (unsigned long long*)bt.p, (float*)dp.p, (float*)dc.p, k); break;
     }
     NUI_CUDA(cudaGetLastError());
     if (pos) NUI_CUDA(cudaMemcpyAsync(pos, dp.p, k * 3 * sizeof(float), cudaMemcpyDeviceToHost, s->ctx->stream));
@@ -2373,9 +2386,8 @@ extern "C" NUI_API nui_status nui_mesh_cases(nui_session* s, uint8_t* cases, siz
   if (bytes < need) return fail(NUI_ERR_INVALID_ARG, "buffer too small");
   DevBuf cc, bt, dcase;
   NUI_CUDA(counted_malloc(&dcase.p, need));
-  unsigned nb = 0;
   unsigned long long total = 0;
-  nui_status st = mc_prepare(s, cc, bt, nb, (uint8_t*)dcase.p, total);
+  nui_status st = mc_prepare(s, cc, bt, (uint8_t*)dcase.p, total);
   if (st != NUI_OK) return st;
   NUI_CUDA(cudaMemcpy(cases, dcase.p, need, cudaMemcpyDeviceToHost));
   if (nverts) *nverts = total;
@@ -2383,12 +2395,11 @@ extern "C" NUI_API nui_status nui_mesh_cases(nui_session* s, uint8_t* cases, siz
 }
 
 // ------------------------------------------------------------------ meshing without allocation
-// Scratch of nui_mesh_device_noalloc: per-column vertex counts (u32) and per-block offsets
+// Scratch of nui_mesh_device_noalloc: per-column chunk marks (u32) and per-block offsets
 // (u64).  A file-scope device array: host code reaches it only through the address that
 // cudaGetSymbolAddress returns for the current device.
 namespace {
 constexpr size_t kNoAllocCols = 262144;   // (res[0]-1)*(res[1]-1) bound
-constexpr size_t kNoAllocBlocks = 4096;   // count blocks + 1 bound
 static __device__ __align__(256) unsigned char g_mesh_scratch[kNoAllocCols * 4 + kNoAllocBlocks * 8];
 constexpr int kMaxDevices = 64;
 unsigned char* g_mesh_scratch_addr[kMaxDevices] = {};
@@ -2411,8 +2422,8 @@ struct DeviceGuard {
 // Device address of the scratch array on `device` (current); looked up on the first call
 // after the library loads or after a context is created on the device (nui_ctx_create
 // forgets the cached address, so that a device reset followed by a new context looks it up
-// again).  Nothing in the array needs to start at zero: the count pass writes every column
-// count and every block total before the scan and the emit pass read them.
+// again).  Nothing in the array needs to start at zero: the count pass writes every column's
+// marks and every block total before the scan and the emit pass read them.
 nui_status noalloc_scratch(int device, unsigned char** out) {
   if (device < 0 || device >= kMaxDevices) return fail(NUI_ERR_INVALID_ARG, "device index out of range");
   std::lock_guard<std::mutex> lock(g_mesh_scratch_mu);
@@ -2445,7 +2456,7 @@ extern "C" NUI_API nui_status nui_mesh_device_noalloc(nui_session* s, float* d_p
   if (s->hash) return fail(NUI_ERR_UNSUPPORTED, "dense sessions only");
   const nui_session_cfg& c = s->cfg;
   const size_t ncols = (size_t)(c.res[0] - 1) * (c.res[1] - 1);
-  const unsigned nb = cdiv(c.res[0] - 1, 128) * (unsigned)(c.res[1] - 1);
+  const unsigned nb = mc_blocks(c);  // with 128 columns a block when no fewer fit
   if (ncols > kNoAllocCols || (size_t)nb + 1 > kNoAllocBlocks)
     return fail(NUI_ERR_INVALID_ARG, "volume too large for the no-allocation mesh scratch");
   DeviceGuard guard;
@@ -2470,30 +2481,30 @@ extern "C" NUI_API nui_status nui_mesh_device_noalloc(nui_session* s, float* d_p
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
   NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, st));
-  mc_upload_tables(st);
+  if (!s->ctx->mc_tables) mc_upload_tables(st);
+  s->ctx->mc_tables = true;
   switch (c.tsdf_format) {
-    case 0: mc_count<0>(s, nb, cc, bt, nullptr); break;
-    case 1: mc_count<1>(s, nb, cc, bt, nullptr); break;
-    case 2: mc_count<2>(s, nb, cc, bt, nullptr); break;
-    case 3: mc_count<3>(s, nb, cc, bt, nullptr); break;
+    case 0: mc_count<0>(s, cc, bt, nullptr); break;
+    case 1: mc_count<1>(s, cc, bt, nullptr); break;
+    case 2: mc_count<2>(s, cc, bt, nullptr); break;
+    case 3: mc_count<3>(s, cc, bt, nullptr); break;
   }
   k_mc_scan<<<1, 1024, 0, st>>>(bt, (int)nb);
   NUI_CUDA(cudaGetLastError());
+  // the emission stops at the capacity and at the total by itself, so the host waits once
+  if (cap > 0 && (d_pos || d_col)) {
+    switch (c.tsdf_format) {
+      case 0: mc_emit<0>(s, cc, bt, d_pos, d_col, cap); break;
+      case 1: mc_emit<1>(s, cc, bt, d_pos, d_col, cap); break;
+      case 2: mc_emit<2>(s, cc, bt, d_pos, d_col, cap); break;
+      case 3: mc_emit<3>(s, cc, bt, d_pos, d_col, cap); break;
+    }
+    NUI_CUDA(cudaGetLastError());
+  }
   unsigned long long total = 0;
   NUI_CUDA(cudaMemcpyAsync(&total, bt + nb, sizeof(total), cudaMemcpyDeviceToHost, st));
   NUI_CUDA(cudaStreamSynchronize(st));
   *nverts = total;
-  const unsigned long long k = total < cap ? total : cap;
-  if (k > 0 && (d_pos || d_col)) {
-    switch (c.tsdf_format) {
-      case 0: mc_emit<0>(s, nb, cc, bt, d_pos, d_col, k); break;
-      case 1: mc_emit<1>(s, nb, cc, bt, d_pos, d_col, k); break;
-      case 2: mc_emit<2>(s, nb, cc, bt, d_pos, d_col, k); break;
-      case 3: mc_emit<3>(s, nb, cc, bt, d_pos, d_col, k); break;
-    }
-    NUI_CUDA(cudaGetLastError());
-    NUI_CUDA(cudaStreamSynchronize(st));
-  }
   if (total > cap) return fail(NUI_ERR_MESH_OVERFLOW, "mesh larger than the output capacity");
   return NUI_OK;
 }
