@@ -96,6 +96,7 @@ enum FrameKind : int { kInactive = -1, kFirstFrame = 0, kTrackFrame = 1 };
 
 // hcount slots read by the frame's status check (k_hash_health)
 constexpr int kHashFailed = 3, kHashChainFaults = 9, kHashFailedBefore = 10;
+constexpr int kHashFaultsBefore = 12;  // step-wise integration: chain faults before it
 
 struct SessionDesc {
   int kind;  // FrameKind
@@ -171,7 +172,7 @@ struct SessionDesc {
                                   // of the swap pass, [7] store blocks used, [8] store-full refusals,
                                   // [9] corrupted excess chains met this frame, [10] failed
                                   // allocations before this frame, [11] pixels the forward
-                                  // render casts
+                                  // render casts, [12] chain faults before this integration
   // forward rendering of the reference maps (0 off, 1 the reference's projection, 2 world to
   // camera): per pixel the last source pixel landing on it (+1), the missing pixels listed in
   // increasing order, per-1024-pixel-block counts then offsets, landed colours

@@ -24,8 +24,7 @@ __device__ __forceinline__ const uchar4* color_level(const SessionDesc& s, int l
   return l == 0 ? reinterpret_cast<const uchar4*>(s.bgra) : s.cpyr[l];
 }
 
-__global__ void __launch_bounds__(256) k_color_level(const SessionDesc* __restrict__ descs, int l) {
-  const SessionDesc& s = descs[blockIdx.y];
+__global__ void __launch_bounds__(256) k_color_level(const __grid_constant__ SessionDesc s, int l) {
   if (s.kind != kTrackFrame || !(s.photo_w > 0.f) || !s.bgra || l >= s.levels || !s.cpyr[l]) return;
   const int dW = s.W >> l, dH = s.H >> l, sW = 2 * dW, sH = 2 * dH;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -49,9 +48,7 @@ __global__ void __launch_bounds__(256) k_color_level(const SessionDesc* __restri
 
 __device__ __forceinline__ unsigned char grad_byte(float v) { return (unsigned char)(int)v; }
 
-__global__ void __launch_bounds__(256) k_color_grad(const SessionDesc* __restrict__ descs, int fam) {
-  const SessionDesc& s = descs[blockIdx.y];
-  const int l = blockIdx.z;
+__device__ __forceinline__ void color_grad_pixel(const SessionDesc& s, int fam, int l) {
   if (s.kind != kTrackFrame || !in_family(s, fam) || !(s.photo_w > 0.f) || !s.bgra || l >= s.levels || !s.cgx[l]) return;
   const int W = s.W >> l, H = s.H >> l;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,6 +73,13 @@ __global__ void __launch_bounds__(256) k_color_grad(const SessionDesc* __restric
   s.cgy[l][i] = make_uchar4(grad_byte(sob_x(s31.x, s11.x, s32.x, s12.x, s33.x, s13.x)),
                             grad_byte(sob_x(s31.y, s11.y, s32.y, s12.y, s33.y, s13.y)),
                             grad_byte(sob_x(s31.z, s11.z, s32.z, s12.z, s33.z, s13.z)), 255);
+}
+
+__global__ void __launch_bounds__(256) k_color_grad(const SessionDesc* __restrict__ descs, int fam) {
+  color_grad_pixel(descs[blockIdx.y], fam, blockIdx.z);
+}
+__global__ void __launch_bounds__(256) k_color_grad_one(const __grid_constant__ SessionDesc d) {
+  color_grad_pixel(d, kFamAll, blockIdx.z);
 }
 
 // Four pixels a thread (16-byte copies when both buffers allow them).

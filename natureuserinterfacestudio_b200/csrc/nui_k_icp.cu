@@ -768,7 +768,7 @@ template __global__ void k_icp_finest<true>(const SessionDesc*, int, int, int, i
 // (tsdfVolume.cl:74-79: v_g_z and z_scaled, both advanced by cell_z per slice), for the
 // pose integration will use: ztab[z] and ztab[rz + 1 + z] after z additions.
 __device__ void fill_ztab(const SessionDesc& s, const TrackState* ts) {
-  if (!s.ztab) return;
+  if (!s.ztab || s.tol) return;  // the tolerance-mode integration computes its positions directly
   const int rz = s.res[2];
   const float c2 = s.cell[2];
   float vgz = 0.5f * c2 - ts->xf.t[2], zs = 0.f;
@@ -808,14 +808,30 @@ __device__ void shift_decide(const SessionDesc& s, TrackState* ts) {
   }
 }
 
-// The table for an integration the host requests directly (step-wise calls), after the
-// shift that integration makes.
+// Start of an integration the host requests directly (step-wise calls): the gate opens, the
+// counters it reports start over (for a voxel hash, the failures before it are noted), the
+// shift is made and the table filled.
 __global__ void k_ztab(const SessionDesc* __restrict__ descs) {
   const SessionDesc& s = descs[blockIdx.x];
-  if (threadIdx.x == 0 && s.kind >= 0) {
-    shift_decide(s, s.ts);
-    fill_ztab(s, s.ts);
+  if (threadIdx.x != 0 || s.kind < 0) return;
+  s.ts->integrate = 1;
+  s.ts->touched = 0ull;
+  if (s.hcount) {
+    s.hcount[kHashFailedBefore] = s.hcount[kHashFailed];
+    s.hcount[kHashFaultsBefore] = s.hcount[kHashChainFaults];
   }
+  shift_decide(s, s.ts);
+  fill_ztab(s, s.ts);
+}
+
+// nui_set_pose: the camera pose and the tracker's estimate.
+__global__ void k_set_pose(TrackState* ts, const __grid_constant__ DevXform m) {
+  const int k = threadIdx.x;
+  if (k < 9) {
+    ts->xf.R[k] = ts->R[k] = m.R[k];
+    ts->xf.R_inv[k] = m.R_inv[k];
+  }
+  if (k < 3) ts->xf.t[k] = ts->t[k] = m.t[k];
 }
 
 // shift_now: the tick's finalize makes the shifting volume's shift of an integrating

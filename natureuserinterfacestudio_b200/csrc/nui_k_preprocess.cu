@@ -92,8 +92,7 @@ __device__ __forceinline__ void bilateral_px2_tol(const float* t, const float* l
   out1 = __fdividef(sd1, sw1);
 }
 
-__global__ void __launch_bounds__(kPreBlockX* kPreBlockY, 4) k_preprocess(const SessionDesc* __restrict__ descs) {
-  const SessionDesc& s = descs[blockIdx.y];
+__device__ __forceinline__ void preprocess_block(const SessionDesc& s) {
   if (s.kind < 0) return;
   const int W = s.W, H = s.H, R = s.radius;
   const int tilesX = (W + kPreTX - 1) / kPreTX;
@@ -186,10 +185,19 @@ __global__ void __launch_bounds__(kPreBlockX* kPreBlockY, 4) k_preprocess(const 
   }
 }
 
+__global__ void __launch_bounds__(kPreBlockX* kPreBlockY, 4) k_preprocess(const SessionDesc* __restrict__ descs) {
+  preprocess_block(descs[blockIdx.y]);
+}
+// The kernel-level calls pass their descriptor (and pose) by value: a descriptor copied to the
+// device first cost each call a blocking copy and the launch a wait for it (five calls on a
+// 160 x 120 frame: 102 us with the copies, 90 without).
+__global__ void __launch_bounds__(kPreBlockX* kPreBlockY, 4) k_preprocess_one(const __grid_constant__ SessionDesc d) {
+  preprocess_block(d);
+}
+
 // One pyramid level: dst(x,y) = mean of the 3x3 taps around src(2x,2y) within the depth
 // threshold of the centre (any valid tap if the centre is NaN); vertices with div = 2^l.
-__global__ void k_pyramid(const SessionDesc* __restrict__ descs, int level) {
-  const SessionDesc& s = descs[blockIdx.y];
+__device__ __forceinline__ void pyramid_pixel(const SessionDesc& s, int level) {
   if (s.kind != kTrackFrame || level >= s.levels) return;
   const int dW = s.W >> level, dH = s.H >> level, sW = dW * 2, sH = dH * 2;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -214,6 +222,9 @@ __global__ void k_pyramid(const SessionDesc* __restrict__ descs, int level) {
   if (s.vlev[level]) s.vlev[level][idx] = w0(level_vertex(s.cam, level, x, y, d));
 }
 
+__global__ void k_pyramid(const SessionDesc* __restrict__ descs, int level) { pyramid_pixel(descs[blockIdx.y], level); }
+__global__ void k_pyramid_one(const __grid_constant__ SessionDesc d, int level) { pyramid_pixel(d, level); }
+
 // A level's vertex map from its depth, for downloads (sessions keep no vertex maps).
 __global__ void k_vertex_map(const SessionDesc* __restrict__ descs, int level, float4* __restrict__ out) {
   const SessionDesc& s = descs[blockIdx.y];
@@ -225,9 +236,7 @@ __global__ void k_vertex_map(const SessionDesc* __restrict__ descs, int level, f
 
 // Frame-0 reference maps: simple normals from the level-0 vertex map, then both maps to
 // world space with the current pose (NuiKinfuOpenCLFeedbackFrame::UpdateBuffers, :71-91).
-__global__ void k_feedback(const SessionDesc* __restrict__ descs) {
-  const SessionDesc& s = descs[blockIdx.y];
-  if (s.kind != kFirstFrame) return;
+__device__ __forceinline__ void feedback_pixel(const SessionDesc& s, const DevXform& m) {
   const int W = s.W, H = s.H;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= W * H) return;
@@ -238,7 +247,6 @@ __global__ void k_feedback(const SessionDesc* __restrict__ descs) {
     return V ? xyz(V[j]) : level_vertex(s.cam, 0, jx, jy, s.dlev[0][j]);
   };
   const float3 c = vtx(idx, x, y);
-  const DevXform& m = s.ts->xf;
   if (isnan3(c)) {
     s.vref[idx] = make_float4(qnan(), qnan(), qnan(), 0.f);
     s.nref[idx] = make_float4(qnan(), qnan(), qnan(), 0.f);
@@ -262,6 +270,14 @@ __global__ void k_feedback(const SessionDesc* __restrict__ descs) {
     if (s.hash) cc = make_uchar4(cc.z, cc.y, cc.x, cc.w);
     s.cmap[idx] = cc;
   }
+}
+
+__global__ void k_feedback(const SessionDesc* __restrict__ descs) {
+  const SessionDesc& s = descs[blockIdx.y];
+  if (s.kind == kFirstFrame) feedback_pixel(s, s.ts->xf);
+}
+__global__ void k_feedback_one(const __grid_constant__ SessionDesc d, const __grid_constant__ DevXform m) {
+  feedback_pixel(d, m);
 }
 
 }  // namespace nui

@@ -28,7 +28,10 @@
 
 namespace nui {
 __global__ void k_preprocess(const SessionDesc*);
+__global__ void k_preprocess_one(const SessionDesc);
 __global__ void k_pyramid(const SessionDesc*, int);
+__global__ void k_pyramid_one(const SessionDesc, int);
+__global__ void k_feedback_one(const SessionDesc, const DevXform);
 __global__ void k_feedback(const SessionDesc*);
 __global__ void k_vertex_map(const SessionDesc*, int, float4*);
 template <bool COLOR>
@@ -37,7 +40,9 @@ template <bool COLOR>
 __global__ void k_icp_finest(const SessionDesc*, int, int, int, int, IcpFinest*);
 __global__ void k_track_finalize(const SessionDesc*, int, int);
 __global__ void k_ztab(const SessionDesc*);
-__global__ void k_color_level(const SessionDesc*, int);
+__global__ void k_color_level(const SessionDesc, int);
+__global__ void k_color_grad_one(const SessionDesc);
+__global__ void k_set_pose(TrackState*, const DevXform);
 __global__ void k_color_grad(const SessionDesc*, int);
 __global__ void k_color_keep(const SessionDesc*, int);
 template <int F>
@@ -226,9 +231,6 @@ struct nui_ctx {
   int* h_status = nullptr;  // 2 * cap * 2
   int par = 0;              // the half the next tick uses
   cudaEvent_t ev_tick[2] = {nullptr, nullptr};
-  // scratch descriptor for kernel-level calls
-  SessionDesc* d_kdesc = nullptr;
-  TrackState* d_kts = nullptr;
   IcpFinest* d_finest = nullptr;  // level-0 ICP over the whole device: 2 x kIcpWideSessions (a set a stream)
   unsigned long long* d_count = nullptr;  // counter of the point-cloud fetch
   struct Graph {
@@ -270,7 +272,9 @@ struct nui_session {
   uchar4* cgy[kMaxLevels] = {};
   float* pts_xyz = nullptr;   // shifting volume: point cache of the slabs that left
   float* pts_rgba = nullptr;
-  SessionDesc* d_desc1 = nullptr;
+  SessionDesc* d_desc1 = nullptr;  // one-entry table of the step-wise calls,
+  SessionDesc h_desc1;             // what it holds
+  bool desc1_set = false;
   // voxel-block hash
   bool hash = false;
   HEntry* entries = nullptr;
@@ -478,6 +482,17 @@ void fill_desc(const nui_session* s, SessionDesc& d, int kind, const uint16_t* r
     d.fwd_blk = s->fwd_blk;
     d.fwd_col = s->fwd_col;
   }
+}
+
+// Puts the descriptor into the session's one-entry table in stream order; a table that holds it
+// already is left alone (a pageable copy costs a step-wise call ~6 us).
+cudaError_t upload_desc1(nui_session* s, const SessionDesc& d) {
+  if (s->desc1_set && std::memcmp(&s->h_desc1, &d, sizeof(d)) == 0) return cudaSuccess;
+  s->desc1_set = false;
+  std::memcpy(&s->h_desc1, &d, sizeof(d));
+  const cudaError_t e = cudaMemcpyAsync(s->d_desc1, &s->h_desc1, sizeof(d), cudaMemcpyHostToDevice, s->ctx->stream);
+  s->desc1_set = e == cudaSuccess;
+  return e;
 }
 
 void plan_add(BatchPlan& p, const nui_session* s) {
@@ -1051,7 +1066,7 @@ void launch_init(nui_session* s) {
 nui_status reset_session(nui_session* s, bool sync = true) {
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
-  NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, s->ctx->stream));
+  NUI_CUDA(upload_desc1(s, d));
   if (s->hash) {
     k_hash_reset<<<1184, 256, 0, s->ctx->stream>>>(s->d_desc1);
   } else {
@@ -1144,9 +1159,7 @@ NUI_API nui_status nui_ctx_create(int device, nui_ctx** out) {
     delete c;
     return fail(NUI_ERR_DEVICE, "context streams");
   }
-  if (counted_malloc(&c->d_kdesc, sizeof(SessionDesc)) != cudaSuccess ||
-      counted_malloc(&c->d_kts, sizeof(TrackState)) != cudaSuccess ||
-      counted_malloc(&c->d_count, sizeof(unsigned long long)) != cudaSuccess) {
+  if (counted_malloc(&c->d_count, sizeof(unsigned long long)) != cudaSuccess) {
     delete c;
     return fail(NUI_ERR_OOM, "context scratch");
   }
@@ -1177,8 +1190,6 @@ NUI_API nui_status nui_ctx_destroy(nui_ctx* c) {
   cudaFree(c->d_status);
   cudaFreeHost(c->h_pose);
   cudaFreeHost(c->h_status);
-  cudaFree(c->d_kdesc);
-  cudaFree(c->d_kts);
   if (c->d_finest) cudaFreeAsync(c->d_finest, c->stream);
   cudaFree(c->d_count);
   cudaStreamDestroy(c->own);
@@ -1591,8 +1602,7 @@ NUI_API nui_status nui_batch_tick_device(nui_ctx* ctx, nui_session* const* ss, i
 
 NUI_API nui_status nui_set_pose(nui_session* s, const float* pose12) {
   if (!s || !pose12) return fail(NUI_ERR_INVALID_ARG, "null argument");
-  TrackState t;
-  NUI_CUDA(cudaMemcpy(&t, s->ts, sizeof(t), cudaMemcpyDeviceToHost));
+  DevXform m;
   double a[9];
   for (int i = 0; i < 9; ++i) a[i] = pose12[i];
   const double c00 = a[4] * a[8] - a[5] * a[7], c01 = a[5] * a[6] - a[3] * a[8], c02 = a[3] * a[7] - a[4] * a[6];
@@ -1601,21 +1611,22 @@ NUI_API nui_status nui_set_pose(nui_session* s, const float* pose12) {
                          c01, a[0] * a[8] - a[2] * a[6], a[2] * a[3] - a[0] * a[5],
                          c02, a[1] * a[6] - a[0] * a[7], a[0] * a[4] - a[1] * a[3]};
   for (int i = 0; i < 9; ++i) {
-    t.xf.R[i] = t.R[i] = pose12[i];
-    t.xf.R_inv[i] = (float)(inv[i] / det);
+    m.R[i] = pose12[i];
+    m.R_inv[i] = (float)(inv[i] / det);
   }
-  for (int i = 0; i < 3; ++i) t.xf.t[i] = t.t[i] = pose12[9 + i];
-  NUI_CUDA(cudaMemcpy(s->ts, &t, sizeof(t), cudaMemcpyHostToDevice));
+  for (int i = 0; i < 3; ++i) m.t[i] = pose12[9 + i];
+  k_set_pose<<<1, 32, 0, s->ctx->stream>>>(s->ts, m);
+  NUI_CUDA(cudaGetLastError());
   return NUI_OK;
 }
 
 NUI_API nui_status nui_get_pose(nui_session* s, float* pose12) {
   if (!s || !pose12) return fail(NUI_ERR_INVALID_ARG, "null argument");
+  DevXform m;
+  NUI_CUDA(cudaMemcpyAsync(&m, &s->ts->xf, sizeof(m), cudaMemcpyDeviceToHost, s->ctx->stream));
   NUI_CUDA(cudaStreamSynchronize(s->ctx->stream));
-  TrackState t;
-  NUI_CUDA(cudaMemcpy(&t, s->ts, sizeof(t), cudaMemcpyDeviceToHost));
-  std::memcpy(pose12, t.xf.R, 9 * sizeof(float));
-  std::memcpy(pose12 + 9, t.xf.t, 3 * sizeof(float));
+  std::memcpy(pose12, m.R, 9 * sizeof(float));
+  std::memcpy(pose12 + 9, m.t, 3 * sizeof(float));
   return NUI_OK;
 }
 
@@ -1803,7 +1814,7 @@ NUI_API nui_status nui_point_cloud_device(nui_session* s, float* d_xyz, float* d
   if (st != NUI_OK) return st;
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
-  NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream));
+  NUI_CUDA(upload_desc1(s, d));
   unsigned long long* counter = ctx->d_count;
   NUI_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), ctx->stream));
   const long long c = (long long)std::min<uint64_t>(cap, (uint64_t)1 << 62);
@@ -1856,12 +1867,13 @@ NUI_API nui_status nui_session_touched_voxels(nui_session* s, uint64_t* n) {
 namespace {
 // Runs a subset of the tick on one session: `what` 0 = preprocess (+pyramid), 1 = track,
 // 2 = integrate, 3 = raycast, 4 = feedback maps (frame-0 path).
-nui_status run_stage(nui_session* s, int what) {
+// sync = false leaves it queued, for a caller that reads its result back behind it.
+nui_status run_stage(nui_session* s, int what, bool sync = true) {
   nui_ctx* ctx = s->ctx;
   SessionDesc d;
   int kind = (what == 4 || (what == 2 && s->frames == 0)) ? kFirstFrame : kTrackFrame;
   fill_desc(s, d, kind, s->raw, s->color_frame ? s->bgra : nullptr);
-  NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream));
+  NUI_CUDA(upload_desc1(s, d));
   BatchPlan p;
   p.n = 1;
   plan_add(p, s);
@@ -1896,7 +1908,7 @@ nui_status run_stage(nui_session* s, int what) {
     if (p.colorIcp) k_color_keep<<<dim3(cdiv(((long)p.maxW * p.maxH + 3) / 4, 256), 1), 256, 0, st>>>(dd, kFamAll);
   }
   NUI_CUDA(cudaGetLastError());
-  NUI_CUDA(cudaStreamSynchronize(st));
+  if (sync) NUI_CUDA(cudaStreamSynchronize(st));
   return NUI_OK;
 }
 
@@ -1930,10 +1942,11 @@ NUI_API nui_status nui_track(nui_session* s, float* err, int* count) {
   if (st != NUI_OK) return st;
   // the track stage must run with the integration threshold of the session, and must
   // not integrate: k_track_finalize only decides the gate
-  st = run_stage(s, 1);
+  st = run_stage(s, 1, false);
   if (st != NUI_OK) return st;
   TrackState t;
-  NUI_CUDA(cudaMemcpy(&t, s->ts, sizeof(t), cudaMemcpyDeviceToHost));
+  NUI_CUDA(cudaMemcpyAsync(&t, s->ts, sizeof(t), cudaMemcpyDeviceToHost, s->ctx->stream));
+  NUI_CUDA(cudaStreamSynchronize(s->ctx->stream));
   if (err) *err = t.error;
   if (count) *count = (int)t.count;
   if (t.status != 0) {
@@ -1946,16 +1959,13 @@ NUI_API nui_status nui_track(nui_session* s, float* err, int* count) {
 
 NUI_API nui_status nui_integrate(nui_session* s) {
   if (!s) return fail(NUI_ERR_INVALID_ARG, "null session");
-  int one = 1;
-  NUI_CUDA(cudaMemcpy(&s->ts->integrate, &one, sizeof(int), cudaMemcpyHostToDevice));
-  NUI_CUDA(cudaMemset(&s->ts->touched, 0, sizeof(unsigned long long)));
   if (!s->hash) return run_stage(s, 2);
-  int before[16], after[16];
-  NUI_CUDA(cudaMemcpy(before, s->hcount, sizeof(before), cudaMemcpyDeviceToHost));
-  nui_status st = run_stage(s, 2);
+  nui_status st = run_stage(s, 2, false);
   if (st != NUI_OK) return st;
-  NUI_CUDA(cudaMemcpy(after, s->hcount, sizeof(after), cudaMemcpyDeviceToHost));
-  if (after[kHashFailed] > before[kHashFailed] || after[kHashChainFaults] > before[kHashChainFaults])
+  int c[16];
+  NUI_CUDA(cudaMemcpyAsync(c, s->hcount, sizeof(c), cudaMemcpyDeviceToHost, s->ctx->stream));
+  NUI_CUDA(cudaStreamSynchronize(s->ctx->stream));
+  if (c[kHashFailed] > c[kHashFailedBefore] || c[kHashChainFaults] > c[kHashFaultsBefore])
     return fail(NUI_ERR_HASH_FULL, "voxel hash: pool or excess list exhausted (or a corrupted chain); blocks dropped");
   return NUI_OK;
 }
@@ -1987,7 +1997,7 @@ NUI_API nui_status nui_debug_download(nui_session* s, int what, int level, void*
       NUI_CUDA(counted_malloc(&tmp, need));
       SessionDesc d;
       fill_desc(s, d, kInactive, nullptr, nullptr);
-      cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, s->ctx->stream);
+      upload_desc1(s, d);
       k_vertex_map<<<dim3(cdiv((long)Nl, 256), 1), 256, 0, s->ctx->stream>>>(s->d_desc1, level, (float4*)tmp);
       cudaError_t e = cudaMemcpyAsync(host, tmp, need, cudaMemcpyDeviceToHost, s->ctx->stream);
       cudaStreamSynchronize(s->ctx->stream);
@@ -2035,7 +2045,7 @@ NUI_API nui_status nui_debug_download(nui_session* s, int what, int level, void*
       NUI_CUDA(counted_malloc(&tmp, need));
       SessionDesc d;
       fill_desc(s, d, kInactive, nullptr, nullptr);
-      cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, s->ctx->stream);
+      upload_desc1(s, d);
       k_hash_export_voxels<<<1184, 256, 0, s->ctx->stream>>>(s->d_desc1, (uint8_t*)tmp);
       cudaError_t e = cudaMemcpyAsync(host, tmp, need, cudaMemcpyDeviceToHost, s->ctx->stream);
       cudaStreamSynchronize(s->ctx->stream);
@@ -2052,7 +2062,7 @@ NUI_API nui_status nui_debug_download(nui_session* s, int what, int level, void*
       NUI_CUDA(counted_malloc(&tmp, need));
       SessionDesc d;
       fill_desc(s, d, kInactive, nullptr, nullptr);
-      cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, s->ctx->stream);
+      upload_desc1(s, d);
       short2* vo = what == 5 ? (short2*)tmp : nullptr;
       uchar4* co = what == 9 ? (uchar4*)tmp : nullptr;
       switch (c.tsdf_format) {
@@ -2096,7 +2106,7 @@ NUI_API nui_status nui_debug_upload_volume(nui_session* s, const int16_t* ref) {
   NUI_CUDA(counted_malloc(&tmp, nv * 4));
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
-  cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, s->ctx->stream);
+  upload_desc1(s, d);
   cudaMemcpyAsync(tmp, ref, nv * 4, cudaMemcpyHostToDevice, s->ctx->stream);
   k_occ_clear<<<256, 256, 0, s->ctx->stream>>>(s->d_desc1);
   switch (s->cfg.tsdf_format) {
@@ -2140,8 +2150,7 @@ NUI_API nui_status nui_k_preprocess(nui_ctx* ctx, const uint16_t* d_raw, int W, 
   d.dlev[0] = d_filtered;
   d.vlev[0] = (float4*)d_vertex4;
   d.dscaled = d_scaled;
-  NUI_CUDA(cudaMemcpyAsync(ctx->d_kdesc, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream));
-  k_preprocess<<<dim3(cdiv(W, 32) * cdiv(H, 16), 1), dim3(kPreBlockX, kPreBlockY), 0, ctx->stream>>>(ctx->d_kdesc);
+  k_preprocess_one<<<dim3(cdiv(W, 32) * cdiv(H, 16), 1), dim3(kPreBlockX, kPreBlockY), 0, ctx->stream>>>(d);
   NUI_CUDA(cudaGetLastError());
   NUI_CUDA(cudaStreamSynchronize(ctx->stream));
   return NUI_OK;
@@ -2164,8 +2173,7 @@ NUI_API nui_status nui_k_pyramid_level(nui_ctx* ctx, const float* d_src, int dW,
   d.dlev[level - 1] = const_cast<float*>(d_src);
   d.dlev[level] = d_dst;
   d.vlev[level] = (float4*)d_vertex4;
-  NUI_CUDA(cudaMemcpyAsync(ctx->d_kdesc, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream));
-  k_pyramid<<<dim3(cdiv((long)dW * dH, 256), 1), 256, 0, ctx->stream>>>(ctx->d_kdesc, level);
+  k_pyramid_one<<<dim3(cdiv((long)dW * dH, 256), 1), 256, 0, ctx->stream>>>(d, level);
   NUI_CUDA(cudaGetLastError());
   NUI_CUDA(cudaStreamSynchronize(ctx->stream));
   return NUI_OK;
@@ -2191,10 +2199,9 @@ NUI_API nui_status nui_k_color_pyramid(nui_ctx* ctx, const uint8_t* d_bgra, int 
     d.cgx[l] = (uchar4*)d_gx[l];
     d.cgy[l] = (uchar4*)d_gy[l];
   }
-  NUI_CUDA(cudaMemcpyAsync(ctx->d_kdesc, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream));
   for (int l = 1; l < levels; ++l)
-    k_color_level<<<dim3(cdiv((long)(W >> l) * (H >> l), 256), 1), 256, 0, ctx->stream>>>(ctx->d_kdesc, l);
-  k_color_grad<<<dim3(cdiv((long)W * H, 256), 1, levels), 256, 0, ctx->stream>>>(ctx->d_kdesc, kFamAll);
+    k_color_level<<<dim3(cdiv((long)(W >> l) * (H >> l), 256), 1), 256, 0, ctx->stream>>>(d, l);
+  k_color_grad_one<<<dim3(cdiv((long)W * H, 256), 1, levels), 256, 0, ctx->stream>>>(d);
   NUI_CUDA(cudaGetLastError());
   NUI_CUDA(cudaStreamSynchronize(ctx->stream));
   return NUI_OK;
@@ -2204,10 +2211,10 @@ NUI_API nui_status nui_k_feedback_maps(nui_ctx* ctx, const float* d_vertex4, int
                                        const float* pose12, float* d_vref4, float* d_nref4) {
   if (!ctx || !d_vertex4 || !pose12 || !d_vref4 || !d_nref4 || W <= 0 || H <= 0)
     return fail(NUI_ERR_INVALID_ARG, "bad argument");
-  TrackState t;
-  std::memset(&t, 0, sizeof(t));
-  std::memcpy(t.xf.R, pose12, 9 * sizeof(float));
-  std::memcpy(t.xf.t, pose12 + 9, 3 * sizeof(float));
+  DevXform m;
+  std::memset(&m, 0, sizeof(m));
+  std::memcpy(m.R, pose12, 9 * sizeof(float));
+  std::memcpy(m.t, pose12 + 9, 3 * sizeof(float));
   SessionDesc d;
   std::memset(&d, 0, sizeof(d));
   d.kind = kFirstFrame;
@@ -2218,10 +2225,7 @@ NUI_API nui_status nui_k_feedback_maps(nui_ctx* ctx, const float* d_vertex4, int
   d.vlev[0] = (float4*)const_cast<float*>(d_vertex4);
   d.vref = (float4*)d_vref4;
   d.nref = (float4*)d_nref4;
-  d.ts = ctx->d_kts;
-  NUI_CUDA(cudaMemcpyAsync(ctx->d_kts, &t, sizeof(t), cudaMemcpyHostToDevice, ctx->stream));
-  NUI_CUDA(cudaMemcpyAsync(ctx->d_kdesc, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream));
-  k_feedback<<<dim3(cdiv((long)W * H, 256), 1), 256, 0, ctx->stream>>>(ctx->d_kdesc);
+  k_feedback_one<<<dim3(cdiv((long)W * H, 256), 1), 256, 0, ctx->stream>>>(d, m);
   NUI_CUDA(cudaGetLastError());
   NUI_CUDA(cudaStreamSynchronize(ctx->stream));
   return NUI_OK;
@@ -2259,7 +2263,7 @@ nui_status nui_hash_mesh_impl(nui_session* s, float* pos, float* col, uint64_t c
   if (nvis == 0) return NUI_OK;
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
-  NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, st));
+  NUI_CUDA(upload_desc1(s, d));
   if (!s->ctx->hash_mc_tables) hash_mc_upload_tables(st, NUI_MC_TRI_PACKED);
   s->ctx->hash_mc_tables = true;
   DevBuf cnt, off, dp, dc;
@@ -2331,7 +2335,7 @@ nui_status mc_prepare(nui_session* s, DevBuf& cc, DevBuf& bt, uint8_t* d_cases, 
   cudaStream_t st = s->ctx->stream;
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
-  NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, st));
+  NUI_CUDA(upload_desc1(s, d));
   if (!s->ctx->mc_tables) mc_upload_tables(st);
   s->ctx->mc_tables = true;
   const unsigned nb = mc_blocks(c);
@@ -2480,7 +2484,7 @@ extern "C" NUI_API nui_status nui_mesh_device_noalloc(nui_session* s, float* d_p
   cudaStream_t st = s->ctx->stream;
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
-  NUI_CUDA(cudaMemcpyAsync(s->d_desc1, &d, sizeof(d), cudaMemcpyHostToDevice, st));
+  NUI_CUDA(upload_desc1(s, d));
   if (!s->ctx->mc_tables) mc_upload_tables(st);
   s->ctx->mc_tables = true;
   switch (c.tsdf_format) {
