@@ -131,8 +131,7 @@ struct SessionDesc {
   uint8_t* wvol;                  // weight plane of NUI_TSDF_F16_U8
   uchar4* cvol;                   // colour volume (nullable), same layout
   uint8_t* occ;                   // per 8^3 brick state (kBrick*)
-  uint8_t* occ2;                  // per 32^3 super-brick state (kSuper*)
-  uint8_t* occ3;                  // per 128^3 region state (kSuper*, over its super-bricks)
+  uint8_t* dist;                  // per brick: distance to the nearest mixed brick (see kMaxDist)
   int max_cw;
   int zchunks;                    // integration: z chunks per column (one thread each)
   unsigned* fast_tiles;           // tolerance-mode integration: 32 x 8 x 8 tiles kept by the cull (list)
@@ -384,18 +383,15 @@ enum BrickState : uint8_t {
   kBrickDirty = 3,
   kBrickNoNeg = 4
 };
-// States of 32^3-voxel super-bricks (4^3 bricks): all bricks empty; some brick mixed or
-// dirty; every brick empty, positive or no-negative (a march can cross it without a sign
-// change); or awaiting re-classification.  128^3-voxel regions (4^3 super-bricks) use the
-// same states over their super-bricks.
-enum SuperState : uint8_t { kSuperEmpty = 0, kSuperMixed = 1, kSuperSkip = 2, kSuperDirty = 3 };
+// Distance of a brick to the nearest mixed (or dirty) one, in bricks along the farthest axis, 0
+// for a mixed brick and at most kMaxDist: no brick less than that far from it holds a weighted
+// voxel of tsdf <= 0, so a march can cross the cube of 2 d - 1 bricks around it without a sign
+// change.
+constexpr int kMaxDist = 6;
+constexpr int kDistY = 8, kDistZ = 4;  // rows of bricks a block of k_brick_dist takes
 __device__ __forceinline__ size_t occ_index(const SessionDesc& s, int x, int y, int z) {
   const size_t bx = (size_t)(s.res[0] + 7) >> 3, by = (size_t)(s.res[1] + 7) >> 3;
   return (size_t)(x >> 3) + bx * ((size_t)(y >> 3) + by * (size_t)(z >> 3));
-}
-__device__ __forceinline__ size_t occ2_index(const SessionDesc& s, int x, int y, int z) {
-  const size_t sx = (size_t)(s.res[0] + 31) >> 5, sy = (size_t)(s.res[1] + 31) >> 5;
-  return (size_t)(x >> 5) + sx * ((size_t)(y >> 5) + sy * (size_t)(z >> 5));
 }
 // round(p / c) for a voxel coordinate, exactly as the IEEE quotient would round: the
 // product with 1/c is within 2 ulp of the quotient, so unless it lies within 4 ulp of a

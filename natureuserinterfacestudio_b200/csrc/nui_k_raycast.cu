@@ -8,14 +8,12 @@
 // trilinear weights pair the x-neighbour voxel with the y fraction and the y-neighbour
 // with the x fraction, as the reference's index walk does (raycast.cl:66-119).
 //
-// Region skipping (exact): when a sample lands in an 8^3 brick, or a 32^3 super-brick,
-// that holds no weighted voxel with tsdf <= 0, no two consecutive samples inside it can
-// form a transition (each reads NaN or a positive value).  The samples that stay inside
-// the region -- by a margin of 1% of a voxel -- are skipped: the march parameter jumps to
-// the last of them along the exact float sequence t <- t + step (march_advance), and only
-// that sample is read (its value, NaN or positive, is the next "previous" sample).  In an
-// all-empty region, or a brick whose voxels are all weighted and positive, it is known
-// without the read.
+// Region skipping (exact): when a sample lands in a brick d bricks away from any that holds a
+// weighted voxel with tsdf <= 0, no two consecutive samples inside the cube of 2 d - 1 bricks
+// around it can form a transition (each reads NaN or a positive value).  The samples that stay
+// inside the cube -- by a margin of 1% of a voxel -- are skipped: the march parameter jumps to
+// the last of them along the exact float sequence t <- t + step (march_advance), and that
+// sample is read only if the next one lands next to a surface.
 #include "nui_raycast.cuh"
 
 namespace nui {
@@ -119,66 +117,36 @@ __global__ void __launch_bounds__(128) k_raycast(const SessionDesc* __restrict__
     if (V.tsdf_at(gx, gy, gz, f)) tsdf = f;
     const float max_time = 3 * (D0 + D1 + D2);
     const float step = s.trunc * 0.8f;
-    const int sx = (V.rx + 31) >> 5, sy = (V.ry + 31) >> 5;
-    const int hx = (V.rx + 127) >> 7, hy = (V.ry + 127) >> 7;
     const float3 idir = f3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
-    bool pend = false;  // tsdf stands for a skipped sample at tc whose class (NaN or > 0) is unread
+    const RayExit E(start, dir, idir, V.c0, V.c1, V.c2);
+    bool pend = false;  // the sample at tc was skipped and is unread (NaN or > 0)
     float tn = tc;
     while (tc < max_time) {
-      float prev = tsdf;
       tn = tc + step;
       V.voxel_of(add3(start, mul3(dir, tn)), gx, gy, gz);
       if (!(gx >= 0 && gy >= 0 && gz >= 0 && gx < V.rx && gy < V.ry && gz < V.rz)) break;
-      const uint8_t st = V.occ ? __ldg(V.occ + V.bidx(gx, gy, gz)) : (uint8_t)kBrickMixed;
       // only the class of a sample (NaN, < 0, 0, > 0) enters the march decisions
-      if (st == kBrickEmpty) {
-        tsdf = qnan();
-      } else if (st == kBrickPositive) {
+      const int d = __ldg(s.dist + V.bidx(gx, gy, gz));
+      if (d > 0 && !(tsdf < 0.f)) {
+        // no transition at this sample (its value is NaN or > 0 and the previous one is not
+        // negative), nor between any two samples of the cube around the brick: skip to the
+        // last one
+        const float te = E.at(V, gx, gy, gz, d);
+        tc = te <= max_time ? march_advance(tn, step, te) : march_advance_capped(tn, step, te, max_time);
+        pend = true;
         tsdf = 1.0f;
-      } else {
-        tsdf = V.load(V.vidx(gx, gy, gz), f) ? f : qnan();
-      }
-      if ((st == kBrickEmpty || st == kBrickPositive || st == kBrickNoNeg) && (!(prev < 0.f) || isnan(tsdf))) {
-        // no transition at this sample (its value is NaN or > 0 and prev is not negative,
-        // or it is NaN), nor between any two samples of the region: skip to the last one
-        int S = 128;
-        bool uniform;
-        const uint8_t s3 = __ldg(s.occ3 + (gx >> 7) + hx * ((gy >> 7) + hy * (gz >> 7)));
-        if (s3 == kSuperEmpty || s3 == kSuperSkip) {
-          uniform = s3 == kSuperEmpty;
-        } else {
-          const uint8_t s2 = __ldg(s.occ2 + (gx >> 5) + sx * ((gy >> 5) + sy * (gz >> 5)));
-          if (s2 == kSuperEmpty || s2 == kSuperSkip) {
-            S = 32;
-            uniform = s2 == kSuperEmpty;
-          } else {
-            S = 8;
-            uniform = st != kBrickNoNeg;
-          }
-        }
-        const float te = V.region_exit(S, gx, gy, gz, start, dir, idir);
-        const float tl = te <= max_time ? march_advance(tn, step, te) : march_advance_capped(tn, step, te, max_time);
-        if (tl == tn || uniform) {
-          pend = false;  // tsdf is the class of the sample at tl
-        } else {
-          pend = true;
-          tsdf = 1.0f;
-        }
-        tc = tl;
         continue;
       }
+      float prev = tsdf;
+      tsdf = V.load(V.vidx(gx, gy, gz), f) ? f : qnan();
       if (pend) {  // the previous sample was skipped: read its class now
         int lx, ly, lz;
         V.voxel_of(add3(start, mul3(dir, tc)), lx, ly, lz);
-        prev = V.tsdf_at(lx, ly, lz, f) ? f : qnan();
+        prev = V.load(V.vidx(lx, ly, lz), f) ? f : qnan();
         pend = false;
       }
-      if (isnan(tsdf) || isnan(prev)) {
-        tc = tn;
-        continue;
-      }
       if (prev < 0.f && tsdf > 0.f) break;
-      if (prev >= 0.f && tsdf <= 0.f) {
+      if (prev >= 0.f && tsdf <= 0.f) {  // (neither is NaN)
         hit = true;
         break;
       }

@@ -6,8 +6,8 @@
 // the crossing -- with the sample parameters computed directly as t0 + k * step (one
 // rounding each, instead of the reference's running float sum), voxels found by a rounded
 // product with 1 / cell, and empty space skipped by arithmetic on k: a sample that lands in
-// a brick, super-brick or region without a weighted voxel of tsdf <= 0 jumps straight to
-// the last sample inside it.  Depths agree with the reference within the 0.5 mm raycast
+// a brick d bricks away from any with a weighted voxel of tsdf <= 0 jumps straight to the last
+// sample inside the cube of 2 d - 1 bricks around it.  Depths agree with the reference within the 0.5 mm raycast
 // tolerance; the int16 and FP32 formats keep the exact kernels (nui_k_raycast.cu).  This
 // file is compiled with contraction on.
 //
@@ -63,69 +63,37 @@ __global__ void __launch_bounds__(128) k_raycast_fast(const SessionDesc* __restr
       const float max_time = 3 * (D0 + D1 + D2);
       const float step = s.trunc * 0.8f, inv_step = 1.0f / step;
       const int kmax = (int)ceilf((max_time - t0) * inv_step);  // first sample at or past max_time
-      const int sx = (V.rx + 31) >> 5, sy = (V.ry + 31) >> 5;
-      const int hx = (V.rx + 127) >> 7, hy = (V.ry + 127) >> 7;
-      bool pend = false;  // tsdf stands for a skipped sample at kc whose class (NaN or > 0) is unread
+      const RayExit E(start, dir, idir, V.c0, V.c1, V.c2);
+      const float tend = max_time + step;
+      bool pend = false;  // the sample at kc was skipped and is unread (NaN or > 0)
       while (kc < kmax) {
-        float prev = tsdf;
         const int kn = kc + 1;
         const float tn = fmaf((float)kn, step, t0);
         V.voxel_of(add3(start, mul3(dir, tn)), gx, gy, gz);
         // inside the volume on all three axes (one unsigned compare an axis)
         if (!((unsigned)gx < (unsigned)V.rx && (unsigned)gy < (unsigned)V.ry && (unsigned)gz < (unsigned)V.rz)) break;
         ++visited;
-        const uint8_t st = V.occ ? __ldg(V.occ + V.bidx(gx, gy, gz)) : (uint8_t)kBrickMixed;
-        if (st == kBrickEmpty) {
-          tsdf = qnan();
-        } else if (st == kBrickPositive) {
+        const int d = __ldg(s.dist + V.bidx(gx, gy, gz));
+        if (d > 0 && !(tsdf < 0.f)) {
+          // no transition here nor between any two samples of the cube around the brick: on to
+          // the last sample strictly inside it
+          kc = min(max(kn, (int)ceilf((fminf(E.at(V, gx, gy, gz, d), tend) - t0) * inv_step) - 1), kmax);
+          pend = true;
           tsdf = 1.0f;
-        } else {
-          tsdf = V.load(V.vidx(gx, gy, gz), f) ? f : qnan();
-          ++reads;
-        }
-        // empty, positive or no-negative (states 0, 2, 4): a region the march may cross
-        const bool crossable = (0x15u >> st) & 1u;
-        if (crossable && (!(prev < 0.f) || isnan(tsdf))) {
-          int S = 128;
-          bool uniform;
-          const uint8_t s3 = __ldg(s.occ3 + (gx >> 7) + hx * ((gy >> 7) + hy * (gz >> 7)));
-          if (s3 == kSuperEmpty || s3 == kSuperSkip) {
-            uniform = s3 == kSuperEmpty;
-          } else {
-            const uint8_t s2 = __ldg(s.occ2 + (gx >> 5) + sx * ((gy >> 5) + sy * (gz >> 5)));
-            if (s2 == kSuperEmpty || s2 == kSuperSkip) {
-              S = 32;
-              uniform = s2 == kSuperEmpty;
-            } else {
-              S = 8;
-              uniform = st != kBrickNoNeg;
-            }
-          }
-          // the last sample strictly inside the region (its exit carries a 1% voxel margin)
-          const float te = fminf(V.region_exit(S, gx, gy, gz, start, dir, idir), max_time + step);
-          const int kl = min(max(kn, (int)ceilf((te - t0) * inv_step) - 1), kmax);
-          if (kl == kn || uniform) {
-            pend = false;  // tsdf is the class of the sample at kl
-          } else {
-            pend = true;
-            tsdf = 1.0f;
-          }
-          kc = kl;
           continue;
         }
+        float prev = tsdf;
+        tsdf = V.load(V.vidx(gx, gy, gz), f) ? f : qnan();
+        ++reads;
         if (pend) {  // the previous sample was skipped: read its class now
           int lx, ly, lz;
           V.voxel_of(add3(start, mul3(dir, fmaf((float)kc, step, t0))), lx, ly, lz);
-          prev = V.tsdf_at(lx, ly, lz, f) ? f : qnan();
+          prev = V.load(V.vidx(lx, ly, lz), f) ? f : qnan();
           ++reads;
           pend = false;
         }
-        if (isnan(tsdf) || isnan(prev)) {
-          kc = kn;
-          continue;
-        }
         if (prev < 0.f && tsdf > 0.f) break;
-        if (prev >= 0.f && tsdf <= 0.f) {
+        if (prev >= 0.f && tsdf <= 0.f) {  // (neither is NaN)
           hit = true;
           break;
         }

@@ -340,7 +340,6 @@ __global__ void __launch_bounds__(32 * kFastWarps, 3) k_integrate_fast(const Ses
       s.occ[occ_index(s, x, y0, z0)] = st;
       ++bricks;
     }
-    if (lane == 0 && s.occ2) s.occ2[occ2_index(s, x0, y0, z0)] = kSuperDirty;
   }
   const unsigned int t = __reduce_add_sync(0xffffffffu, touched_total);
   const unsigned int b = __reduce_add_sync(0xffffffffu, bricks);

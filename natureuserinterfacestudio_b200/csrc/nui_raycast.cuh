@@ -100,27 +100,33 @@ struct RayVol {
            t011 * (1 - a) * b * c + t100 * a * (1 - b) * (1 - c) + t101 * a * (1 - b) * c +
            t110 * a * b * (1 - c) + t111 * a * b * c;
   }
-  // Largest ray parameter up to which a sample stays (by 1% of a voxel) inside the
-  // p-box of the aligned region of S^3 voxels (S a power of two) holding (gx, gy, gz),
-  // clipped to the volume; samples with parameter below it map to voxels of that region.
-  // The margin also absorbs the rounding of the reciprocal direction used here.
-  __device__ __forceinline__ float region_exit(int S, int gx, int gy, int gz, float3 start, float3 dir,
-                                               float3 idir) const {
-    const int b[3] = {gx & ~(S - 1), gy & ~(S - 1), gz & ~(S - 1)};
-    const int r[3] = {rx, ry, rz};
-    const float c[3] = {c0, c1, c2};
-    const float o[3] = {start.x, start.y, start.z};
-    const float d[3] = {dir.x, dir.y, dir.z};
-    const float id[3] = {idir.x, idir.y, idir.z};
-    float te = 3.4e38f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const float lo = ((float)b[a] - 0.5f + 0.01f) * c[a];
-      const float hi = ((float)min(b[a] + S, r[a]) - 0.5f - 0.01f) * c[a];
-      if (d[a] > 0.f) te = fminf(te, (hi - o[a]) * id[a]);
-      else if (d[a] < 0.f) te = fminf(te, (lo - o[a]) * id[a]);
-    }
-    return te;
+};
+
+// Where a ray leaves the cube of 2 d - 1 bricks around a brick, clipped to the volume: per axis
+// the parameter of a plane of bricks is linear in its voxel index e, a e + b, with the plane
+// moved inwards by 1% of a voxel, which absorbs the rounding, so that samples of a smaller
+// parameter map to voxels of the cube.
+struct RayExit {
+  float ax, ay, az, bx, by, bz;
+  int mx, my, mz;  // +-8: voxels a brick of distance moves the exit plane by
+  __device__ __forceinline__ static void axis(float o, float d, float id, float c, float& a, float& b, int& m) {
+    m = d < 0.f ? -8 : 8;
+    a = d == 0.f ? 0.f : c * id;
+    // leaving upwards: the plane e = (g & ~7) + 8 d; downwards: e + 8 for e = (g & ~7) - 8 d
+    b = d == 0.f ? 3.4e38f : ((d > 0.f ? -0.51f : 7.51f) * c - o) * id;
+  }
+  __device__ __forceinline__ RayExit(float3 o, float3 d, float3 id, float cx, float cy, float cz) {
+    axis(o.x, d.x, id.x, cx, ax, bx, mx);
+    axis(o.y, d.y, id.y, cy, ay, by, my);
+    axis(o.z, d.z, id.z, cz, az, bz, mz);
+  }
+  // e clipped: at most r (only an upward plane can pass it), at least -8 (a downward one at 0)
+  __device__ __forceinline__ static float plane(int g, int m, int d, int r, float a, float b) {
+    return __fmaf_rn((float)max(min((g & ~7) + m * d, r), -8), a, b);
+  }
+  template <class V>
+  __device__ __forceinline__ float at(const V& v, int gx, int gy, int gz, int d) const {
+    return fminf(fminf(plane(gx, mx, d, v.rx, ax, bx), plane(gy, my, d, v.ry, ay, by)), plane(gz, mz, d, v.rz, az, bz));
   }
 };
 

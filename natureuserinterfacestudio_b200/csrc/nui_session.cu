@@ -55,7 +55,7 @@ template <int F>
 __global__ void k_volume_init(const SessionDesc*);
 template <int F>
 __global__ void k_brick_summary(const SessionDesc*, int);
-__global__ void k_super_summary(const SessionDesc*, int);
+__global__ void k_brick_dist(const SessionDesc*, int);
 template <int F>
 __global__ void k_raycast(const SessionDesc*, int);
 template <int F>
@@ -188,7 +188,7 @@ struct BatchPlan {
   int maxIters[kMaxLevels];
   long maxIntegThreads[4];  // per format: columns * zchunks
   long maxBricks[4];        // per format: 8^3 bricks
-  long maxHyper;            // 128^3 regions, all dense formats
+  long maxDistBlocks;       // blocks of the brick distances, all dense formats
   long maxHashBlk;          // scan blocks of 1024 entries
   int hashMask;             // bit per hash sdf format
   int fmtMask;
@@ -261,10 +261,9 @@ struct nui_session {
   uint8_t* wvol = nullptr;
   uchar4* cvol = nullptr;
   uint8_t* occ = nullptr;
-  uint8_t* occ2 = nullptr;
+  uint8_t* dist = nullptr;  // brick distances
   float* ztab = nullptr;
   unsigned* fast_tiles = nullptr;
-  uint8_t* occ3 = nullptr;
   float* tile_max = nullptr;
   TrackState* ts = nullptr;
   uchar4* cprev = nullptr;        // colour tracking: the previous frame's colours and the
@@ -311,6 +310,7 @@ struct nui_session {
 // ------------------------------------------------------------------ helpers
 namespace {
 
+unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 size_t voxel_bytes(int fmt) { return fmt == NUI_TSDF_F32 ? 8 : (fmt == NUI_TSDF_F16_U8 ? 3 : 4); }
 
 bool cfg_valid(const nui_session_cfg* c, std::string& why) {
@@ -421,11 +421,10 @@ void fill_desc(const nui_session* s, SessionDesc& d, int kind, const uint16_t* r
   d.wvol = s->wvol;
   d.cvol = s->cvol;
   d.occ = s->occ;
-  d.occ2 = s->occ2;
+  d.dist = s->dist;
   d.ztab = s->ztab;
   d.tol = c.tsdf_format >= NUI_TSDF_F16_U8 ? 1 : 0;
   d.fast_tiles = s->fast_tiles;
-  d.occ3 = s->occ3;
   d.max_cw = c.max_color_weight;
   d.zchunks = pick_zchunks(s->cfg, s->ctx->tune.integrate_threads_log2);
   d.voxel_shift = s->hash ? 0 : c.voxel_shift;
@@ -515,8 +514,8 @@ void plan_add(BatchPlan& p, const nui_session* s) {
   p.fmtMask |= 1 << c.tsdf_format;
   const long nb = (long)((c.res[0] + 7) / 8) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8);
   p.maxBricks[c.tsdf_format] = std::max(p.maxBricks[c.tsdf_format], nb);
-  const long nh = (long)((c.res[0] + 127) / 128) * ((c.res[1] + 127) / 128) * ((c.res[2] + 127) / 128);
-  p.maxHyper = std::max(p.maxHyper, nh);
+  const long db = (long)cdiv((c.res[1] + 7) / 8, kDistY) * cdiv((c.res[2] + 7) / 8, kDistZ);
+  p.maxDistBlocks = std::max(p.maxDistBlocks, db);
   if (c.voxel_shift > 0) {
     p.shiftFmtMask |= 1 << c.tsdf_format;
     if (c.color_volume) p.shiftColor = 1;
@@ -533,7 +532,7 @@ void plan_merge(BatchPlan& a, const BatchPlan& b) {
     a.maxIntegThreads[f] = std::max(a.maxIntegThreads[f], b.maxIntegThreads[f]);
     a.maxBricks[f] = std::max(a.maxBricks[f], b.maxBricks[f]);
   }
-  a.maxHyper = std::max(a.maxHyper, b.maxHyper);
+  a.maxDistBlocks = std::max(a.maxDistBlocks, b.maxDistBlocks);
   a.maxHashBlk = std::max(a.maxHashBlk, b.maxHashBlk);
   a.hashMask |= b.hashMask;
   a.fmtMask |= b.fmtMask;
@@ -543,7 +542,6 @@ void plan_merge(BatchPlan& a, const BatchPlan& b) {
   a.hashSwap |= b.hashSwap;
 }
 
-unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b); }
 unsigned dense_n(const BatchPlan& p) { return (unsigned)(p.n - p.hashTail); }
 
 
@@ -571,13 +569,18 @@ void launch_summary(const BatchPlan& p, const SessionDesc* d, cudaStream_t st, i
   if (F >= NUI_TSDF_F16_U8 && !force && !(p.shiftFmtMask & (1 << F))) return;
   k_brick_summary<F><<<dim3(cdiv(p.maxBricks[F], kSummaryBricks), dense_n(p)), 256, 0, st>>>(d, force);
 }
-// Brick re-classification after integration, then the super-bricks it touched.
+// The brick distances of the raycasts, from the classified bricks.
+void launch_distances(const BatchPlan& p, const SessionDesc* d, cudaStream_t st, int force) {
+  if (!p.fmtMask) return;
+  k_brick_dist<<<dim3((unsigned)p.maxDistBlocks, dense_n(p)), 128, 0, st>>>(d, force);
+}
+// Brick re-classification after integration, then their distances.
 void launch_summaries(const BatchPlan& p, const SessionDesc* d, cudaStream_t st, int force) {
   launch_summary<0>(p, d, st, force);
   launch_summary<1>(p, d, st, force);
   launch_summary<2>(p, d, st, force);
   launch_summary<3>(p, d, st, force);
-  if (p.fmtMask) k_super_summary<<<dim3((unsigned)p.maxHyper, dense_n(p)), 1024, 0, st>>>(d, force);
+  launch_distances(p, d, st, force);
 }
 // Blocks of the raycasts: 2 x 2 warps, each a tw x (32 / tw) pixel tile.
 unsigned ray_blocks(const BatchPlan& p, int tw) { return cdiv(p.maxW, 2 * tw) * cdiv(p.maxH, 2 * (32 / tw)); }
@@ -1413,9 +1416,7 @@ NUI_API size_t nui_session_device_bytes(const nui_session_cfg* c) {
   if (c->tsdf_format >= NUI_TSDF_F16_U8)  // tolerance-mode tile list
     b += (size_t)((c->res[0] + 31) / 32) * ((c->res[1] + 7) / 8) * ((c->res[2] + 7) / 8) * 4;
   if (c->color_volume) b += nv * 4;
-  b += (size_t)((c->res[0] + 7) / 8) * ((c->res[1] + 7) / 8) * ((c->res[2] + 7) / 8);
-  b += (size_t)((c->res[0] + 31) / 32) * ((c->res[1] + 31) / 32) * ((c->res[2] + 31) / 32);
-  b += (size_t)((c->res[0] + 127) / 128) * ((c->res[1] + 127) / 128) * ((c->res[2] + 127) / 128);
+  b += 2 * (size_t)((c->res[0] + 7) / 8) * ((c->res[1] + 7) / 8) * ((c->res[2] + 7) / 8);
   b += 2 * ((size_t)c->res[2] + 1) * sizeof(float);
   if (c->voxel_shift > 0) b += (size_t)c->shift_point_cap * 28;
   return b;
@@ -1513,9 +1514,7 @@ nui_status session_create(nui_ctx* ctx, const nui_session_cfg* cfg, nui_session*
     if (ok && c.tsdf_format >= NUI_TSDF_F16_U8)
       ok = alloc((void**)&s->fast_tiles, (size_t)((c.res[0] + 31) / 32) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8) * 4);
     const size_t nbricks = (size_t)((c.res[0] + 7) / 8) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8);
-    const size_t nsuper = (size_t)((c.res[0] + 31) / 32) * ((c.res[1] + 31) / 32) * ((c.res[2] + 31) / 32);
-    const size_t nhyper = (size_t)((c.res[0] + 127) / 128) * ((c.res[1] + 127) / 128) * ((c.res[2] + 127) / 128);
-    if (ok) ok = alloc((void**)&s->occ, nbricks) && alloc((void**)&s->occ2, nsuper) && alloc((void**)&s->occ3, nhyper) &&
+    if (ok) ok = alloc((void**)&s->occ, nbricks) && alloc((void**)&s->dist, nbricks) &&
                  alloc((void**)&s->ztab, 2 * ((size_t)c.res[2] + 1) * sizeof(float));
     if (ok && c.color_volume) ok = alloc((void**)&s->cvol, nv * 4) && alloc((void**)&s->bgra, N * 4) && alloc((void**)&s->cmap, N * 4);
   }
@@ -1670,8 +1669,9 @@ std::vector<std::pair<void*, size_t>> state_segments(const nui_session* s) {
     add(s->wvol, nv);
     add(s->cvol, nv * 4);
     add(s->occ, (size_t)((c.res[0] + 7) / 8) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8));
-    add(s->occ2, (size_t)((c.res[0] + 31) / 32) * ((c.res[1] + 31) / 32) * ((c.res[2] + 31) / 32));
-    add(s->occ3, (size_t)((c.res[0] + 127) / 128) * ((c.res[1] + 127) / 128) * ((c.res[2] + 127) / 128));
+    // (snapshots also hold a byte per 32^3 and per 128^3 voxels, not used any more)
+    v.emplace_back(nullptr, (size_t)((c.res[0] + 31) / 32) * ((c.res[1] + 31) / 32) * ((c.res[2] + 31) / 32));
+    v.emplace_back(nullptr, (size_t)((c.res[0] + 127) / 128) * ((c.res[1] + 127) / 128) * ((c.res[2] + 127) / 128));
     add(s->pts_xyz, (size_t)c.shift_point_cap * 12);
     add(s->pts_rgba, (size_t)c.shift_point_cap * 16);
   }
@@ -1709,7 +1709,8 @@ NUI_API nui_status nui_session_snapshot(nui_session* s, void* host, size_t bytes
   std::memcpy(host, &h, sizeof(h));
   char* p = (char*)host + sizeof(h);
   for (auto& seg : state_segments(s)) {
-    NUI_CUDA(cudaMemcpy(p, seg.first, seg.second, cudaMemcpyDefault));
+    if (seg.first) NUI_CUDA(cudaMemcpy(p, seg.first, seg.second, cudaMemcpyDefault));
+    else std::memset(p, 0, seg.second);
     p += seg.second;
   }
   return NUI_OK;
@@ -1728,10 +1729,22 @@ NUI_API nui_status nui_session_restore(nui_session* s, const void* host, size_t 
   NUI_CUDA(cudaStreamSynchronize(s->ctx->stream));
   const char* p = (const char*)host + sizeof(h);
   for (auto& seg : state_segments(s)) {
-    NUI_CUDA(cudaMemcpy(seg.first, p, seg.second, cudaMemcpyDefault));
+    if (seg.first) NUI_CUDA(cudaMemcpy(seg.first, p, seg.second, cudaMemcpyDefault));
     p += seg.second;
   }
   s->frames = h.frames;
+  if (!s->hash) {  // the brick distances follow from the bricks
+    SessionDesc d;
+    fill_desc(s, d, kInactive, nullptr, nullptr);
+    NUI_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the copies above
+    NUI_CUDA(upload_desc1(s, d));
+    BatchPlan p1;
+    p1.n = 1;
+    plan_add(p1, s);
+    launch_distances(p1, s->d_desc1, s->ctx->stream, 1);
+    NUI_CUDA(cudaGetLastError());
+    NUI_CUDA(cudaStreamSynchronize(s->ctx->stream));
+  }
   return NUI_OK;
 }
 
