@@ -790,37 +790,71 @@ struct HashRead {
     const int b = block(vx >> 3, vy >> 3, vz >> 3);
     return b < 0 ? -1 : b + ((vx & 7) + 8 * (vy & 7) + 64 * (vz & 7));
   }
-  // Neighbourhood reads.  Voxels (i + LO .. i + HI) on each axis span at most two blocks
-  // per axis, so at most eight: each is looked up once, by every lane at the same call
-  // site, and a voxel read then selects its block among them.  (Reading each neighbour
-  // through its own lookup sent the lanes of a warp into two dozen separate divergent
-  // calls.)
+  // The eight corners of the cell at (ix, iy, iz), x fastest, 1 where there is no block.  They
+  // lie in one block unless a coordinate is the block's last: only then are neighbours looked
+  // up, and a corner that does not cross an axis is in the block of the corner without it.
+  __device__ __forceinline__ void corners(int ix, int iy, int iz, float (&v)[8]) {
+    const int bx = ix >> 3, by = iy >> 3, bz = iz >> 3, lx = ix & 7, ly = iy & 7, lz = iz & 7;
+    const bool cx = lx == 7, cy = ly == 7, cz = lz == 7;
+    int P[8];
+    P[0] = P[1] = P[2] = P[3] = P[4] = P[5] = P[6] = P[7] = block(bx, by, bz);
+    if (cx || cy || cz) {
+      if (cx) P[1] = block(bx + 1, by, bz);
+      if (cy) P[2] = block(bx, by + 1, bz);
+      P[3] = cy ? P[2] : P[1];
+      if (cx && cy) P[3] = block(bx + 1, by + 1, bz);
+      if (cz) P[4] = block(bx, by, bz + 1);
+      P[5] = cz ? P[4] : P[1];
+      if (cx && cz) P[5] = block(bx + 1, by, bz + 1);
+      P[6] = cz ? P[4] : P[2];
+      if (cy && cz) P[6] = block(bx, by + 1, bz + 1);
+      P[7] = cz ? (cy ? P[6] : P[5]) : P[3];
+      if (cx && cy && cz) P[7] = block(bx + 1, by + 1, bz + 1);
+    }
+    const int x1 = cx ? 0 : lx + 1, y0 = 8 * ly, y1 = cy ? 0 : y0 + 8, z0 = 64 * lz, z1 = cz ? 0 : z0 + 64;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int o = ((k & 1) ? x1 : lx) + ((k & 2) ? y1 : y0) + ((k & 4) ? z1 : z0);
+      v[k] = P[k] < 0 ? 1.0f : HVox<HF>::load(s.hsdf, (unsigned)(P[k] + o));
+    }
+  }
+  // Neighbourhood reads: voxels (i - 1 .. i + 2) on each axis span at most two blocks per axis,
+  // so at most eight: each is looked up once, by every lane at the same call site (reading each
+  // neighbour through its own lookup sent the lanes of a warp into two dozen separate divergent
+  // calls) and its pool offset put into the thread's column of a shared table.  A voxel's block
+  // and its place in it then come from one sum of three per-axis codes: the block's row of the
+  // table (in bytes) above bit 16, the place below it.
   struct Hood {
-    int b0x, b0y, b0z;  // first block on each axis
-    int P[8];           // pool offsets, index (bx - b0x) + 2 (by - b0y) + 4 (bz - b0z); -1: none
+    int x[4], y[4], z[4];  // codes of offsets -1 .. 2
+    const char* P;         // the thread's column; rows kHoodThreads words apart
   };
-  template <int LO, int HI>
-  __device__ __forceinline__ void hood(Hood& h, int ix, int iy, int iz) {
-    h.b0x = (ix + LO) >> 3;
-    h.b0y = (iy + LO) >> 3;
-    h.b0z = (iz + LO) >> 3;
-    const int sx = ((ix + HI) >> 3) - h.b0x, sy = ((iy + HI) >> 3) - h.b0y, sz = ((iz + HI) >> 3) - h.b0z;
+  static constexpr int kHoodThreads = 256;
+  __device__ __forceinline__ void hood(Hood& h, int (*table)[kHoodThreads], int ix, int iy, int iz) {
+    const int bx = (ix - 1) >> 3, by = (iy - 1) >> 3, bz = (iz - 1) >> 3;
+    const int sx = ((ix + 2) >> 3) - bx, sy = ((iy + 2) >> 3) - by, sz = ((iz + 2) >> 3) - bz;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int ox = k & 1, oy = (k >> 1) & 1, oz = k >> 2;
-      h.P[k] = (ox <= sx && oy <= sy && oz <= sz) ? block(h.b0x + ox, h.b0y + oy, h.b0z + oz) : -1;
+      table[k][threadIdx.x] = (ox <= sx && oy <= sy && oz <= sz) ? block(bx + ox, by + oy, bz + oz) : -1;
     }
-  }
-  // pool index of voxel (x, y, z) of the neighbourhood, or -1 if its block is not allocated
-  __device__ __forceinline__ int hood_index(const Hood& h, int x, int y, int z) const {
-    const int sel = ((x >> 3) - h.b0x) + 2 * ((y >> 3) - h.b0y) + 4 * ((z >> 3) - h.b0z);
-    int b = h.P[0];
+    constexpr int kRow = (kHoodThreads * 4) << 16;
 #pragma unroll
-    for (int k = 1; k < 8; ++k) b = sel == k ? h.P[k] : b;
-    return b < 0 ? -1 : b + (x & 7) + 8 * (y & 7) + 64 * (z & 7);
+    for (int o = 0; o < 4; ++o) {
+      const int X = ix - 1 + o, Y = iy - 1 + o, Z = iz - 1 + o;
+      h.x[o] = (X & 7) + ((X >> 3) - bx) * kRow;
+      h.y[o] = 8 * (Y & 7) + ((Y >> 3) - by) * 2 * kRow;
+      h.z[o] = 64 * (Z & 7) + ((Z >> 3) - bz) * 4 * kRow;
+    }
+    h.P = reinterpret_cast<const char*>(&table[0][threadIdx.x]);
   }
-  __device__ __forceinline__ float hood_sdf(const Hood& h, int x, int y, int z) const {
-    const int bi = hood_index(h, x, y, z);
+  // pool index of the voxel at offsets (dx, dy, dz) in -1 .. 2, or -1 if its block is not allocated
+  __device__ __forceinline__ int hood_index(const Hood& h, int dx, int dy, int dz) const {
+    const int c = h.x[dx + 1] + h.y[dy + 1] + h.z[dz + 1];
+    const int b = *reinterpret_cast<const int*>(h.P + (c >> 16));
+    return b < 0 ? -1 : b + (c & 0xffff);
+  }
+  __device__ __forceinline__ float hood_sdf(const Hood& h, int dx, int dy, int dz) const {
+    const int bi = hood_index(h, dx, dy, dz);
     return bi < 0 ? 1.0f : HVox<HF>::load(s.hsdf, (unsigned)bi);
   }
 };
@@ -830,40 +864,44 @@ struct HashRead {
 // values read are those of the reference's per-voxel findVoxelBlockIndex.
 
 // The march of castRay (KinfuHashRaycast.cl:170-232) from (pr, total) until a surface
-// (sdf <= 0) or the end of the range.
+// (sdf <= 0) or the end of the range.  The lanes of a warp step through free space first, each
+// until its sample lies in the interpolation band, and then interpolate together (a lane's
+// steps are the same either way; interpolating as each lane came to it left 11 of 32 lanes
+// working an instruction).
 template <int HF>
 __device__ __forceinline__ void hash_march(HashRead<HF>& R, const SessionDesc& s, float3& pr, float& total,
                                            const float totalMax, const float3 dir, const float stepScale, float& sdfv) {
-  float stepLen;
   while (total < totalMax) {
-    const int vx = (int)roundf(pr.x), vy = (int)roundf(pr.y), vz = (int)roundf(pr.z);
-    const int bi = R.find(vx, vy, vz);
-    if (bi < 0) {
-      sdfv = 1.0f;
-      stepLen = 8.0f;
-    } else {
-      sdfv = HVox<HF>::load(s.hsdf, (unsigned)bi);
-      if (sdfv <= 0.1f && sdfv >= -0.5f) {
-        const int ix = (int)floorf(pr.x), iy = (int)floorf(pr.y), iz = (int)floorf(pr.z);
-        const float3 cf = f3(pr.x - (float)ix, pr.y - (float)iy, pr.z - (float)iz);
-        typename HashRead<HF>::Hood h;
-        R.template hood<0, 1>(h, ix, iy, iz);
-        float v1 = R.hood_sdf(h, ix, iy, iz), v2 = R.hood_sdf(h, ix + 1, iy, iz);
-        float r1 = (1.0f - cf.x) * v1 + cf.x * v2;
-        v1 = R.hood_sdf(h, ix, iy + 1, iz);
-        v2 = R.hood_sdf(h, ix + 1, iy + 1, iz);
-        r1 = (1.0f - cf.y) * r1 + cf.y * ((1.0f - cf.x) * v1 + cf.x * v2);
-        v1 = R.hood_sdf(h, ix, iy, iz + 1);
-        v2 = R.hood_sdf(h, ix + 1, iy, iz + 1);
-        float r2 = (1.0f - cf.x) * v1 + cf.x * v2;
-        v1 = R.hood_sdf(h, ix, iy + 1, iz + 1);
-        v2 = R.hood_sdf(h, ix + 1, iy + 1, iz + 1);
-        r2 = (1.0f - cf.y) * r2 + cf.y * ((1.0f - cf.x) * v1 + cf.x * v2);
-        sdfv = (1.0f - cf.z) * r1 + cf.z * r2;
+    bool band = false;
+    while (total < totalMax) {
+      const int vx = (int)roundf(pr.x), vy = (int)roundf(pr.y), vz = (int)roundf(pr.z);
+      const int bi = R.find(vx, vy, vz);
+      float stepLen;
+      if (bi < 0) {
+        sdfv = 1.0f;
+        stepLen = 8.0f;
+      } else {
+        sdfv = HVox<HF>::load(s.hsdf, (unsigned)bi);
+        band = sdfv <= 0.1f && sdfv >= -0.5f;
+        if (band) break;
+        if (sdfv <= 0.0f) return;
+        stepLen = fmaxf(sdfv * stepScale, 1.0f);
       }
-      if (sdfv <= 0.0f) return;
-      stepLen = fmaxf(sdfv * stepScale, 1.0f);
+      pr = add3(pr, mul3(dir, stepLen));
+      total += stepLen;
     }
+    if (!band) return;
+    const int ix = (int)floorf(pr.x), iy = (int)floorf(pr.y), iz = (int)floorf(pr.z);
+    const float3 cf = f3(pr.x - (float)ix, pr.y - (float)iy, pr.z - (float)iz);
+    float v[8];
+    R.corners(ix, iy, iz, v);
+    float r1 = (1.0f - cf.x) * v[0] + cf.x * v[1];
+    r1 = (1.0f - cf.y) * r1 + cf.y * ((1.0f - cf.x) * v[2] + cf.x * v[3]);
+    float r2 = (1.0f - cf.x) * v[4] + cf.x * v[5];
+    r2 = (1.0f - cf.y) * r2 + cf.y * ((1.0f - cf.x) * v[6] + cf.x * v[7]);
+    sdfv = (1.0f - cf.z) * r1 + cf.z * r2;
+    if (sdfv <= 0.0f) return;
+    const float stepLen = fmaxf(sdfv * stepScale, 1.0f);
     pr = add3(pr, mul3(dir, stepLen));
     total += stepLen;
   }
@@ -904,12 +942,13 @@ __device__ __forceinline__ void hash_finish(HashRead<HF>& R, const SessionDesc& 
     float fb[8];
     float nearest = 1.0e20f;
     // one neighbourhood for the corners and the gradient's outer samples
+    __shared__ int table[8][HashRead<HF>::kHoodThreads];
     typename HashRead<HF>::Hood h;
-    R.template hood<-1, 2>(h, ix, iy, iz);
+    R.hood(h, table, ix, iy, iz);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int ox = k & 1, oy = (k >> 1) & 1, oz = (k >> 2) & 1;
-      const int bi = R.hood_index(h, ix + ox, iy + oy, iz + oz);
+      const int bi = R.hood_index(h, ox, oy, oz);
       fb[k] = bi < 0 ? 1.0f : HVox<HF>::load(s.hsdf, (unsigned)bi);
       const float3 dd = f3(ox ? nc.x : cf.x, oy ? nc.y : cf.y, oz ? nc.z : cf.z);
       const float cd = sqrtf(dot3(dd, dd));
@@ -931,7 +970,7 @@ __device__ __forceinline__ void hash_finish(HashRead<HF>& R, const SessionDesc& 
       return;
     }
     float p1, p2, v1;
-    auto nr = [&](int dx, int dy, int dz) { return R.hood_sdf(h, ix + dx, iy + dy, iz + dz); };
+    auto nr = [&](int dx, int dy, int dz) { return R.hood_sdf(h, dx, dy, dz); };
     float3 g;
     p1 = fb[0] * nc.y * nc.z + fb[2] * cf.y * nc.z + fb[4] * nc.y * cf.z + fb[6] * cf.y * cf.z;
     p2 = nr(-1, 0, 0) * nc.y * nc.z + nr(-1, +1, 0) * cf.y * nc.z +
