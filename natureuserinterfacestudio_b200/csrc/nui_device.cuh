@@ -21,7 +21,6 @@ constexpr int kIcpHalf = 144;                       // floats from the first arr
 constexpr int kIcpStageBytes = (kIcpHalf + 128) * 4;  // per warp (also holds its 64 sums)
 constexpr int kSummaryBricks = 32;  // bricks a block of k_brick_summary looks at
 constexpr int kFastWarps = 4;  // warps per block of the tolerance-mode integration
-constexpr int kFastWarpSmem = 64 * 32 * 4 + 64 * 32 * 4;  // its shared memory per warp (bytes)
 
 // Camera intrinsics block (gpu_def.h:13-27).
 struct DevCam {

@@ -552,11 +552,10 @@ void launch_integrate(const BatchPlan& p, const SessionDesc* d, cudaStream_t st)
   if (F >= NUI_TSDF_F16_U8) {  // tolerance mode: cull the 32 x 8 x 8 tiles, then a warp per kept tile
     const long tiles = p.maxBricks[F] / 4 + 1;  // >= the tiles of any session of the format
     k_integrate_cull<F><<<dim3(cdiv(tiles, 256), dense_n(p)), 256, 0, st>>>(d);
-    const long blocks = std::min<long>(cdiv(tiles, 32 * kFastWarps), 1024);
-    const int smem = kFastWarps * kFastWarpSmem;
-    static std::once_flag opt_in;  // more than 48 KB of dynamic shared memory a block
-    std::call_once(opt_in, [&] { cudaFuncSetAttribute(k_integrate_fast<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
-    k_integrate_fast<F><<<dim3((unsigned)std::max<long>(blocks, 1), dense_n(p)), 32 * kFastWarps, smem, st>>>(d);
+    // a block a tile: enough blocks that one session's kept tiles (~2000 of a 512^3 volume's
+    // 65536) spread over the SMs, no more than a few per SM of each of many
+    const long blocks = std::min<long>(cdiv(tiles, 16), std::max<long>(128, 2368 / dense_n(p)));
+    k_integrate_fast<F><<<dim3((unsigned)std::max<long>(blocks, 1), dense_n(p)), 32 * kFastWarps, 0, st>>>(d);
     return;
   }
   k_integrate<F><<<dim3(cdiv(p.maxIntegThreads[F], 256), dense_n(p)), 256, 0, st>>>(d);

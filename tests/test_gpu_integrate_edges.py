@@ -1,0 +1,61 @@
+"""Tolerance-mode integration where its tiles (32 x 8 x 8 voxels, two z slices a warp) can go
+wrong: single tiles, x sizes whose rows are not whole or not 16-byte aligned, y and z remainders
+that leave a warp one slice or none, several sessions of unlike sizes in one launch."""
+import numpy as np
+import pytest
+
+from natureuserinterfacestudio_b200 import _lib as L
+from oracle import oracle as O
+
+from _util import cfg_for, frames, integration_near_ties, oracle_preprocess
+from test_gpu_parity import _brick_states
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(32, 8, 8), (33, 9, 9), (40, 17, 15), (48, 8, 10), (80, 23, 11), (96, 40, 29), (130, 64, 63)]
+
+
+@pytest.mark.parametrize("fmt", [L.TSDF_F16_U8, L.TSDF_F16_F16])
+@pytest.mark.parametrize("res", SIZES)
+def test_edges_of_tiles(gpu_ctx, res, fmt):
+    """Tolerance: that of the larger volumes' comparison with the oracle -- 1e-3 truncation units
+    (half precision rounds to 2.4e-4 near 1) and equal weights outside near ties; brick states
+    exactly those of the voxels; nothing written outside the volume's voxels (the planes end with
+    the volume, so the last brick's states would show it)."""
+    W, H = 96, 72
+    seq = frames(3, W=W, H=H, seed=4)
+    cfg, ref = (cfg_for(W=W, H=H, res=res, fmt=f, trunc=0.2) for f in (fmt, L.TSDF_I16))
+    eng = O.Engine(ref)
+    s = L.Session(gpu_ctx, cfg)
+    exact = L.Session(gpu_ctx, ref)  # the exact kernel of the int16 format, at the same poses
+    amb = np.zeros(res[0] * res[1] * res[2], bool)
+    for i, (d, _, R, t) in enumerate(seq):
+        amb |= integration_near_ties(ref, eng.tsdf, R, t, oracle_preprocess(d, ref)["scaled"], eps_px=3e-3)
+        for k in (s, exact):
+            k.upload(d)
+            k.set_pose(R, t)
+            k.integrate()
+        vg, vo = s.volume_ref_layout().astype(np.float64), exact.volume_ref_layout().astype(np.float64)
+        bad = vg[:, 1] != vo[:, 1]
+        both = (vg[:, 1] > 0) & (vo[:, 1] > 0)
+        bad |= both & (np.abs(vg[:, 0] - vo[:, 0]) / 32766.0 > 1e-3)
+        assert not np.any(bad & ~amb), (i, int(np.sum(bad & ~amb)), int(np.sum(bad)))
+        assert exact.touched() > 0 and np.array_equal(s.download(13), _brick_states(s, res)), i
+    s.close()
+    exact.close()
+
+
+def test_unlike_sizes_in_one_launch(gpu_ctx):
+    """Each session of a batch integrates what it does alone, bit for bit (the roundings of a
+    voxel do not depend on the split)."""
+    W, H = 96, 72
+    seq = frames(3, W=W, H=H, seed=4)
+    cfgs = [cfg_for(W=W, H=H, res=r, fmt=L.TSDF_F16_U8, trunc=0.2) for r in SIZES]
+    solo, both = ([L.Session(gpu_ctx, c) for c in cfgs] for _ in range(2))
+    for i, (d, _, _, _) in enumerate(seq):
+        for s in solo:
+            s.process(d)
+        gpu_ctx.batch_tick(both, [d] * len(both))
+        for a, b, r in zip(solo, both, SIZES):
+            assert np.array_equal(a.download(6).view(np.uint16), b.download(6).view(np.uint16)), (i, r)
+            assert np.array_equal(a.download(14), b.download(14)) and np.array_equal(a.download(13), b.download(13)), (i, r)
