@@ -696,8 +696,9 @@ __global__ void __launch_bounds__(256, COLOR ? 2 : 4)
   if (s.kind != kTrackFrame || !in_family(s, fam) || !(s.photo_w > 0.f || wide == 2) || iter >= s.iters[0]) return;
   TrackState* ts = s.ts;
   IcpFinest& f = work[blockIdx.y];
-  // the first iteration starts from the coarser levels' estimate
-  if (iter == 0 ? ts->status != 0 : (f.lm.status != 0 || f.lm.level_done != 0)) return;
+  // the first iteration starts from the coarser levels' estimate; a session that lost tracking
+  // there has no state in f (which holds what another frame left)
+  if (ts->status != 0 || (iter > 0 && (f.lm.status != 0 || f.lm.level_done != 0))) return;
   extern __shared__ __align__(16) float icp_stage[];
   __shared__ IcpPoses P;
   __shared__ double sums[kIcpTerms];

@@ -42,6 +42,26 @@ def test_one_session_and_many_agree(gpu_ctx, W, H, color):
         s.close()
 
 
+@pytest.mark.gpu
+def test_lost_at_a_coarse_level_stays_lost(gpu_ctx):
+    """A frame that loses tracking in the clusters' levels does not go on at level 0 from what
+    an earlier frame (of another session) left in the whole-device route's workspace: the flat
+    wall of test_gpu_lost after a frame whose single iteration ends level 0 undone."""
+    W = H = 512
+    other = L.Session(gpu_ctx, cfg_for(W=W, H=H, res=(64, 64, 64), trunc=0.1, iters=(1, 0, 0)))
+    wall = L.Session(gpu_ctx, cfg_for(W=W, H=H, res=(64, 64, 64)))
+    flat = np.full((H, W), 1500, np.uint16)
+    ok, first = wall.process(flat)
+    assert ok
+    for d, _, _, _ in frames(3, W=W, H=H, seed=5, deg=4.0):
+        assert other.process(d)[0]
+        ok, p = wall.process(flat)
+        assert not ok and np.array_equal(p, first)
+        assert wall.work_counters()["icp_iters"][:3] == [0, 0, 1]  # lost by the first iteration of the coarsest level
+    for s in (other, wall):
+        s.close()
+
+
 def _f32(x):
     """The float32 nearest to a rational (ties to even), as a Fraction; normal range."""
     if x == 0:
