@@ -79,15 +79,15 @@ struct IcpLm {
   unsigned icp_iters[kMaxLevels];
 };
 
-// Level 0 of one session spread over many blocks (k_icp_finest): the blocks' sums (depth in
-// 0..28, photometric in 32..60), the tracker state from iteration to iteration, and the
-// blocks that have finished the current one (zero between launches).
-constexpr int kIcpWideBlocks = 320;  // blocks a session, at most
+// The ICP of one session over many blocks (k_icp_wide): the blocks' sums (depth in 0..28,
+// photometric in 32..60) of an even and an odd iteration, the blocks' arrivals in the iterations
+// and the blocks that have left (zero between launches), and whether a wait ran out.
+constexpr int kIcpWideBlocks = 160;  // blocks a session, at most
 constexpr int kIcpWideSessions = 4;  // sessions a launch, at most
-struct IcpFinest {
-  double part[kIcpWideBlocks][64];
-  IcpLm lm;
-  unsigned done;
+constexpr int kIcpPolls = 1 << 21;   // polls of the arrivals a block makes (each ~0.4 us)
+struct IcpWide {
+  double part[2][kIcpWideBlocks][64];
+  unsigned arrived, left, stalled;
 };
 
 // What one session does in the current tick (host-written, read by every kernel).

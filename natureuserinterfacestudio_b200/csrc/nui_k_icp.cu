@@ -125,21 +125,25 @@ __device__ __forceinline__ bool color_row(const SessionDesc& s, int i, const flo
 }
 
 // ---------------------------------------------------------------- FP64 host step
-// The 6x6 algebra of the host step runs on one thread at the end of every ICP launch, so
-// its latency is the launch's tail: every loop below is unrolled with constant indices,
-// which keeps the matrices in registers (no local-memory round trips).
+// The 6x6 algebra of the host step runs at the end of every iteration, while all other blocks
+// wait, so its latency counts: the rows are spread over the lanes of a warp, so that the
+// quotients of a column form at once, and every value still comes from the same operations in
+// the same order as in a serial elimination.
 
 // Determinant by Gaussian elimination with partial pivoting (the first row holding the
-// largest |entry| of the column); destroys A.
-__device__ __forceinline__ double det6(double (&A)[6][6]) {
+// largest |entry| of the column): lane r < 6 holds row r. Called by a whole warp; every lane
+// gets the result.
+__device__ __forceinline__ double det6(double (&a)[6]) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
   double det = 1.0;
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
     int piv = c;
-    double best = fabs(A[c][c]);
+    double best = fabs(__shfl_sync(full, a[c], c));
 #pragma unroll
     for (int r = c + 1; r < 6; ++r) {
-      const double v = fabs(A[r][c]);
+      const double v = fabs(__shfl_sync(full, a[c], r));
       if (v > best) {
         best = v;
         piv = r;
@@ -147,62 +151,46 @@ __device__ __forceinline__ double det6(double (&A)[6][6]) {
     }
     if (best == 0.0) return 0.0;
     if (piv != c) {
+      const int src = lane == c ? piv : lane == piv ? c : lane;
 #pragma unroll
-      for (int r = c + 1; r < 6; ++r)
-        if (piv == r) {
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            const double t = A[c][k];
-            A[c][k] = A[r][k];
-            A[r][k] = t;
-          }
-        }
+      for (int k = c; k < 6; ++k) a[k] = __shfl_sync(full, a[k], src);
       det = -det;
     }
-    det *= A[c][c];
+    const double p = __shfl_sync(full, a[c], c);
+    det *= p;
+    const double f = a[c] / p;
 #pragma unroll
-    for (int r = c + 1; r < 6; ++r) {
-      const double f = A[r][c] / A[c][c];
-#pragma unroll
-      for (int k = c; k < 6; ++k) A[r][k] -= f * A[c][k];
+    for (int k = c + 1; k < 6; ++k) {
+      const double q = __shfl_sync(full, a[k], c);
+      if (lane > c) a[k] -= f * q;
     }
   }
   return det;
 }
 
 // Cholesky factorisation A = L L^T and the two triangular solves; false if a pivot is not
-// positive.
-__device__ __forceinline__ bool llt_solve6(const double (&A)[6][6], const double (&b)[6], double (&x)[6]) {
-  double L[6][6];
+// positive.  Lane i < 6 holds row i of A, lane 6 the right-hand side, which goes through the
+// factorisation as a seventh row (the forward substitution). Called by a whole warp; every lane
+// gets x.
+__device__ __forceinline__ bool llt_solve6(double (&a)[6], double (&x)[6]) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  double diag[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
-    double s = A[j][j];
+    const double d = __shfl_sync(full, a[j], j);
+    if (!(d > 0.0)) return false;
+    diag[j] = sqrt(d);
+    a[j] = a[j] / diag[j];  // L[i][j] below the diagonal
 #pragma unroll
-    for (int k = 0; k < j; ++k) s -= L[j][k] * L[j][k];
-    if (!(s > 0.0)) return false;
-    L[j][j] = sqrt(s);
-#pragma unroll
-    for (int i = j + 1; i < 6; ++i) {
-      double t = A[i][j];
-#pragma unroll
-      for (int k = 0; k < j; ++k) t -= L[i][k] * L[j][k];
-      L[i][j] = t / L[j][j];
-    }
-  }
-  double y[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    double t = b[i];
-#pragma unroll
-    for (int k = 0; k < i; ++k) t -= L[i][k] * y[k];
-    y[i] = t / L[i][i];
+    for (int k = j + 1; k < 6; ++k) a[k] -= a[j] * __shfl_sync(full, a[j], k);
   }
 #pragma unroll
   for (int i = 5; i >= 0; --i) {
-    double t = y[i];
+    double t = __shfl_sync(full, a[i], 6);
 #pragma unroll
-    for (int k = i + 1; k < 6; ++k) t -= L[k][i] * x[k];
-    x[i] = t / L[i][i];
+    for (int k = i + 1; k < 6; ++k) t -= __shfl_sync(full, a[i], k) * x[k];
+    x[i] = t / diag[i];
   }
   return true;
 }
@@ -255,91 +243,84 @@ __device__ __forceinline__ void lm_copy(T* d, const U* s) {
   }
 }
 
-// The LM step on the reduced sums (NuiKinfuOpenCLDepthTracker.cpp:324-496), spread over
-// the threads of the cluster's first block in phases separated by block barriers: the
-// bookkeeping on one thread, the 27 normalised sums on 27 threads, the Cholesky solve and
-// the determinant on two threads of different warps at once, the increments' sines and
-// cosines on three threads, the composition on one.  Every value comes from the same FP64
-// operations in the same order as a one-thread step; only their latencies overlap (one
-// thread took ~8 us per iteration, while the cluster's other blocks waited).  The block's
-// first two warps call it and its barriers are theirs alone (a block has up to 32 warps).
+// The LM step on the reduced sums (NuiKinfuOpenCLDepthTracker.cpp:324-496) by a block's first
+// two warps, in phases separated by barriers of theirs alone: accept or reject and the 27
+// normalised sums a thread each, the Cholesky solve and the determinant on a warp each, the
+// increments' sines and cosines on three threads, the composition on one.  Every value comes
+// from the same FP64 operations in the same order as a one-thread step, which took 8 us (4.5
+// with the solve and the determinant on a thread each; 3.9 now).
 struct IcpStepScratch {
   double A[6][6], b[6], x[6], det, sc[6];
-  float cnt;
   int go, solved;
 };
 __device__ __forceinline__ void icp_step_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+// Term t of the 29 among a warp's 64 sums: (i, j) of the upper triangle of [row, 1] by rows,
+// at 8 i + j; then r^2 (6, 6) and the count (7, 7).
+__device__ __forceinline__ int icp_term_at(int t) {
+  if (t >= 27) return t == 27 ? 54 : 63;
+  int i = 0, j = t;
+  while (j >= 7 - i) j -= 7 - i, ++i;
+  return 8 * i + i + j;
+}
 __device__ __noinline__ void icp_host_step(IcpLm* ts, IcpStepScratch& w, const double* sums, int iter,
                                               unsigned min_count) {
   const int tid = threadIdx.x;
-  if (tid == 0) {  // bookkeeping: error, LM accept / reject
-    float err = (float)sums[27];
-    const float cnt = (float)sums[28];
-    err = (cnt > 0.f) ? sqrtf(err) / cnt : 3.402823466e+38f;
+  // accept or reject (every thread, alike)
+  float err = (float)sums[27];
+  const float cnt = (float)sums[28];
+  err = (cnt > 0.f) ? sqrtf(err) / cnt : 3.402823466e+38f;
+  // level start: lambda = 1, Rgood = Rcurr, errorOld = 1e20
+  const float err_old = iter == 0 ? 1e20f : ts->err_old, l0 = iter == 0 ? 1.0f : ts->lambda;
+  const bool reject = cnt < (float)min_count || err > err_old;
+  const float lambda = reject ? l0 * 10.0f : l0 / 10.0f;
+  double v = 0.0;
+  if (tid < 27) v = reject ? ts->good[tid] : sums[tid];
+  icp_step_sync();  // (the state has been read)
+  if (tid == 0) {
     ts->error = err;
     ts->count = cnt;
     ts->iterations_run += 1;
-    w.cnt = cnt;
+    ts->lambda = lambda;
+    ts->err_old = reject ? err_old : err;
+    if (iter == 0) ts->level_done = reject ? 1 : 0;
     w.go = 1;
-    if (iter == 0) {  // level start: lambda = 1, Rgood = Rcurr, errorOld = 1e20
-      ts->lambda = 1.0f;
-      for (int i = 0; i < 9; ++i) ts->Rg[i] = ts->R[i];
-      for (int i = 0; i < 3; ++i) ts->tg[i] = ts->t[i];
-      ts->err_old = 1e20f;
-      ts->level_done = 0;
-    }
-    if (cnt < (float)min_count || err > ts->err_old) {
-      ts->lambda *= 10.0f;
-      for (int i = 0; i < 9; ++i) ts->R[i] = ts->Rg[i];
-      for (int i = 0; i < 3; ++i) ts->t[i] = ts->tg[i];
-      if (iter == 0) {
-        ts->level_done = 1;
-        w.go = 0;
-      }
-    } else {
-      ts->lambda /= 10.0f;
-      for (int i = 0; i < 9; ++i) ts->Rg[i] = ts->R[i];
-      for (int i = 0; i < 3; ++i) ts->tg[i] = ts->t[i];
-      ts->err_old = err;
-      for (int k = 0; k < 27; ++k) ts->good[k] = sums[k];
-    }
   }
-  icp_step_sync();
-  if (!w.go) return;
+  if (tid >= 32 && tid < 44) {  // back to the last good pose, or this one is good
+    const int k = tid - 32;
+    float *c = k < 9 ? ts->R + k : ts->t + k - 9, *g = k < 9 ? ts->Rg + k : ts->tg + k - 9;
+    if (reject && iter > 0) *c = *g;
+    else *g = *c;
+  }
+  if (reject && iter == 0) return;
   if (tid < 27) {  // sum sh = (i, j) of the upper triangle of [J|r] by rows, over the count
-    int i = 0, j = tid;
-    while (j >= 7 - i) j -= 7 - i, ++i;
-    j += i;
-    double v = ts->good[tid] / (double)w.cnt;
+    if (!reject) ts->good[tid] = v;
+    const int at = icp_term_at(tid), i = at >> 3, j = at & 7;
+    v = v / (double)cnt;
     if (j == 6) {
       w.b[i] = v;
     } else {
-      if (i == j) v *= (double)(1.0f + ts->lambda);
+      if (i == j) v *= (double)(1.0f + lambda);
       w.A[i][j] = v;
       w.A[j][i] = v;
     }
   }
   icp_step_sync();
-  // a singular system (|det| < 1e-15 or NaN) or a failed factorisation loses tracking; the
-  // determinant's elimination works on a copy
-  if (tid == 0) {
-    double A[6][6], b[6], x[6];
+  // a singular system (|det| < 1e-15 or NaN) or a failed factorisation loses tracking
+  double a[6];
+  const int row = min(tid & 31, 6);
 #pragma unroll
-    for (int r = 0; r < 6; ++r) {
-      b[r] = w.b[r];
+  for (int k = 0; k < 6; ++k) a[k] = row < 6 ? w.A[row][k] : w.b[k];
+  if (tid < 32) {
+    double x[6];
+    const bool solved = llt_solve6(a, x);
+    if (tid == 0) {
+      w.solved = solved ? 1 : 0;
 #pragma unroll
-      for (int c = 0; c < 6; ++c) A[r][c] = w.A[r][c];
+      for (int r = 0; r < 6; ++r) w.x[r] = x[r];
     }
-    w.solved = llt_solve6(A, b, x) ? 1 : 0;
-#pragma unroll
-    for (int r = 0; r < 6; ++r) w.x[r] = x[r];
-  } else if (tid == 32) {
-    double A[6][6];
-#pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-      for (int c = 0; c < 6; ++c) A[r][c] = w.A[r][c];
-    w.det = det6(A);
+  } else {
+    const double det = det6(a);
+    if (tid == 32) w.det = det;
   }
   icp_step_sync();
   if (tid == 0) {
@@ -452,8 +433,13 @@ __device__ __forceinline__ bool icp_depth_row(const IcpView& c, int x, int y, fl
   return true;
 }
 
-// The depth rows of the level's pixels that fall to this block (runs of blockDim.x x per
-// pixels: runs rank, rank + C, ...), their outer products added to the warp's 8 x 8 FP64
+// How a level's pixels are dealt: runs of T x per pixels, of which this thread's part (a block
+// or a warp of T threads, thread `tid` of it) takes run `rank`, rank + C, ...
+struct IcpDeal {
+  int T, tid, per, rank, C;
+};
+
+// The depth rows of the level's pixels that fall to this thread's part, their outer products added to the warp's 8 x 8 FP64
 // sums (d0, d1: this lane's two of them).  The 29 sums of a pixel are the upper triangle of
 // the outer product of [row, 1]: JtJ, Jtr, r^2 and the count.  The rows' FP32 values are
 // widened, so every product is exact and only the sums round.
@@ -462,12 +448,12 @@ __device__ __forceinline__ bool icp_depth_row(const IcpView& c, int x, int y, fl
 // of 29 a thread (58 registers), which lets 1024 threads of 64 registers share an SM instead of
 // 512 of 128, so twice the warps wait at once (track at 640 x 480: 337 -> 281 us; 39 sessions:
 // 164 -> 147 M warp instructions a launch).
-__device__ __forceinline__ void icp_depth_pass(const SessionDesc& s, int level, int per, int rank, int C,
+__device__ __forceinline__ void icp_depth_pass(const SessionDesc& s, int level, const IcpDeal& deal,
                                                const IcpPoses& P, float* stage, double& d0, double& d1) {
   const IcpView view(s, level);
   const int w = s.W >> level, n = w * (s.H >> level);
   const float* __restrict__ Dl = s.dlev[level];
-  const int T = (int)blockDim.x, lane = threadIdx.x & 31;
+  const int T = deal.T, per = deal.per, C = deal.C, lane = threadIdx.x & 31;
   const int c = lane >> 2, src = (lane & 3) * 4 + (c < 4 ? c : kIcpHalf + c - 4);
   float4* const sa = reinterpret_cast<float4*>(stage) + lane;
   float4* const sb = reinterpret_cast<float4*>(stage + kIcpHalf) + lane;
@@ -475,8 +461,8 @@ __device__ __forceinline__ void icp_depth_pass(const SessionDesc& s, int level, 
   // and row advance with its index, by T within a run and by the rest of the other blocks'
   // runs after it
   const int jump = T * ((C - 1) * per + 1), ty = T / w, tx = T - ty * w, jy = jump / w, jx = jump - jy * w;
-  int base = rank * T * per, k = 0;
-  int i = base + (int)threadIdx.x, y = i / w, x = i - y * w;
+  int base = deal.rank * T * per, k = 0;
+  int i = base + deal.tid, y = i / w, x = i - y * w;
   float dn = i < n ? __ldg(Dl + i) : qnan();
   while (base < n) {
     const int cx = x, cy = y;
@@ -506,56 +492,52 @@ __device__ __forceinline__ void icp_depth_pass(const SessionDesc& s, int level, 
   }
 }
 
-// The photometric rows of the model points that fall to this block, their 28 FP32 terms and
+// The photometric rows of the model points that fall to this thread's part, their 28 FP32 terms and
 // the count added to this thread's FP64 sums.
-__device__ __forceinline__ void icp_color_pass(const SessionDesc& s, int per, int rank, int C, const IcpPoses& P,
+__device__ __forceinline__ void icp_color_pass(const SessionDesc& s, const IcpDeal& deal, const IcpPoses& P,
                                                double (&acc)[kIcpTerms]) {
-  const int NM = s.W * s.H, T = (int)blockDim.x;
+  const int NM = s.W * s.H, T = deal.T, per = deal.per;
   const float4 r0 = P.cur[0], r1 = P.cur[1], r2 = P.cur[2];
   const float R[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
   const float3 tc = f3(r0.w, r1.w, r2.w);
 #pragma unroll 1
-  for (int base = rank * T * per; base < NM; base += C * T * per)
+  for (int base = deal.rank * T * per; base < NM; base += deal.C * T * per)
 #pragma unroll 1
     for (int k = 0; k < per; ++k) {
-      const int i = base + k * T + (int)threadIdx.x;
+      const int i = base + k * T + deal.tid;
       ColorRow row;
       if (i >= NM || !color_row(s, i, R, tc, row)) continue;
       row.add_to(acc);
     }
 }
 
-// Term t of the 29 among a warp's 64 sums: (i, j) of the upper triangle of [row, 1] by rows,
-// at 8 i + j; then r^2 (6, 6) and the count (7, 7).
-__device__ __forceinline__ int icp_term_at(int t) {
-  if (t >= 27) return t == 27 ? 54 : 63;
-  int i = 0, j = t;
-  while (j >= 7 - i) j -= 7 - i, ++i;
-  return 8 * i + i + j;
+// Block sums from the warps' sums, each warp's left in its part of the staging memory: the
+// lanes of a warp are dealt over 32 / warps terms (icp_my_term), a lane takes a warp's term (at
+// index `at` of its 64 doubles) and the lanes add up pairwise; every lane of a term's group
+// gets its sum.  (A thread a term, adding the warps one after another, took 0.9 us of 32 warps.)
+// All threads must call it; the block has 8, 16 or 32 warps.
+__device__ __forceinline__ int icp_my_term() { return (int)(threadIdx.x / (blockDim.x >> 5)); }
+__device__ __forceinline__ double icp_group_sum(double v) {
+  for (int off = (int)(blockDim.x >> 6); off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
 }
-
-// Block sums from the warps' sums, each warp's left in its part of the staging memory: term
-// threadIdx.x (< kIcpTerms) at index `at` of every warp's 64 doubles, added in warp order.
-// All threads must call it.
 __device__ __forceinline__ double icp_warps_sum(const float* stage0, int at) {
+  const int src = (int)(threadIdx.x & ((blockDim.x >> 5) - 1));
   __syncthreads();
-  double D = 0.0;
-  if (threadIdx.x < kIcpTerms)
-    for (int wi = 0; wi < (int)(blockDim.x >> 5); ++wi)
-      D += reinterpret_cast<const double*>(stage0 + wi * (kIcpStageBytes / 4))[at];
+  const double v = reinterpret_cast<const double*>(stage0 + src * (kIcpStageBytes / 4))[at];
   __syncthreads();  // the staging memory is used again
-  return D;
+  return icp_group_sum(v);
 }
 
-// The block's sums of one pass: term threadIdx.x (< kIcpTerms) of the depth rows, and with
-// photo of the photometric rows too.  All threads must call it.
-__device__ __forceinline__ double icp_depth_sums(const SessionDesc& s, int level, int per, int rank, int C,
+// The block's sums of one pass, this thread's term (icp_my_term, at `at` of a warp's 64 for the
+// depth rows): of the depth rows, and of the photometric ones.  All threads must call it.
+__device__ __forceinline__ double icp_depth_sums(const SessionDesc& s, int level, const IcpDeal& deal,
                                                  const IcpPoses& P, float* stage0, int at) {
   float* const stage = stage0 + (threadIdx.x >> 5) * (kIcpStageBytes / 4);  // this warp's
   double* const wsum = reinterpret_cast<double*>(stage);
   const int lane = threadIdx.x & 31;
   double d0 = 0.0, d1 = 0.0;
-  icp_depth_pass(s, level, per, rank, C, P, stage, d0, d1);
+  icp_depth_pass(s, level, deal, P, stage, d0, d1);
   wsum[2 * lane] = d0;
   wsum[2 * lane + 1] = d1;
   return icp_warps_sum(stage0, at);
@@ -563,12 +545,12 @@ __device__ __forceinline__ double icp_depth_sums(const SessionDesc& s, int level
 // (a warp's sums by a reduce-scatter over its lanes, terms padded to 32: at each of five
 // steps a lane keeps half of its values, sends the other half to its partner and adds what it
 // receives, so lane k ends with the warp's sum of term k after 31 exchanges)
-__device__ __forceinline__ double icp_color_sums(const SessionDesc& s, int per, int rank, int C, const IcpPoses& P,
+__device__ __forceinline__ double icp_color_sums(const SessionDesc& s, const IcpDeal& deal, const IcpPoses& P,
                                                  float* stage0) {
   double acc[kIcpTerms];
 #pragma unroll
   for (int k = 0; k < kIcpTerms; ++k) acc[k] = 0.0;
-  icp_color_pass(s, per, rank, C, P, acc);
+  icp_color_pass(s, deal, P, acc);
   const int lane = threadIdx.x & 31;
   double v[32];
 #pragma unroll
@@ -584,7 +566,7 @@ __device__ __forceinline__ double icp_color_sums(const SessionDesc& s, int per, 
     }
   }
   reinterpret_cast<double*>(stage0 + (threadIdx.x >> 5) * (kIcpStageBytes / 4))[lane] = v[0];
-  return icp_warps_sum(stage0, threadIdx.x);
+  return icp_warps_sum(stage0, icp_my_term());
 }
 
 // All ICP iterations of every level of one frame, one thread-block cluster per session
@@ -606,7 +588,7 @@ __device__ __forceinline__ double icp_color_sums(const SessionDesc& s, int per, 
 // the rows' 29 FP64 sums a thread need 128 (up to 512).
 template <bool COLOR>
 __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
-    k_icp_cluster(const SessionDesc* __restrict__ descs, int fam, int ppt, int wide) {
+    k_icp_cluster(const SessionDesc* __restrict__ descs, int fam, int ppt) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const SessionDesc& s = descs[blockIdx.y];
@@ -626,20 +608,21 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
   // every block has read the initial state before block 0 writes any of it
   cluster.sync();
   if (status0 != 0) return;
-  const int at = icp_term_at(threadIdx.x);
-  const int last = wide && (s.photo_w > 0.f || wide == 2) ? 1 : 0;  // k_icp_finest runs level 0 of a colour-tracked session
-  for (int level = s.levels - 1; level >= last; --level) {
+  const int term = icp_my_term(), at = icp_term_at(term);
+  const bool writes = term < kIcpTerms && (threadIdx.x & ((blockDim.x >> 5) - 1)) == 0;  // a thread a term
+  for (int level = s.levels - 1; level >= 0; --level) {
     // runs no longer than leave every block one: a level's few runs would otherwise fall
     // unevenly on the cluster's blocks (19 runs of 1024 pixels for 16 at 160 x 120), and a
     // pass waits for its slowest block
     const int per = max(1, min(ppt, (s.W >> level) * (s.H >> level) / (C * (int)blockDim.x)));
+    const IcpDeal deal{(int)blockDim.x, (int)threadIdx.x, per, rank, C};
     const bool photo = COLOR && s.photo_w > 0.f && level == 0;
     for (int iter = 0; iter < s.iters[level]; ++iter) {
-      double D = icp_depth_sums(s, level, per, rank, C, P, icp_stage, at);
-      if (threadIdx.x < kIcpTerms) part[0][threadIdx.x] = D;
+      double D = icp_depth_sums(s, level, deal, P, icp_stage, at);
+      if (writes) part[0][term] = D;
       if (photo) {
-        D = icp_color_sums(s, per, rank, C, P, icp_stage);
-        if (threadIdx.x < kIcpTerms) part[1][threadIdx.x] = D;
+        D = icp_color_sums(s, deal, P, icp_stage);
+        if (writes) part[1][term] = D;
       }
       cluster.sync();  // every block's sums are visible to block 0
       if (rank == 0 && threadIdx.x < 64) {
@@ -677,91 +660,123 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
   cluster.sync();  // no block leaves while another may still read block 0's shared memory
 }
 
-// One iteration of the finest level of a small batch's sessions, over as many blocks a session
-// as the device holds: a cluster is at most 16 blocks, on which an iteration of a
-// colour-tracked 640 x 480 session took 125 us, of which the LM step is 5 (locate on a voxel
-// hash with colour, ten such iterations: 2.2 ms with the clusters alone, 0.91 ms so).  Each
-// block leaves its sums in the session's part of `work`; the last block to finish (a counter,
-// no block waits for another) adds them in block order and runs the LM step on the state in
-// `work`, which the next iteration's launch reads.  The launches follow one another by
-// programmatic dependence: a launch's blocks come up while the previous one drains and wait
-// for its results.  An iteration after the level's end returns at once.
+// All ICP iterations of a small batch's sessions, each over its share of the whole device (a
+// block an SM, launched cooperatively: all blocks are resident, so they may wait for one
+// another).  Every iteration a block leaves its sums in the session's part of `work` and counts
+// itself in; when all have, every block adds all the sums, in the same order, and runs the LM
+// step on its own copy of the state, so nothing has to be sent back.  A wait that runs out (it
+// cannot with all blocks resident) marks the workspace and loses the frame, as every later launch
+// on the workspace does at once.
+//
+// What bounds it is latency: an iteration is a pass of a few us, a trip through L2 and the LM
+// step.  A cluster is at most 16 SMs, on which a pass of a colour-tracked 640 x 480 level takes
+// 120 us; a launch an iteration costs 2 us even after the level has ended (a level that starts
+// close to its end runs one iteration of the ten).  At 640 x 480 a depth iteration takes 12 us
+// (pass 3.3, waiting 1.0, sums 1.5, LM step 3.9; 7 us at the coarser levels) and a photometric
+// one 20.
 template <bool COLOR>
-__global__ void __launch_bounds__(256, COLOR ? 2 : 4)
-    k_icp_finest(const SessionDesc* __restrict__ descs, int fam, int ppt, int iter, int wide,
-                 IcpFinest* __restrict__ work) {
-  cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();
+__global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
+    k_icp_wide(const SessionDesc* __restrict__ descs, int fam, IcpWide* __restrict__ work) {
   const SessionDesc& s = descs[blockIdx.y];
-  if (s.kind != kTrackFrame || !in_family(s, fam) || !(s.photo_w > 0.f || wide == 2) || iter >= s.iters[0]) return;
+  if (s.kind != kTrackFrame || !in_family(s, fam)) return;  // the same for every block of the session
   TrackState* ts = s.ts;
-  IcpFinest& f = work[blockIdx.y];
-  // the first iteration starts from the coarser levels' estimate; a session that lost tracking
-  // there has no state in f (which holds what another frame left)
-  if (ts->status != 0 || (iter > 0 && (f.lm.status != 0 || f.lm.level_done != 0))) return;
+  IcpWide& f = work[blockIdx.y];
   extern __shared__ __align__(16) float icp_stage[];
   __shared__ IcpPoses P;
-  __shared__ double sums[kIcpTerms];
+  __shared__ double sums[32];
   __shared__ IcpLm lm;
   __shared__ IcpStepScratch hw;
-  __shared__ int is_last;
-  icp_pose_rows(P.cur, iter == 0 ? ts->R : f.lm.R, iter == 0 ? ts->t : f.lm.t);
+  __shared__ int state;  // -1: the wait ran out
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5), B = (int)gridDim.x;
+  lm_copy(&lm, ts);  // (written again only when every block has counted itself in for the last time)
   icp_pose_rows(P.prev, ts->xf.R_inv, ts->xf.t);
+  icp_pose_rows(P.cur, ts->R, ts->t);
+  if (threadIdx.x == 0) state = *(volatile unsigned*)&f.stalled ? -1 : 0;
   __syncthreads();
-  const int B = (int)gridDim.x;
-  const double D = icp_depth_sums(s, 0, ppt, blockIdx.x, B, P, icp_stage, icp_term_at(threadIdx.x));
-  const bool photo = COLOR && s.photo_w > 0.f;
-  const double E = photo ? icp_color_sums(s, ppt, blockIdx.x, B, P, icp_stage) : 0.0;
-  if (threadIdx.x < kIcpTerms) {
-    f.part[blockIdx.x][threadIdx.x] = D;
-    f.part[blockIdx.x][32 + threadIdx.x] = E;
-    __threadfence();
+  if (lm.status != 0) return;
+  // runs of a warp, dealt over the blocks first
+  const IcpDeal deal{32, lane, 1, warp * B + (int)blockIdx.x, warps * B};
+  const int term = icp_my_term(), at = icp_term_at(term), src = (int)(threadIdx.x & (warps - 1));
+  unsigned turn = 0;  // iterations of this launch
+  bool go = state == 0;
+  for (int level = s.levels - 1; level >= 0 && go; --level) {
+    const bool photo = COLOR && s.photo_w > 0.f && level == 0;
+    for (int iter = 0; iter < s.iters[level]; ++iter) {
+      // (two sets of sums in turn: a block may be one iteration ahead of one that still reads)
+      double(*const part)[64] = f.part[turn & 1];
+      const double D = icp_depth_sums(s, level, deal, P, icp_stage, at);
+      if (term < kIcpTerms && src == 0) part[blockIdx.x][term] = D;
+      if (photo) {
+        const double E = icp_color_sums(s, deal, P, icp_stage);
+        if (term < kIcpTerms && src == 0) part[blockIdx.x][32 + term] = E;
+      }
+      __syncthreads();
+      ++turn;
+      if (threadIdx.x == 0) {
+        unsigned e;
+        int polls = 0;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&f.arrived) : "memory");
+        do {
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(&f.arrived) : "memory");
+        } while (e < turn * (unsigned)B && ++polls < kIcpPolls);
+        if (e < turn * (unsigned)B) {
+          f.stalled = 1u;
+          state = -1;
+        }
+      }
+      __syncthreads();
+      if (state != 0) {
+        go = false;
+        break;
+      }
+      // the blocks' sums: warp w adds the terms (a lane each) of blocks w, w + warps, ..., then
+      // the warps' sums are added pairwise
+      double a = 0.0, c = 0.0;
+      for (int b0 = warp; b0 < B; b0 += 5 * warps) {
+        double u[5], v[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          const int b = b0 + k * warps;
+          u[k] = b < B ? __ldcg(&part[b][lane]) : 0.0;
+          v[k] = COLOR && photo && b < B ? __ldcg(&part[b][32 + lane]) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 5; ++k) a += u[k], c += v[k];
+      }
+      double* const w = reinterpret_cast<double*>(icp_stage);
+      w[33 * warp + lane] = a;
+      if (COLOR) w[33 * (warps + warp) + lane] = c;
+      __syncthreads();
+      a = icp_group_sum(w[33 * src + term]);
+      if (COLOR) c = icp_group_sum(w[33 * (warps + src) + term]);
+      // the photometric normal equations and residual enter weighted, the count stays the depth
+      // count
+      if (src == 0) sums[term] = photo && term < kIcpTerms - 1 ? a + (double)s.photo_w * c : a;
+      if (threadIdx.x == 0) lm.icp_iters[level] += 1u;
+      __syncthreads();
+      if (threadIdx.x < 64) icp_host_step(&lm, hw, sums, iter, s.icp_min_count[level]);
+      __syncthreads();
+      icp_pose_rows(P.cur, lm.R, lm.t);
+      const int lost = lm.status, done = lm.level_done;
+      __syncthreads();
+      if (lost != 0) go = false;
+      if (lost != 0 || done) break;
+    }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) is_last = atomicAdd(&f.done, 1u) == (unsigned)B - 1u;
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  // the blocks' sums: thread t of a warp adds terms t and 32 + t of an eighth of the blocks,
-  // then the eighths in order
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = (B + 7) / 8;
-  double a = 0.0, c = 0.0;
-#pragma unroll 4
-  for (int b = warp * per; b < min(B, (warp + 1) * per); ++b) {
-    a += __ldcg(&f.part[b][lane]);
-    c += __ldcg(&f.part[b][32 + lane]);
+  if (blockIdx.x == 0) lm_copy(ts, &lm);
+  if (threadIdx.x != 0) return;
+  if (state != 0) {
+    ts->status = 3;
+  } else if (atomicAdd(&f.left, 1u) == (unsigned)B - 1u) {  // every block has made its last read
+    f.left = 0u;
+    f.arrived = 0u;
   }
-  double* const w = reinterpret_cast<double*>(icp_stage);
-  w[64 * warp + lane] = a;
-  w[64 * warp + 32 + lane] = c;
-  if (iter == 0) {
-    lm_copy(&lm, ts);
-  } else {
-    for (int k = threadIdx.x; k < (int)(sizeof(IcpLm) / 4); k += blockDim.x)
-      reinterpret_cast<int*>(&lm)[k] = reinterpret_cast<const int*>(&f.lm)[k];
-  }
-  __syncthreads();
-  if (threadIdx.x < kIcpTerms) {
-    a = c = 0.0;
-    for (int b = 0; b < 8; ++b) a += w[64 * b + threadIdx.x], c += w[64 * b + 32 + threadIdx.x];
-    // the photometric normal equations and residual enter weighted, the count stays the
-    // depth count
-    sums[threadIdx.x] = photo && threadIdx.x < kIcpTerms - 1 ? a + (double)s.photo_w * c : a;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) lm.icp_iters[0] += 1u;
-  if (threadIdx.x < 64) icp_host_step(&lm, hw, sums, iter, s.icp_min_count[0]);
-  __syncthreads();
-  for (int k = threadIdx.x; k < (int)(sizeof(IcpLm) / 4); k += blockDim.x)
-    reinterpret_cast<int*>(&f.lm)[k] = reinterpret_cast<const int*>(&lm)[k];
-  if (threadIdx.x == 0) f.done = 0u;
-  if (lm.status != 0 || lm.level_done || iter + 1 == s.iters[0]) lm_copy(ts, &lm);
 }
 
-template __global__ void k_icp_cluster<false>(const SessionDesc*, int, int, int);
-template __global__ void k_icp_cluster<true>(const SessionDesc*, int, int, int);
-template __global__ void k_icp_finest<false>(const SessionDesc*, int, int, int, int, IcpFinest*);
-template __global__ void k_icp_finest<true>(const SessionDesc*, int, int, int, int, IcpFinest*);
+template __global__ void k_icp_cluster<false>(const SessionDesc*, int, int);
+template __global__ void k_icp_cluster<true>(const SessionDesc*, int, int);
+template __global__ void k_icp_wide<false>(const SessionDesc*, int, IcpWide*);
+template __global__ void k_icp_wide<true>(const SessionDesc*, int, IcpWide*);
 
 // After the last ICP launch (or on frame 0): publish the pose, decide the integration
 // gate (NuiKinfuTrackingEngine.cpp:115-127) and reset the estimate for the next frame.

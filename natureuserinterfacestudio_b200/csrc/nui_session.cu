@@ -35,9 +35,9 @@ __global__ void k_feedback_one(const SessionDesc, const DevXform);
 __global__ void k_feedback(const SessionDesc*);
 __global__ void k_vertex_map(const SessionDesc*, int, float4*);
 template <bool COLOR>
-__global__ void k_icp_cluster(const SessionDesc*, int, int, int);
+__global__ void k_icp_cluster(const SessionDesc*, int, int);
 template <bool COLOR>
-__global__ void k_icp_finest(const SessionDesc*, int, int, int, int, IcpFinest*);
+__global__ void k_icp_wide(const SessionDesc*, int, IcpWide*);
 __global__ void k_track_finalize(const SessionDesc*, int, int);
 __global__ void k_ztab(const SessionDesc*);
 __global__ void k_color_level(const SessionDesc, int);
@@ -231,7 +231,8 @@ struct nui_ctx {
   int* h_status = nullptr;  // 2 * cap * 2
   int par = 0;              // the half the next tick uses
   cudaEvent_t ev_tick[2] = {nullptr, nullptr};
-  IcpFinest* d_finest = nullptr;  // level-0 ICP over the whole device: 2 x kIcpWideSessions (a set a stream)
+  IcpWide* d_icp_wide = nullptr;  // ICP over the whole device: 2 x kIcpWideSessions (a set a stream)
+  int wide_blocks = 0;            // blocks of k_icp_wide the device holds at once, one an SM (0: not to be launched)
   unsigned long long* d_count = nullptr;  // counter of the point-cloud fetch
   struct Graph {
     cudaGraphExec_t exec;
@@ -702,7 +703,7 @@ void launch_shift(const BatchPlan& p, const SessionDesc* d, cudaStream_t st) {
 // track): 292 us with 1024 threads, 313 with 512, 381 with 256; 64 sessions (39 dense, 25
 // voxel-hash with colour; six ticks): 47.5 ms with 512 / 256, 49.5 with 512 / 512, 48.0 with
 // 256 / 256.
-void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool color, int fam, int wide, cudaStream_t st) {
+void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool color, int fam, cudaStream_t st) {
   static std::once_flag opt_in;
   std::call_once(opt_in, [] {
     cudaFuncSetAttribute(k_icp_cluster<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -723,52 +724,45 @@ void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool co
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, color ? k_icp_cluster<true> : k_icp_cluster<false>, d, fam, p.tune.icp_pixels_per_thread, wide);
+  cudaLaunchKernelEx(&cfg, color ? k_icp_cluster<true> : k_icp_cluster<false>, d, fam, p.tune.icp_pixels_per_thread);
 }
 
-// Whether level 0 leaves the clusters for launches over the whole device (k_icp_finest, one an
-// iteration): 1 for the colour-tracked sessions, 2 for all, 0 for none.  A cluster holds at
-// most 16 SMs, but a launch costs ~2 us even when the level has ended, so the images must be
-// large enough; a photometric row costs twice a depth row and its level tends to run all its
-// iterations.  Measured, one session, without and with: locate on a voxel hash with colour at
-// 640 x 480 2.2 -> 0.91 ms, colour track at 352 x 208 628 -> 407 us, depth track at 640 x 480
-// 296 -> 286 us (no gain at 320 x 240).
-int icp_wide(const BatchPlan& p, int n, bool color) {
-  const long px = (long)p.maxW * p.maxH;
-  if (n > kIcpWideSessions) return 0;
-  return px >= 1 << 18 ? 2 : color && px >= 1 << 14 ? 1 : 0;
-}
+// Whether the ICP of n sessions leaves the clusters for the whole device (k_icp_wide, a share of
+// `blocks` blocks a session): for few sessions, of any size, as even small levels gain from
+// one warp a scheduler more than a wait through L2 costs over a cluster's barrier.  Measured, one
+// session, clusters (level 0 of large images over the device by a launch an iteration) and
+// k_icp_wide: track at 640 x 480 253 -> 194 us, 320 x 240 218 -> 181, 188 x 132 172 -> 162, with
+// colour 352 x 208 333 -> 261; locate on a voxel hash with colour 875 -> 750.  Beyond four, a
+// session's share nears a cluster's.
+bool icp_wide(int n, int blocks) { return n <= kIcpWideSessions && blocks >= n; }
 
-// One iteration of level 0 of the colour-tracked sessions over the whole device.
-void launch_icp_finest(const BatchPlan& p, const SessionDesc* d, int n, bool color, int fam, int iter, int wide, IcpFinest* work,
-                       cudaStream_t st) {
-  const int per = 4;  // pixels a thread and run: 300 blocks of four an SM at 640 x 480
+// One block an SM, the SMs shared by the sessions.
+void launch_icp_wide(const SessionDesc* d, int n, bool color, int fam, int blocks, IcpWide* work, cudaStream_t st) {
+  const int threads = color ? 512 : 1024;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min(cdiv((long)p.maxW * p.maxH, 256 * per), (unsigned)kIcpWideBlocks), n);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = 8 * kIcpStageBytes;
+  cfg.gridDim = dim3(std::min(blocks / n, kIcpWideBlocks), n);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = (size_t)(threads / 32) * kIcpStageBytes;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
   cfg.attrs = at;
-  cfg.numAttrs = iter > 0 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, color ? k_icp_finest<true> : k_icp_finest<false>, d, fam, per, iter, wide, work);
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, color ? k_icp_wide<true> : k_icp_wide<false>, d, fam, work);
 }
 
 // Colour pyramid (if any session tracks with colour), the ICP iterations of every level,
 // the integration gate and the published pose, for the sessions of family fam among the n
 // descriptors at d.
 void launch_track(const BatchPlan& p, const SessionDesc* d, int n, cudaStream_t st, float* d_pose, int* d_status,
-                  bool color, IcpFinest* work, int fam = kFamAll, bool tick = true) {
+                  bool color, IcpWide* work, int wide_blocks, int fam = kFamAll, bool tick = true) {
   if (n <= 0) return;
   const unsigned npix = cdiv((long)p.maxW * p.maxH, 256);
   if (color) k_color_grad<<<dim3(npix, n, 1), 256, 0, st>>>(d, fam);  // finest level
-  // every level and iteration of every session in one launch: a cluster of
-  // icp_cluster_blocks blocks per session
-  const int wide = icp_wide(p, n, color);
-  launch_icp_cluster(p, d, n, color, fam, wide, st);
-  for (int i = 0; wide && i < p.maxIters[0]; ++i) launch_icp_finest(p, d, n, color, fam, i, wide, work, st);
+  // every level and iteration of every session in one launch
+  if (icp_wide(n, wide_blocks)) launch_icp_wide(d, n, color, fam, wide_blocks, work, st);
+  else launch_icp_cluster(p, d, n, color, fam, st);
   k_track_finalize<<<n, 32, 0, st>>>(d, tick ? 1 : 0, fam);
   k_publish<<<cdiv(n, 64), 64, 0, st>>>(d, n, d_pose, d_status, fam);
   if (color) k_color_keep<<<dim3(cdiv(((long)p.maxW * p.maxH + 3) / 4, 256), n), 256, 0, st>>>(d, fam);
@@ -805,14 +799,16 @@ void enqueue_tick(nui_ctx* ctx, const BatchPlan& p, const SessionDesc* d, float*
     if (ev) cudaEventRecord(ctx->ev[9], hs);
     if (ranged) {
       launch_track(p, d + p.denseHead, p.n - p.denseHead, hs, d_pose, d_status, (p.colorIcp & 2) != 0,
-                   ctx->d_finest + kIcpWideSessions);
-      launch_track(p, d, p.denseHead, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_finest);
+                   ctx->d_icp_wide + kIcpWideSessions, ctx->wide_blocks / 2);
+      launch_track(p, d, p.denseHead, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_icp_wide, ctx->wide_blocks / 2);
     } else {
-      launch_track(p, d, p.n, hs, d_pose, d_status, (p.colorIcp & 2) != 0, ctx->d_finest + kIcpWideSessions, kFamHash);
-      launch_track(p, d, p.n, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_finest, kFamDense);
+      launch_track(p, d, p.n, hs, d_pose, d_status, (p.colorIcp & 2) != 0, ctx->d_icp_wide + kIcpWideSessions,
+                   ctx->wide_blocks / 2, kFamHash);
+      launch_track(p, d, p.n, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_icp_wide, ctx->wide_blocks / 2,
+                   kFamDense);
     }
   } else {
-    launch_track(p, d, p.n, st, d_pose, d_status, p.colorIcp != 0, ctx->d_finest);
+    launch_track(p, d, p.n, st, d_pose, d_status, p.colorIcp != 0, ctx->d_icp_wide, ctx->wide_blocks);
   }
   mark(3);
   if (ev) ctx->side_timed = fork;
@@ -877,12 +873,20 @@ nui_status ensure_cap(nui_ctx* ctx, int n) {
   return NUI_OK;
 }
 
-// The workspace of k_icp_finest, once a tick of the context may need it.
-nui_status ensure_finest(nui_ctx* ctx, const BatchPlan& p) {
-  if (ctx->d_finest || !icp_wide(p, std::min(p.n, kIcpWideSessions), p.colorIcp != 0)) return NUI_OK;
-  const size_t bytes = sizeof(IcpFinest) * 2 * kIcpWideSessions;
-  NUI_CUDA(counted_pool_alloc((void**)&ctx->d_finest, bytes, ctx->pool, ctx->stream));
-  NUI_CUDA(cudaMemsetAsync(ctx->d_finest, 0, bytes, ctx->stream));
+// The workspace of k_icp_wide, at the context's first tracking, and the blocks that are
+// sure to be resident together: one an SM, if the device launches cooperatively and an SM holds
+// a block of either variant.
+nui_status ensure_icp_wide(nui_ctx* ctx) {
+  if (ctx->d_icp_wide) return NUI_OK;
+  const size_t bytes = sizeof(IcpWide) * 2 * kIcpWideSessions;
+  NUI_CUDA(counted_pool_alloc((void**)&ctx->d_icp_wide, bytes, ctx->pool, ctx->stream));
+  NUI_CUDA(cudaMemsetAsync(ctx->d_icp_wide, 0, bytes, ctx->stream));
+  int sms = 0, coop = 0, depth = 0, color = 0;
+  NUI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+  NUI_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+  NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&depth, k_icp_wide<false>, 1024, 32 * kIcpStageBytes));
+  NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&color, k_icp_wide<true>, 512, 16 * kIcpStageBytes));
+  ctx->wide_blocks = coop && depth > 0 && color > 0 ? sms : 0;
   return NUI_OK;
 }
 
@@ -945,7 +949,7 @@ nui_status tick_launch(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
   }
   if (floor) plan_merge(p, *floor);
   p.tune = ctx->tune;
-  if ((st = ensure_finest(ctx, p)) != NUI_OK) return st;
+  if ((st = ensure_icp_wide(ctx)) != NUI_OK) return st;
   NUI_CUDA(cudaMemcpyAsync(ctx->d_descs, hd, sizeof(SessionDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
   if (use_graph && !ctx->timing) {
     auto it = ctx->graphs.find(p);
@@ -1192,7 +1196,7 @@ NUI_API nui_status nui_ctx_destroy(nui_ctx* c) {
   cudaFree(c->d_status);
   cudaFreeHost(c->h_pose);
   cudaFreeHost(c->h_status);
-  if (c->d_finest) cudaFreeAsync(c->d_finest, c->stream);
+  if (c->d_icp_wide) cudaFreeAsync(c->d_icp_wide, c->stream);
   cudaFree(c->d_count);
   cudaStreamDestroy(c->own);
   cudaStreamDestroy(c->side);
@@ -1897,9 +1901,9 @@ nui_status run_stage(nui_session* s, int what, bool sync = true) {
     for (int l = 1; l < p.maxLevels; ++l)
       k_pyramid<<<dim3(cdiv((long)(p.maxW >> l) * (p.maxH >> l), 256), 1), 256, 0, st>>>(dd, l);
   } else if (what == 1) {
-    const nui_status fs = ensure_finest(ctx, p);
+    const nui_status fs = ensure_icp_wide(ctx);
     if (fs != NUI_OK) return fs;
-    launch_track(p, dd, p.n, st, ctx->d_pose, ctx->d_status, p.colorIcp != 0, ctx->d_finest, kFamAll, false);
+    launch_track(p, dd, p.n, st, ctx->d_pose, ctx->d_status, p.colorIcp != 0, ctx->d_icp_wide, ctx->wide_blocks, kFamAll, false);
   } else if (what == 2) {
     k_ztab<<<1, 32, 0, st>>>(dd);
     launch_shift(p, dd, st);

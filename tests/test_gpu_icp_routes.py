@@ -1,5 +1,5 @@
-"""The launch routes of the ICP: one session over the whole device (k_icp_finest at level 0),
-clusters with and without the photometric rows, block sizes by image size -- the same poses by
+"""The launch routes of the ICP: few sessions over the whole device (k_icp_wide), clusters with
+and without the photometric rows, block sizes by image size -- the same poses by
 every route, at the edges of the rules -- and the shared-reciprocal quotients of the
 photometric rows against the division they replace."""
 import random
@@ -18,7 +18,7 @@ from _util import cfg_for, frames, rot_angle
 @pytest.mark.parametrize("W,H,color", [(512, 512, False), (508, 512, False), (516, 508, False), (128, 128, True),
                                        (124, 128, True), (132, 124, True), (64, 48, False)])
 def test_one_session_and_many_agree(gpu_ctx, W, H, color):
-    """n = 1 (the whole-device route from 2^18 pixels, 2^14 with colour) against the same
+    """n = 1 (the whole-device route) against the same
     stream nine times in a batch (clusters only): the routes regroup FP64 sums, so poses agree
     within the 1e-5 that the ICP shapes are held to; depth poses agree with the oracle's."""
     cfg = cfg_for(W=W, H=H, res=(64, 64, 64), color=color, trunc=0.1)
