@@ -341,13 +341,14 @@ NUI_API nui_status nui_ctx_last_tick_kernels(nui_ctx* ctx, int* n);
 /* Launch shapes of a context's tick, chosen by nui_ctx_autotune (or set by hand).  No
  * choice changes a result bit except the two ICP shapes, which regroup the FP64 partial
  * sums of the normal equations (poses agree to the rounding of those sums).
- *   integrate_threads_log2   dense integration: each volume column is split into z chunks,
- *                            one thread each, until a session's launch has >= 2^this
- *                            threads (chunks of >= 16 slices); 14..22, default 18
- *   icp_pixels_per_thread    ICP block: 256 threads x this many pixels; 2, 4, 8 or 16 (4)
+ *   integrate_threads_log2   accepted and reported, without effect: the exact dense
+ *                            integration takes 256 threads per 32 voxel columns; 14..22 (18)
+ *   icp_pixels_per_thread    ICP clusters: a run of a block is its threads (256 to 1024) x this
+ *                            many pixels; 2, 4, 8 or 16 (4)
  *   icp_cluster_blocks       ICP: thread blocks of the cluster that tracks one session;
  *                            2..16 (12: six SMs at two blocks an SM, so that three
- *                            clusters fill an 18-SM GPC; above 8 a non-portable size)
+ *                            clusters fill an 18-SM GPC; above 8 a non-portable size); up
+ *                            to four sessions are tracked over the whole device instead
  *   raycast_tile_width       dense raycast: a warp shades a tile this wide and 32 / this
  *                            high, a block 2 x 2 such tiles; 4, 8, 16 or 32 (8)
  *   hash_raycast_tile_width  the same for the voxel-hash raycast (8)

@@ -132,7 +132,6 @@ struct SessionDesc {
   uint8_t* occ;                   // per 8^3 brick state (kBrick*)
   uint8_t* dist;                  // per brick: distance to the nearest mixed brick (see kMaxDist)
   int max_cw;
-  int zchunks;                    // integration: z chunks per column (one thread each)
   unsigned* fast_tiles;           // tolerance-mode integration: 32 x 8 x 8 tiles kept by the cull (list)
   float* ztab;                    // integration: running sums shared by all columns, 2 (rz + 1)
   // shifting volume (0: fixed): shift distance in voxels, basis translation, and the point

@@ -186,7 +186,7 @@ struct BatchPlan {
   int n;
   int maxW, maxH, maxLevels;
   int maxIters[kMaxLevels];
-  long maxIntegThreads[4];  // per format: columns * zchunks
+  long maxColumns[4];  // per format: voxel columns of a volume
   long maxBricks[4];        // per format: 8^3 bricks
   long maxDistBlocks;       // blocks of the brick distances, all dense formats
   long maxHashBlk;          // scan blocks of 1024 entries
@@ -377,14 +377,6 @@ void icp_thresholds(const nui_session_cfg& c, unsigned* out) {
   }
 }
 
-// Integration z chunks of a volume: threads per launch >= 2^log2_threads, every chunk
-// >= 16 slices.  The chunking changes no result (every chunk replays its column's sums).
-int pick_zchunks(const nui_session_cfg& c, int log2_threads) {
-  const long ncol = (long)c.res[0] * c.res[1], target = 1L << log2_threads;
-  int z = (int)std::max(1L, (target + ncol - 1) / ncol);
-  return std::min(z, std::max(1, c.res[2] / 16));
-}
-
 void fill_desc(const nui_session* s, SessionDesc& d, int kind, const uint16_t* raw, const uint8_t* bgra) {
   std::memset(&d, 0, sizeof(d));
   const nui_session_cfg& c = s->cfg;
@@ -427,7 +419,6 @@ void fill_desc(const nui_session* s, SessionDesc& d, int kind, const uint16_t* r
   d.tol = c.tsdf_format >= NUI_TSDF_F16_U8 ? 1 : 0;
   d.fast_tiles = s->fast_tiles;
   d.max_cw = c.max_color_weight;
-  d.zchunks = pick_zchunks(s->cfg, s->ctx->tune.integrate_threads_log2);
   d.voxel_shift = s->hash ? 0 : c.voxel_shift;
   for (int i = 0; i < 3; ++i) d.shift_basis[i] = c.shift_basis[i];
   d.pts_xyz = s->pts_xyz;
@@ -510,8 +501,7 @@ void plan_add(BatchPlan& p, const nui_session* s) {
     p.maxHashBlk = std::max(p.maxHashBlk, ((long)c.hash_buckets + c.hash_excess + 1023) / 1024);
     return;
   }
-  long th = (long)c.res[0] * c.res[1] * pick_zchunks(c, p.tune.integrate_threads_log2);
-  p.maxIntegThreads[c.tsdf_format] = std::max(p.maxIntegThreads[c.tsdf_format], th);
+  p.maxColumns[c.tsdf_format] = std::max(p.maxColumns[c.tsdf_format], (long)c.res[0] * c.res[1]);
   p.fmtMask |= 1 << c.tsdf_format;
   const long nb = (long)((c.res[0] + 7) / 8) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8);
   p.maxBricks[c.tsdf_format] = std::max(p.maxBricks[c.tsdf_format], nb);
@@ -530,7 +520,7 @@ void plan_merge(BatchPlan& a, const BatchPlan& b) {
   a.maxLevels = std::max(a.maxLevels, b.maxLevels);
   for (int l = 0; l < kMaxLevels; ++l) a.maxIters[l] = std::max(a.maxIters[l], b.maxIters[l]);
   for (int f = 0; f < 4; ++f) {
-    a.maxIntegThreads[f] = std::max(a.maxIntegThreads[f], b.maxIntegThreads[f]);
+    a.maxColumns[f] = std::max(a.maxColumns[f], b.maxColumns[f]);
     a.maxBricks[f] = std::max(a.maxBricks[f], b.maxBricks[f]);
   }
   a.maxDistBlocks = std::max(a.maxDistBlocks, b.maxDistBlocks);
@@ -559,7 +549,7 @@ void launch_integrate(const BatchPlan& p, const SessionDesc* d, cudaStream_t st)
     k_integrate_fast<F><<<dim3((unsigned)std::max<long>(blocks, 1), dense_n(p)), 32 * kFastWarps, 0, st>>>(d);
     return;
   }
-  k_integrate<F><<<dim3(cdiv(p.maxIntegThreads[F], 256), dense_n(p)), 256, 0, st>>>(d);
+  k_integrate<F><<<dim3(cdiv(p.maxColumns[F], 32), dense_n(p)), 256, 0, st>>>(d);
 }
 template <int F>
 void launch_summary(const BatchPlan& p, const SessionDesc* d, cudaStream_t st, int force) {
@@ -1365,7 +1355,6 @@ NUI_API nui_status nui_ctx_autotune(nui_ctx* c, const nui_session_cfg* cfgs, int
     }
     best.*field = pick;
   };
-  if (dense) tune_one(&nui_tuning::integrate_threads_log2, {16, 17, 18, 19, 20}, 3);
   // the ICP shapes and ray tiles by the whole tick: with dense and hash sessions the hash
   // sessions' tracking and raycast run on the second stream, beside stages 2-5
   tune_one(&nui_tuning::icp_cluster_blocks, {8, 12, 16}, 6);

@@ -1,6 +1,8 @@
-"""Tolerance-mode integration where its tiles (32 x 8 x 8 voxels, two z slices a warp) can go
-wrong: single tiles, x sizes whose rows are not whole or not 16-byte aligned, y and z remainders
-that leave a warp one slice or none, several sessions of unlike sizes in one launch."""
+"""Integration where its splits can go wrong.  Tolerance mode (tiles of 32 x 8 x 8 voxels, two z
+slices a warp): single tiles, x sizes whose rows are not whole or not 16-byte aligned, y and z
+remainders that leave a warp one slice or none, several sessions of unlike sizes in one launch.
+The exact formats (32 columns a block, chunks of z a warp): columns that do not fill a block, z
+sizes below, at and past a chunk's and the largest."""
 import numpy as np
 import pytest
 
@@ -59,3 +61,21 @@ def test_unlike_sizes_in_one_launch(gpu_ctx):
         for a, b, r in zip(solo, both, SIZES):
             assert np.array_equal(a.download(6).view(np.uint16), b.download(6).view(np.uint16)), (i, r)
             assert np.array_equal(a.download(14), b.download(14)) and np.array_equal(a.download(13), b.download(13)), (i, r)
+
+
+@pytest.mark.parametrize("res", [(8, 8, 8), (33, 9, 15), (31, 33, 17), (64, 40, 129), (24, 20, 1024), (9, 8, 1023)])
+def test_exact_columns(gpu_ctx, res):
+    """The first frame's int16 volume equals the oracle's, the FP32 one its values' twin: the
+    same voxels with the same weights."""
+    d = frames(1, W=96, H=72, seed=4)[0][0]
+    cfg, c32 = (cfg_for(W=96, H=72, res=res, fmt=f, trunc=0.2) for f in (L.TSDF_I16, L.TSDF_F32))
+    eng = O.Engine(cfg)
+    s, f = L.Session(gpu_ctx, cfg), L.Session(gpu_ctx, c32)
+    assert s.process(d)[0] and f.process(d)[0] and eng.frame(d)
+    assert s.touched() == f.touched() == eng.touched() > 0
+    v = eng.volume().reshape(-1, 2)
+    assert np.array_equal(s.volume_ref_layout().reshape(-1, 2), v)
+    w = f.volume_ref_layout().reshape(-1, 2)
+    assert np.array_equal(w[:, 1], v[:, 1]) and np.max(np.abs(w[:, 0] - v[:, 0].astype(np.int32))) <= 1
+    s.close()
+    f.close()
