@@ -90,6 +90,14 @@ struct IcpWide {
   unsigned arrived, left, stalled;
 };
 
+// Where a tick's results go (14 floats and 2 ints a slot), and whether a shifting volume's
+// shift is made by the tracking.
+struct TrackOut {
+  float* pose;
+  int* status;
+  int shift_now;
+};
+
 // What one session does in the current tick (host-written, read by every kernel).
 enum FrameKind : int { kInactive = -1, kFirstFrame = 0, kTrackFrame = 1 };
 
@@ -133,7 +141,6 @@ struct SessionDesc {
   uint8_t* dist;                  // per brick: distance to the nearest mixed brick (see kMaxDist)
   int max_cw;
   unsigned* fast_tiles;           // tolerance-mode integration: 32 x 8 x 8 tiles kept by the cull (list)
-  float* ztab;                    // integration: running sums shared by all columns, 2 (rz + 1)
   // shifting volume (0: fixed): shift distance in voxels, basis translation, and the point
   // cache of the slabs that leave the volume (pts_cap points of xyz / rgba floats)
   int voxel_shift;

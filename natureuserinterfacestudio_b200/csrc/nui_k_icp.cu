@@ -569,6 +569,108 @@ __device__ __forceinline__ double icp_color_sums(const SessionDesc& s, const Icp
   return icp_warps_sum(stage0, icp_my_term());
 }
 
+// NuiKinfuOpenCLShiftScene::integrateVolume -> shiftVolume (NuiKinfuOpenCLShiftScene.cpp:
+// 288-362): before a shifting volume integrates, every axis on which the camera lies
+// voxel_shift or more voxels from the basis moves the volume by voxel_shift voxels; the
+// camera's local translation moves back by the same distance and the offset forward.  The
+// frame's shift is left in ts->shift for the fetch / roll kernels that follow.
+__device__ void shift_decide(const SessionDesc& s, TrackState* ts) {
+  ts->shift[0] = ts->shift[1] = ts->shift[2] = 0;
+  const int vs = s.voxel_shift;
+  if (vs <= 0 || s.fmt < 0) return;
+  float st[3];
+  int tr[3];
+  for (int a = 0; a < 3; ++a) {
+    st[a] = ts->xf.t[a] - s.shift_basis[a];
+    const int f = (int)floorf(st[a] / s.cell[a]);
+    tr[a] = st[a] < 0.f ? max(-vs, f) : min(vs, f);
+  }
+  for (int a = 0; a < 3; ++a)
+    if (abs(tr[a]) >= vs) {
+      ts->shift[a] = tr[a];
+      ts->voff[a] += tr[a];
+      st[a] -= (float)tr[a] * s.cell[a];
+    }
+  for (int a = 0; a < 3; ++a) {
+    ts->xf.t[a] = st[a] + s.shift_basis[a];
+    ts->t[a] = ts->xf.t[a];
+  }
+}
+
+// After the last ICP iteration (or on frame 0): the pose, the integration gate
+// (NuiKinfuTrackingEngine.cpp:115-127), and the estimate for the next frame.
+// shift_now: the tick's finalize makes the shifting volume's shift of an integrating
+// frame here; the step-wise track leaves it to the integration call (k_open_gate).
+__device__ __forceinline__ void track_finalize(const SessionDesc& s, TrackState* ts, int shift_now) {
+  if (s.kind == kFirstFrame) {
+    ts->integrate = ts->status == 0 ? 1 : 0;
+    ts->shift[0] = ts->shift[1] = ts->shift[2] = 0;
+    if (ts->integrate && shift_now) shift_decide(s, ts);
+    return;
+  }
+  ts->shift[0] = ts->shift[1] = ts->shift[2] = 0;
+  if (ts->status != 0) {  // tracking lost: keep the previous pose, skip the rest
+    for (int i = 0; i < 9; ++i) ts->R[i] = ts->xf.R[i];
+    for (int i = 0; i < 3; ++i) ts->t[i] = ts->xf.t[i];
+    ts->integrate = 0;
+    return;
+  }
+  double a[9];
+  for (int i = 0; i < 9; ++i) a[i] = ts->R[i];
+  const double c00 = a[4] * a[8] - a[5] * a[7], c01 = a[5] * a[6] - a[3] * a[8], c02 = a[3] * a[7] - a[4] * a[6];
+  const double det = a[0] * c00 + a[1] * c01 + a[2] * c02;
+  const double inv[9] = {c00, a[2] * a[7] - a[1] * a[8], a[1] * a[5] - a[2] * a[4],
+                         c01, a[0] * a[8] - a[2] * a[6], a[2] * a[3] - a[0] * a[5],
+                         c02, a[1] * a[6] - a[0] * a[7], a[0] * a[4] - a[1] * a[3]};
+  for (int i = 0; i < 9; ++i) {
+    ts->xf.R[i] = ts->R[i];
+    ts->xf.R_inv[i] = (float)(inv[i] / det);
+  }
+  for (int i = 0; i < 3; ++i) ts->xf.t[i] = ts->t[i];
+  // rotation angle of R^-1 * R_last and translation distance
+  double tr = 0;
+  for (int i = 0; i < 3; ++i)
+    for (int k = 0; k < 3; ++k) tr += (double)ts->R[k * 3 + i] * (double)ts->lastR[k * 3 + i];
+  const double cv = fmin(1.0, fmax(-1.0, (tr - 1.0) / 2.0));
+  const double rn = acos(cv);
+  // translations compared globally: local + the volume's offset (0 for a fixed volume)
+  double tn = 0;
+  for (int i = 0; i < 3; ++i) {
+    const float g = ts->voff[i] ? ts->t[i] + (float)ts->voff[i] * s.cell[i] : ts->t[i];
+    tn += ((double)(g - ts->lastT[i])) * ((double)(g - ts->lastT[i]));
+  }
+  tn = sqrt(tn);
+  ts->integrate = ((float)((rn + tn) / 2) >= s.integ_thr) ? 1 : 0;
+  if (ts->integrate) {
+    if (shift_now) shift_decide(s, ts);
+    for (int i = 0; i < 9; ++i) ts->lastR[i] = ts->R[i];
+    for (int i = 0; i < 3; ++i) ts->lastT[i] = ts->voff[i] ? ts->t[i] + (float)ts->voff[i] * s.cell[i] : ts->t[i];
+  }
+}
+
+// The end of a session's tracking, by one thread: the above for an active session, then status,
+// gate and pose of this tick into the packed arrays that the host reads back with one copy.
+__device__ __noinline__ void track_end(const SessionDesc& s, const TrackOut& out) {
+  TrackState* ts = s.ts;
+  if (ts == nullptr) return;
+  if (s.kind >= 0) track_finalize(s, ts, out.shift_now);
+  if (!out.pose || !out.status) return;
+  float* const pose = out.pose + 14 * s.slot;
+  out.status[2 * s.slot] = s.kind < 0 ? 0 : ts->status;
+  out.status[2 * s.slot + 1] = ts->integrate;
+  for (int k = 0; k < 9; ++k) pose[k] = ts->xf.R[k];
+  for (int k = 0; k < 3; ++k) pose[9 + k] = ts->xf.t[k];
+  pose[12] = ts->error;
+  pose[13] = ts->count;
+}
+
+// The same as a launch of its own, behind the clusters (inside them it cost a batch of 64 more
+// than the launch: 40.0 ms for six ticks against 39.4).
+__global__ void k_track_end(const SessionDesc* __restrict__ descs, int fam, const TrackOut out) {
+  const SessionDesc& s = descs[blockIdx.x];
+  if (threadIdx.x == 0 && in_family(s, fam)) track_end(s, out);
+}
+
 // All ICP iterations of every level of one frame, one thread-block cluster per session
 // (NuiKinfuOpenCLDepthTracker::IterativeClosestPoint, NuiKinfuOpenCLDepthTracker.cpp:240-504).
 // The C blocks of a cluster (C = 2..16, a launch attribute: the ICP tuning's blocks per
@@ -676,9 +778,13 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
 // one 20.
 template <bool COLOR>
 __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
-    k_icp_wide(const SessionDesc* __restrict__ descs, int fam, IcpWide* __restrict__ work) {
+    k_icp_wide(const SessionDesc* __restrict__ descs, int fam, IcpWide* __restrict__ work, const TrackOut out) {
   const SessionDesc& s = descs[blockIdx.y];
-  if (s.kind != kTrackFrame || !in_family(s, fam)) return;  // the same for every block of the session
+  if (!in_family(s, fam)) return;  // (this and the next: the same for every block of the session)
+  if (s.kind != kTrackFrame) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) track_end(s, out);
+    return;
+  }
   TrackState* ts = s.ts;
   IcpWide& f = work[blockIdx.y];
   extern __shared__ __align__(16) float icp_stage[];
@@ -693,7 +799,10 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
   icp_pose_rows(P.cur, ts->R, ts->t);
   if (threadIdx.x == 0) state = *(volatile unsigned*)&f.stalled ? -1 : 0;
   __syncthreads();
-  if (lm.status != 0) return;
+  if (lm.status != 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) track_end(s, out);
+    return;
+  }
   // runs of a warp, dealt over the blocks first
   const IcpDeal deal{32, lane, 1, warp * B + (int)blockIdx.x, warps * B};
   const int term = icp_my_term(), at = icp_term_at(term), src = (int)(threadIdx.x & (warps - 1));
@@ -763,11 +872,14 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
       if (lost != 0 || done) break;
     }
   }
-  if (blockIdx.x == 0) lm_copy(ts, &lm);
-  if (threadIdx.x != 0) return;
-  if (state != 0) {
-    ts->status = 3;
-  } else if (atomicAdd(&f.left, 1u) == (unsigned)B - 1u) {  // every block has made its last read
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0 && state != 0) lm.status = 3;
+    __syncthreads();
+    lm_copy(ts, &lm);
+    __syncthreads();
+    if (threadIdx.x == 0) track_end(s, out);
+  }
+  if (threadIdx.x == 0 && state == 0 && atomicAdd(&f.left, 1u) == (unsigned)B - 1u) {  // every block has made its last read
     f.left = 0u;
     f.arrived = 0u;
   }
@@ -775,59 +887,13 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
 
 template __global__ void k_icp_cluster<false>(const SessionDesc*, int, int);
 template __global__ void k_icp_cluster<true>(const SessionDesc*, int, int);
-template __global__ void k_icp_wide<false>(const SessionDesc*, int, IcpWide*);
-template __global__ void k_icp_wide<true>(const SessionDesc*, int, IcpWide*);
-
-// After the last ICP launch (or on frame 0): publish the pose, decide the integration
-// gate (NuiKinfuTrackingEngine.cpp:115-127) and reset the estimate for the next frame.
-// Running sums of integrateTsdfVolumeKernel that do not depend on the voxel column
-// (tsdfVolume.cl:74-79: v_g_z and z_scaled, both advanced by cell_z per slice), for the
-// pose integration will use: ztab[z] and ztab[rz + 1 + z] after z additions.
-__device__ void fill_ztab(const SessionDesc& s, const TrackState* ts) {
-  if (!s.ztab || s.tol) return;  // the tolerance-mode integration computes its positions directly
-  const int rz = s.res[2];
-  const float c2 = s.cell[2];
-  float vgz = 0.5f * c2 - ts->xf.t[2], zs = 0.f;
-  for (int z = 0; z <= rz; ++z) {
-    s.ztab[z] = vgz;
-    s.ztab[rz + 1 + z] = zs;
-    vgz += c2;
-    zs += c2;
-  }
-}
-
-// NuiKinfuOpenCLShiftScene::integrateVolume -> shiftVolume (NuiKinfuOpenCLShiftScene.cpp:
-// 288-362): before a shifting volume integrates, every axis on which the camera lies
-// voxel_shift or more voxels from the basis moves the volume by voxel_shift voxels; the
-// camera's local translation moves back by the same distance and the offset forward.  The
-// frame's shift is left in ts->shift for the fetch / roll kernels that follow.
-__device__ void shift_decide(const SessionDesc& s, TrackState* ts) {
-  ts->shift[0] = ts->shift[1] = ts->shift[2] = 0;
-  const int vs = s.voxel_shift;
-  if (vs <= 0 || s.fmt < 0) return;
-  float st[3];
-  int tr[3];
-  for (int a = 0; a < 3; ++a) {
-    st[a] = ts->xf.t[a] - s.shift_basis[a];
-    const int f = (int)floorf(st[a] / s.cell[a]);
-    tr[a] = st[a] < 0.f ? max(-vs, f) : min(vs, f);
-  }
-  for (int a = 0; a < 3; ++a)
-    if (abs(tr[a]) >= vs) {
-      ts->shift[a] = tr[a];
-      ts->voff[a] += tr[a];
-      st[a] -= (float)tr[a] * s.cell[a];
-    }
-  for (int a = 0; a < 3; ++a) {
-    ts->xf.t[a] = st[a] + s.shift_basis[a];
-    ts->t[a] = ts->xf.t[a];
-  }
-}
+template __global__ void k_icp_wide<false>(const SessionDesc*, int, IcpWide*, const TrackOut);
+template __global__ void k_icp_wide<true>(const SessionDesc*, int, IcpWide*, const TrackOut);
 
 // Start of an integration the host requests directly (step-wise calls): the gate opens, the
-// counters it reports start over (for a voxel hash, the failures before it are noted), the
-// shift is made and the table filled.
-__global__ void k_ztab(const SessionDesc* __restrict__ descs) {
+// counters it reports start over (for a voxel hash, the failures before it are noted) and the
+// shift is made.
+__global__ void k_open_gate(const SessionDesc* __restrict__ descs) {
   const SessionDesc& s = descs[blockIdx.x];
   if (threadIdx.x != 0 || s.kind < 0) return;
   s.ts->integrate = 1;
@@ -837,7 +903,6 @@ __global__ void k_ztab(const SessionDesc* __restrict__ descs) {
     s.hcount[kHashFaultsBefore] = s.hcount[kHashChainFaults];
   }
   shift_decide(s, s.ts);
-  fill_ztab(s, s.ts);
 }
 
 // nui_set_pose: the camera pose and the tracker's estimate.
@@ -848,62 +913,6 @@ __global__ void k_set_pose(TrackState* ts, const __grid_constant__ DevXform m) {
     ts->xf.R_inv[k] = m.R_inv[k];
   }
   if (k < 3) ts->xf.t[k] = ts->t[k] = m.t[k];
-}
-
-// shift_now: the tick's finalize makes the shifting volume's shift of an integrating
-// frame here; the step-wise track leaves it to the integration call (k_ztab).
-__global__ void k_track_finalize(const SessionDesc* __restrict__ descs, int shift_now, int fam) {
-  const SessionDesc& s = descs[blockIdx.x];
-  if (threadIdx.x != 0 || s.kind < 0 || !in_family(s, fam)) return;
-  TrackState* ts = s.ts;
-  if (s.kind == kFirstFrame) {
-    ts->integrate = ts->status == 0 ? 1 : 0;
-    ts->shift[0] = ts->shift[1] = ts->shift[2] = 0;
-    if (ts->integrate) {
-      if (shift_now) shift_decide(s, ts);
-      fill_ztab(s, ts);
-    }
-    return;
-  }
-  ts->shift[0] = ts->shift[1] = ts->shift[2] = 0;
-  if (ts->status != 0) {  // tracking lost: keep the previous pose, skip the rest
-    for (int i = 0; i < 9; ++i) ts->R[i] = ts->xf.R[i];
-    for (int i = 0; i < 3; ++i) ts->t[i] = ts->xf.t[i];
-    ts->integrate = 0;
-    return;
-  }
-  double a[9];
-  for (int i = 0; i < 9; ++i) a[i] = ts->R[i];
-  const double c00 = a[4] * a[8] - a[5] * a[7], c01 = a[5] * a[6] - a[3] * a[8], c02 = a[3] * a[7] - a[4] * a[6];
-  const double det = a[0] * c00 + a[1] * c01 + a[2] * c02;
-  const double inv[9] = {c00, a[2] * a[7] - a[1] * a[8], a[1] * a[5] - a[2] * a[4],
-                         c01, a[0] * a[8] - a[2] * a[6], a[2] * a[3] - a[0] * a[5],
-                         c02, a[1] * a[6] - a[0] * a[7], a[0] * a[4] - a[1] * a[3]};
-  for (int i = 0; i < 9; ++i) {
-    ts->xf.R[i] = ts->R[i];
-    ts->xf.R_inv[i] = (float)(inv[i] / det);
-  }
-  for (int i = 0; i < 3; ++i) ts->xf.t[i] = ts->t[i];
-  // rotation angle of R^-1 * R_last and translation distance
-  double tr = 0;
-  for (int i = 0; i < 3; ++i)
-    for (int k = 0; k < 3; ++k) tr += (double)ts->R[k * 3 + i] * (double)ts->lastR[k * 3 + i];
-  const double cv = fmin(1.0, fmax(-1.0, (tr - 1.0) / 2.0));
-  const double rn = acos(cv);
-  // translations compared globally: local + the volume's offset (0 for a fixed volume)
-  double tn = 0;
-  for (int i = 0; i < 3; ++i) {
-    const float g = ts->voff[i] ? ts->t[i] + (float)ts->voff[i] * s.cell[i] : ts->t[i];
-    tn += ((double)(g - ts->lastT[i])) * ((double)(g - ts->lastT[i]));
-  }
-  tn = sqrt(tn);
-  ts->integrate = ((float)((rn + tn) / 2) >= s.integ_thr) ? 1 : 0;
-  if (ts->integrate) {
-    if (shift_now) shift_decide(s, ts);
-    fill_ztab(s, ts);
-    for (int i = 0; i < 9; ++i) ts->lastR[i] = ts->R[i];
-    for (int i = 0; i < 3; ++i) ts->lastT[i] = ts->voff[i] ? ts->t[i] + (float)ts->voff[i] * s.cell[i] : ts->t[i];
-  }
 }
 
 }  // namespace nui

@@ -9,8 +9,8 @@
 // incrementally along z (v_x += R_inv[2]*cell*fx, ...); rounding of that running sum
 // decides which pixel a voxel projects to, so each thread replays the same additions.
 // A block owns 32 columns: its first warp replays their additions over all z and leaves the
-// sums at every chunk of z, the second computes each column's interval of z, and then every warp
-// integrates chunks, evaluating the projections of kZUnroll slices before it issues their
+// sums at every chunk of z, the second computes each column's interval of z, the third the sums
+// that all columns share, and then every warp integrates chunks, evaluating the projections of kZUnroll slices before it issues their
 // loads so that several voxel reads are in flight per thread.
 #include "nui_device.cuh"
 
@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(kTsdfThreads, 4) k_integrate(const SessionDesc
   if ((long)blockIdx.x * 32 >= ncol) return;
   __shared__ float2 at[kMaxChunks][32];  // (v_x, v_y) of a column where a chunk starts
   __shared__ int span[2][32];            // a column's interval of z
+  __shared__ float zt_vgz[1024], zt_zs[1024];  // v_g_z and z_scaled after z additions (tsdfVolume.cl:74-79)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long col = (long)blockIdx.x * 32 + lane;
   const bool live = col < ncol;
@@ -46,8 +47,6 @@ __global__ void __launch_bounds__(kTsdfThreads, 4) k_integrate(const SessionDesc
   const float vgx = ((float)(vx - rx / 2) + 0.5f) * c0 - m.t[0];
   const float vgy = ((float)(vy - ry / 2) + 0.5f) * c1 - m.t[1];
   const float vgz0 = (0.5f) * c2 - m.t[2];
-  const float* __restrict__ zt_vgz = s.ztab;            // v_g_z after z additions
-  const float* __restrict__ zt_zs = s.ztab + rz + 1;    // z_scaled after z additions
   const float part = vgx * vgx + vgy * vgy;
   const float fx = s.cam.fx, fy = s.cam.fy, ccx = s.cam.cx, ccy = s.cam.cy;
   float v_x = (Ri[0] * vgx + Ri[1] * vgy + Ri[2] * vgz0) * fx;
@@ -67,6 +66,15 @@ __global__ void __launch_bounds__(kTsdfThreads, 4) k_integrate(const SessionDesc
         v_x += dx;
         v_y += dy;
       }
+    }
+  }
+  if (threadIdx.x == 64) {
+    float vgz = vgz0, zs = 0.f;
+    for (int z = 0; z < rz; ++z) {
+      zt_vgz[z] = vgz;
+      zt_zs[z] = zs;
+      vgz += c2;
+      zs += c2;
     }
   }
   // Conservative z interval of this column: only voxels whose exact projection can land

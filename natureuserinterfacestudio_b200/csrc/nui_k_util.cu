@@ -1,25 +1,8 @@
-// Small utility kernels: per-session result publication and conversion between the
+// Small utility kernels: the start and end of a tick, and conversion between the
 // session volume layout and the reference layout ((x + y*rx)*rz + z, short2).
 #include "nui_device.cuh"
 
 namespace nui {
-
-// One thread per session: status, gate and pose of this tick into a packed array that
-// the host reads back with one copy.
-__global__ void k_publish(const SessionDesc* __restrict__ descs, int n, float* pose, int* status, int fam) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !pose || !status) return;
-  const SessionDesc& s = descs[i];
-  if (s.ts == nullptr || !in_family(s, fam)) return;
-  const TrackState* ts = s.ts;
-  const int o = s.slot;
-  status[2 * o] = s.kind < 0 ? 0 : ts->status;
-  status[2 * o + 1] = ts->integrate;
-  for (int k = 0; k < 9; ++k) pose[14 * o + k] = ts->xf.R[k];
-  for (int k = 0; k < 3; ++k) pose[14 * o + 9 + k] = ts->xf.t[k];
-  pose[14 * o + 12] = ts->error;
-  pose[14 * o + 13] = ts->count;
-}
 
 // Start of a tick: clear the per-frame counters of every active session, and the flag of a
 // frame that lost tracking (the state stayed on the frame before it; this frame starts

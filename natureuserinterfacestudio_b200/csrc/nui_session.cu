@@ -6,7 +6,7 @@
 // is this fixed sequence of launches, each covering every session of the batch
 // (blockIdx.y = session):
 //   k_preprocess, k_pyramid x (levels-1), k_feedback, k_icp x sum(iterations),
-//   k_track_finalize, k_integrate<fmt>, k_raycast<fmt>
+//   k_track_end, k_integrate<fmt>, k_raycast<fmt>
 // Which session does what in a tick (first frame / tracking / inactive) is data in the
 // session table, so the same sequence serves every tick and is captured once.
 #include <cuda_runtime.h>
@@ -37,9 +37,9 @@ __global__ void k_vertex_map(const SessionDesc*, int, float4*);
 template <bool COLOR>
 __global__ void k_icp_cluster(const SessionDesc*, int, int);
 template <bool COLOR>
-__global__ void k_icp_wide(const SessionDesc*, int, IcpWide*);
-__global__ void k_track_finalize(const SessionDesc*, int, int);
-__global__ void k_ztab(const SessionDesc*);
+__global__ void k_icp_wide(const SessionDesc*, int, IcpWide*, const TrackOut);
+__global__ void k_track_end(const SessionDesc*, int, const TrackOut);
+__global__ void k_open_gate(const SessionDesc*);
 __global__ void k_color_level(const SessionDesc, int);
 __global__ void k_color_grad_one(const SessionDesc);
 __global__ void k_set_pose(TrackState*, const DevXform);
@@ -64,7 +64,6 @@ template <int F>
 __global__ void k_raycast_fast(const SessionDesc*, int);
 template <int F>
 __global__ void k_raycast_finish_fast(const SessionDesc*);
-__global__ void k_publish(const SessionDesc*, int, float*, int*, int);
 __global__ void k_tick_begin(const SessionDesc*, int);
 __global__ void k_hash_health(const SessionDesc*, int, int*);
 __global__ void k_occ_clear(const SessionDesc*);
@@ -263,7 +262,6 @@ struct nui_session {
   uchar4* cvol = nullptr;
   uint8_t* occ = nullptr;
   uint8_t* dist = nullptr;  // brick distances
-  float* ztab = nullptr;
   unsigned* fast_tiles = nullptr;
   float* tile_max = nullptr;
   TrackState* ts = nullptr;
@@ -415,7 +413,6 @@ void fill_desc(const nui_session* s, SessionDesc& d, int kind, const uint16_t* r
   d.cvol = s->cvol;
   d.occ = s->occ;
   d.dist = s->dist;
-  d.ztab = s->ztab;
   d.tol = c.tsdf_format >= NUI_TSDF_F16_U8 ? 1 : 0;
   d.fast_tiles = s->fast_tiles;
   d.max_cw = c.max_color_weight;
@@ -727,7 +724,8 @@ void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool co
 bool icp_wide(int n, int blocks) { return n <= kIcpWideSessions && blocks >= n; }
 
 // One block an SM, the SMs shared by the sessions.
-void launch_icp_wide(const SessionDesc* d, int n, bool color, int fam, int blocks, IcpWide* work, cudaStream_t st) {
+void launch_icp_wide(const SessionDesc* d, int n, bool color, int fam, int blocks, IcpWide* work, const TrackOut& out,
+                     cudaStream_t st) {
   const int threads = color ? 512 : 1024;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(std::min(blocks / n, kIcpWideBlocks), n);
@@ -739,7 +737,7 @@ void launch_icp_wide(const SessionDesc* d, int n, bool color, int fam, int block
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, color ? k_icp_wide<true> : k_icp_wide<false>, d, fam, work);
+  cudaLaunchKernelEx(&cfg, color ? k_icp_wide<true> : k_icp_wide<false>, d, fam, work, out);
 }
 
 // Colour pyramid (if any session tracks with colour), the ICP iterations of every level,
@@ -750,11 +748,14 @@ void launch_track(const BatchPlan& p, const SessionDesc* d, int n, cudaStream_t 
   if (n <= 0) return;
   const unsigned npix = cdiv((long)p.maxW * p.maxH, 256);
   if (color) k_color_grad<<<dim3(npix, n, 1), 256, 0, st>>>(d, fam);  // finest level
-  // every level and iteration of every session in one launch
-  if (icp_wide(n, wide_blocks)) launch_icp_wide(d, n, color, fam, wide_blocks, work, st);
-  else launch_icp_cluster(p, d, n, color, fam, st);
-  k_track_finalize<<<n, 32, 0, st>>>(d, tick ? 1 : 0, fam);
-  k_publish<<<cdiv(n, 64), 64, 0, st>>>(d, n, d_pose, d_status, fam);
+  // every level and iteration of every session in one launch, and the tracking's end
+  const TrackOut out{d_pose, d_status, tick ? 1 : 0};
+  if (icp_wide(n, wide_blocks)) {
+    launch_icp_wide(d, n, color, fam, wide_blocks, work, out, st);
+  } else {
+    launch_icp_cluster(p, d, n, color, fam, st);
+    k_track_end<<<n, 32, 0, st>>>(d, fam, out);
+  }
   if (color) k_color_keep<<<dim3(cdiv(((long)p.maxW * p.maxH + 3) / 4, 256), n), 256, 0, st>>>(d, fam);
 }
 
@@ -1409,7 +1410,6 @@ NUI_API size_t nui_session_device_bytes(const nui_session_cfg* c) {
     b += (size_t)((c->res[0] + 31) / 32) * ((c->res[1] + 7) / 8) * ((c->res[2] + 7) / 8) * 4;
   if (c->color_volume) b += nv * 4;
   b += 2 * (size_t)((c->res[0] + 7) / 8) * ((c->res[1] + 7) / 8) * ((c->res[2] + 7) / 8);
-  b += 2 * ((size_t)c->res[2] + 1) * sizeof(float);
   if (c->voxel_shift > 0) b += (size_t)c->shift_point_cap * 28;
   return b;
 }
@@ -1506,8 +1506,7 @@ nui_status session_create(nui_ctx* ctx, const nui_session_cfg* cfg, nui_session*
     if (ok && c.tsdf_format >= NUI_TSDF_F16_U8)
       ok = alloc((void**)&s->fast_tiles, (size_t)((c.res[0] + 31) / 32) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8) * 4);
     const size_t nbricks = (size_t)((c.res[0] + 7) / 8) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8);
-    if (ok) ok = alloc((void**)&s->occ, nbricks) && alloc((void**)&s->dist, nbricks) &&
-                 alloc((void**)&s->ztab, 2 * ((size_t)c.res[2] + 1) * sizeof(float));
+    if (ok) ok = alloc((void**)&s->occ, nbricks) && alloc((void**)&s->dist, nbricks);
     if (ok && c.color_volume) ok = alloc((void**)&s->cvol, nv * 4) && alloc((void**)&s->bgra, N * 4) && alloc((void**)&s->cmap, N * 4);
   }
   if (ok && c.photometric_weight > 0.f)
@@ -1894,7 +1893,7 @@ nui_status run_stage(nui_session* s, int what, bool sync = true) {
     if (fs != NUI_OK) return fs;
     launch_track(p, dd, p.n, st, ctx->d_pose, ctx->d_status, p.colorIcp != 0, ctx->d_icp_wide, ctx->wide_blocks, kFamAll, false);
   } else if (what == 2) {
-    k_ztab<<<1, 32, 0, st>>>(dd);
+    k_open_gate<<<1, 32, 0, st>>>(dd);
     launch_shift(p, dd, st);
     launch_integrate<0>(p, dd, st);
     launch_integrate<1>(p, dd, st);
@@ -1946,7 +1945,7 @@ NUI_API nui_status nui_track(nui_session* s, float* err, int* count) {
   nui_status st = ensure_cap(s->ctx, 1);
   if (st != NUI_OK) return st;
   // the track stage must run with the integration threshold of the session, and must
-  // not integrate: k_track_finalize only decides the gate
+  // not integrate: the tracking only decides the gate
   st = run_stage(s, 1, false);
   if (st != NUI_OK) return st;
   TrackState t;
