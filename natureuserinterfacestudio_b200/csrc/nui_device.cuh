@@ -422,4 +422,22 @@ __device__ __forceinline__ int round_div(float p, float c, float inv) {
   return (int)roundf(p / c);
 }
 
+// The pixel of a thread of the refinement kernels (blocks of 256 threads: 2 x 4 warps, a warp a
+// tile of TW x 32 / TW pixels), -1 outside the image.  What bounds them is the voxel reads' lines:
+// a dense volume's lie along x, so its warps take 32 pixels of a row (512^3: 22 us a frame, 24 / 27
+// / 35 with 16 / 8 / 4; 24 with a block's pixels all in one row), a voxel hash's are 8^3 blocks and
+// entries to look up, so its warps take 16 x 2 (70 us for int16 and 33 for FP16 voxels of 5 mm; 73
+// and 31 with 8 x 4, 95 and 44 with a block's pixels in one row).
+constexpr int kFinishDense = 32, kFinishHash = 16;
+template <int TW>
+struct FinishTile {
+  static constexpr int bw = 2 * TW, bh = 4 * (32 / TW);  // pixels of a block
+  __device__ __forceinline__ static int pixel(int W, int H) {
+    const int tiles_x = (W + bw - 1) / bw, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int x = ((int)blockIdx.x % tiles_x) * bw + (warp & 1) * TW + lane % TW;
+    const int y = ((int)blockIdx.x / tiles_x) * bh + (warp >> 1) * (32 / TW) + lane / TW;
+    return x < W && y < H ? y * W + x : -1;
+  }
+};
+
 }  // namespace nui

@@ -1037,8 +1037,8 @@ template <int HF>
 __global__ void __launch_bounds__(256, 4) k_hash_finish(const SessionDesc* __restrict__ descs) {
   const SessionDesc& s = descs[blockIdx.y];
   if (!s.hash || s.fwd || s.hfmt != HF || s.kind != kTrackFrame || s.ts->status != 0) return;
-  const int pid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pid >= s.W * s.H) return;
+  const int pid = FinishTile<kFinishHash>::pixel(s.W, s.H);
+  if (pid < 0) return;
   const float4 e = s.vref[pid];
   HashRead<HF> R{s, 0, 0, 0, -1};  // (a warp-shared lookup cache made this kernel slower)
   const float stepScale = s.mu * (1.0f / s.voxel) * 0.6f;

@@ -164,8 +164,8 @@ template <int FMT>
 __global__ void __launch_bounds__(256, 4) k_raycast_finish(const SessionDesc* __restrict__ descs) {
   const SessionDesc& s = descs[blockIdx.y];
   if (s.kind != kTrackFrame || s.fmt != FMT || s.ts->status != 0) return;
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= s.W * s.H) return;
+  const int id = FinishTile<kFinishDense>::pixel(s.W, s.H);
+  if (id < 0) return;
   const float4 e = s.vref[id];
   const float4 nanv = make_float4(qnan(), qnan(), qnan(), 0.f);
   float4 vout = nanv, nout = nanv;

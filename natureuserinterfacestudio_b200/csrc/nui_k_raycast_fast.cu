@@ -116,8 +116,8 @@ template <int FMT>
 __global__ void __launch_bounds__(256, 4) k_raycast_finish_fast(const SessionDesc* __restrict__ descs) {
   const SessionDesc& s = descs[blockIdx.y];
   if (s.kind != kTrackFrame || s.fmt != FMT || s.ts->status != 0) return;
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = id < s.W * s.H;
+  const int id = FinishTile<kFinishDense>::pixel(s.W, s.H);
+  const bool live = id >= 0;
   bool refined = false;
   if (live) {
     const float4 e = s.vref[id];

@@ -570,6 +570,10 @@ void launch_summaries(const BatchPlan& p, const SessionDesc* d, cudaStream_t st,
   launch_distances(p, d, st, force);
 }
 // Blocks of the raycasts: 2 x 2 warps, each a tw x (32 / tw) pixel tile.
+template <int TW>
+unsigned finish_blocks(const BatchPlan& p) {
+  return cdiv(p.maxW, FinishTile<TW>::bw) * cdiv(p.maxH, FinishTile<TW>::bh);
+}
 unsigned ray_blocks(const BatchPlan& p, int tw) { return cdiv(p.maxW, 2 * tw) * cdiv(p.maxH, 2 * (32 / tw)); }
 template <int F>
 void launch_raycast(const BatchPlan& p, const SessionDesc* d, cudaStream_t st) {
@@ -577,11 +581,11 @@ void launch_raycast(const BatchPlan& p, const SessionDesc* d, cudaStream_t st) {
   const int tw = p.tune.raycast_tile_width;
   if (F >= NUI_TSDF_F16_U8) {  // tolerance mode
     k_raycast_fast<F><<<dim3(ray_blocks(p, tw), dense_n(p)), 128, 0, st>>>(d, tw);
-    k_raycast_finish_fast<F><<<dim3(cdiv((long)p.maxW * p.maxH, 256), dense_n(p)), 256, 0, st>>>(d);
+    k_raycast_finish_fast<F><<<dim3(finish_blocks<kFinishDense>(p), dense_n(p)), 256, 0, st>>>(d);
     return;
   }
   k_raycast<F><<<dim3(ray_blocks(p, tw), dense_n(p)), 128, 0, st>>>(d, tw);
-  k_raycast_finish<F><<<dim3(cdiv((long)p.maxW * p.maxH, 256), dense_n(p)), 256, 0, st>>>(d);
+  k_raycast_finish<F><<<dim3(finish_blocks<kFinishDense>(p), dense_n(p)), 256, 0, st>>>(d);
 }
 
 void launch_hash_integrate(const BatchPlan& p, const SessionDesc* d0, cudaStream_t st) {
@@ -643,8 +647,8 @@ void launch_hash_raycast(const BatchPlan& p, const SessionDesc* d0, cudaStream_t
   const unsigned tiles = ray_blocks(p, tw);
   if (p.hashMask & 1) k_hash_raycast<0><<<dim3(tiles, hn), 128, 0, st>>>(d, tw);
   if (p.hashMask & 2) k_hash_raycast<1><<<dim3(tiles, hn), 128, 0, st>>>(d, tw);
-  if (p.hashMask & 1) k_hash_finish<0><<<dim3(px, hn), 256, 0, st>>>(d);
-  if (p.hashMask & 2) k_hash_finish<1><<<dim3(px, hn), 256, 0, st>>>(d);
+  if (p.hashMask & 1) k_hash_finish<0><<<dim3(finish_blocks<kFinishHash>(p), hn), 256, 0, st>>>(d);
+  if (p.hashMask & 2) k_hash_finish<1><<<dim3(finish_blocks<kFinishHash>(p), hn), 256, 0, st>>>(d);
 }
 
 // The shifts of the shifting volumes (after tracking, before integration): per axis, the
