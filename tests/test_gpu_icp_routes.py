@@ -3,6 +3,7 @@ and without the photometric rows, block sizes by image size -- the same poses by
 every route, at the edges of the rules -- and the shared-reciprocal quotients of the
 photometric rows against the division they replace."""
 import random
+import threading
 from fractions import Fraction
 
 import numpy as np
@@ -60,6 +61,36 @@ def test_lost_at_a_coarse_level_stays_lost(gpu_ctx):
         assert wall.work_counters()["icp_iters"][:3] == [0, 0, 1]  # lost by the first iteration of the coarsest level
     for s in (other, wall):
         s.close()
+
+
+@pytest.mark.gpu
+def test_contexts_on_threads_track_at_once():
+    """Each context's whole-device launch fills the device, and several may be launched at once
+    (threads, each with a context and its streams): every one runs to its end, with the poses it
+    gives alone."""
+    W, H = 320, 240
+    seq = frames(6, W=W, H=H, seed=5)
+    cfg = cfg_for(W=W, H=H, res=(64, 64, 64), trunc=0.1)
+
+    def run(out, laps):
+        ctx = L.Context(0)
+        for _ in range(laps):
+            s = L.Session(ctx, cfg)
+            out.append([s.process(d) for d, _, _, _ in seq])
+            s.close()
+
+    alone, many = [], [[] for _ in range(4)]
+    run(alone, 1)
+    ts = [threading.Thread(target=run, args=(o, 12)) for o in many]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    for o in many:
+        assert len(o) == 12
+        for lap in o:
+            for (ok, p), (ok0, p0) in zip(lap, alone[0]):
+                assert ok == ok0 and np.array_equal(p, p0)
 
 
 def _f32(x):
