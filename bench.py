@@ -355,7 +355,7 @@ def run_ours(args, rank, world):
             s.close()
 
     if rank == 0:
-        cpu = cpu_baseline(args) if world == 1 and not args.no_cpu else None
+        cpu = cpu_baseline_or_reason(args) if world == 1 and not args.no_cpu else None
         lat_t = np.array(per_tick)
         line = {
             "metric": METRIC,
@@ -876,10 +876,21 @@ def run_configs(args):
     return 0
 
 
+def cpu_baseline_or_reason(args, **kw):
+    """The CPU baseline, or why there is none (the reference's kernels are built from its tree)."""
+    try:
+        return cpu_baseline(args, **kw)
+    except (RuntimeError, OSError) as e:
+        return {"unavailable": str(e).splitlines()[0]}
+
+
 def run_reference(args, rank, world):
     if rank != 0:
         return 0
-    cpu = cpu_baseline(args, seconds=max(5.0, min(60.0, 3.0 * args.steps)))
+    cpu = cpu_baseline_or_reason(args, seconds=max(5.0, min(60.0, 3.0 * args.steps)))
+    if "unavailable" in cpu:
+        print(json.dumps({"impl": "reference", "unavailable": cpu["unavailable"]}))
+        return 0
     n_hash = sum(1 for i in range(args.sessions) if i % 5 >= 3)
     line = {"impl": "reference", "metric": METRIC,
             "value": cpu["value"], "unit": "frames/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
