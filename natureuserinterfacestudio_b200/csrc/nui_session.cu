@@ -187,6 +187,7 @@ struct BatchPlan {
   int maxIters[kMaxLevels];
   long maxColumns[4];  // per format: voxel columns of a volume
   long maxBricks[4];        // per format: 8^3 bricks
+  long maxTiles[4];         // per format: 32 x 8 x 8 tiles
   long maxDistBlocks;       // blocks of the brick distances, all dense formats
   long maxHashBlk;          // scan blocks of 1024 entries
   int hashMask;             // bit per hash sdf format
@@ -502,6 +503,8 @@ void plan_add(BatchPlan& p, const nui_session* s) {
   p.fmtMask |= 1 << c.tsdf_format;
   const long nb = (long)((c.res[0] + 7) / 8) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8);
   p.maxBricks[c.tsdf_format] = std::max(p.maxBricks[c.tsdf_format], nb);
+  const long nt = (long)((c.res[0] + 31) / 32) * ((c.res[1] + 7) / 8) * ((c.res[2] + 7) / 8);
+  p.maxTiles[c.tsdf_format] = std::max(p.maxTiles[c.tsdf_format], nt);
   const long db = (long)cdiv((c.res[1] + 7) / 8, kDistY) * cdiv((c.res[2] + 7) / 8, kDistZ);
   p.maxDistBlocks = std::max(p.maxDistBlocks, db);
   if (c.voxel_shift > 0) {
@@ -519,6 +522,7 @@ void plan_merge(BatchPlan& a, const BatchPlan& b) {
   for (int f = 0; f < 4; ++f) {
     a.maxColumns[f] = std::max(a.maxColumns[f], b.maxColumns[f]);
     a.maxBricks[f] = std::max(a.maxBricks[f], b.maxBricks[f]);
+    a.maxTiles[f] = std::max(a.maxTiles[f], b.maxTiles[f]);
   }
   a.maxDistBlocks = std::max(a.maxDistBlocks, b.maxDistBlocks);
   a.maxHashBlk = std::max(a.maxHashBlk, b.maxHashBlk);
@@ -537,8 +541,9 @@ unsigned dense_n(const BatchPlan& p) { return (unsigned)(p.n - p.hashTail); }
 template <int F>
 void launch_integrate(const BatchPlan& p, const SessionDesc* d, cudaStream_t st) {
   if (!(p.fmtMask & (1 << F))) return;
-  if (F >= NUI_TSDF_F16_U8) {  // tolerance mode: cull the 32 x 8 x 8 tiles, then a warp per kept tile
-    const long tiles = p.maxBricks[F] / 4 + 1;  // >= the tiles of any session of the format
+  if (F >= NUI_TSDF_F16_U8) {  // tolerance mode: cull the 32 x 8 x 8 tiles, a thread each, then a block per kept tile
+    // (not the bricks over four: a row of 40 voxels has two tiles but five bricks)
+    const long tiles = p.maxTiles[F];
     k_integrate_cull<F><<<dim3(cdiv(tiles, 256), dense_n(p)), 256, 0, st>>>(d);
     // a block a tile: enough blocks that one session's kept tiles (~2000 of a 512^3 volume's
     // 65536) spread over the SMs, no more than a few per SM of each of many

@@ -79,3 +79,22 @@ def test_exact_columns(gpu_ctx, res):
     assert np.array_equal(w[:, 1], v[:, 1]) and np.max(np.abs(w[:, 0] - v[:, 0].astype(np.int32))) <= 1
     s.close()
     f.close()
+
+
+@pytest.mark.parametrize("fmt", [L.TSDF_F16_U8, L.TSDF_F16_F16])
+@pytest.mark.parametrize("res", [(40, 160, 160), (8, 160, 200)])
+def test_rows_of_more_tiles_than_a_quarter_of_their_bricks(gpu_ctx, res, fmt):
+    """Rows that end with a tile of one to three bricks: the volume's last tiles, hundreds past a
+    quarter of its bricks, are integrated like the others (same comparison)."""
+    ntx, nbx, n = (res[0] + 31) // 32, (res[0] + 7) // 8, (res[1] // 8) * (res[2] // 8)
+    first = -(-(nbx * n // 4 + 1) // 256) * 256  # tiles from here on had no thread in the cull
+    assert first < ntx * n
+    d, _, R, t = frames(1, W=96, H=72, seed=4)[0]
+    ref = L.Session(gpu_ctx, cfg_for(W=96, H=72, res=res, fmt=L.TSDF_I16, trunc=0.2))
+    ref.upload(d)
+    ref.set_pose(R, t)
+    ref.integrate()
+    w = ref.volume_ref_layout().reshape(res[1], res[0], res[2], 2)[..., 1]
+    assert np.sum(w[:, :, 8 * -(-first // (ntx * (res[1] // 8))):] > 0) > 100  # in view
+    ref.close()
+    test_edges_of_tiles(gpu_ctx, res, fmt)
