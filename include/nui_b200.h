@@ -339,12 +339,12 @@ NUI_API nui_status nui_ctx_stage_ms(nui_ctx* ctx, int stage, float* ms);
 /* Kernel launches in the captured graph of the context's last graphed batch tick. */
 NUI_API nui_status nui_ctx_last_tick_kernels(nui_ctx* ctx, int* n);
 /* Launch shapes of a context's tick, chosen by nui_ctx_autotune (or set by hand).  No
- * choice changes a result bit except the two ICP shapes, which regroup the FP64 partial
- * sums of the normal equations (poses agree to the rounding of those sums).
+ * choice changes a result bit (the order of the ICP's FP64 sums follows from the image size
+ * alone, whatever else is in the tick).
  *   integrate_threads_log2   accepted and reported, without effect: the exact dense
  *                            integration takes 256 threads per 32 voxel columns; 14..22 (18)
- *   icp_pixels_per_thread    ICP clusters: a run of a block is its threads (256 to 1024) x this
- *                            many pixels; 2, 4, 8 or 16 (4)
+ *   icp_pixels_per_thread    accepted and reported, without effect: pixels are dealt to the
+ *                            blocks in units of the image; 2, 4, 8 or 16 (4)
  *   icp_cluster_blocks       ICP: thread blocks of the cluster that tracks one session;
  *                            2..16 (12: six SMs at two blocks an SM, so that three
  *                            clusters fill an 18-SM GPC; above 8 a non-portable size); up

@@ -18,7 +18,8 @@ constexpr int kPreBlockX = 32, kPreBlockY = 8;  // k_preprocess block: 32 x 16 p
 // Shared memory a warp stages its rows in: two arrays of 32 x 4 floats, the second 16 banks
 // on, so that the 32 lanes reading the eight components of four rows hit 32 banks.
 constexpr int kIcpHalf = 144;                       // floats from the first array to the second
-constexpr int kIcpStageBytes = (kIcpHalf + 128) * 4;  // per warp (also holds its 64 sums)
+constexpr int kIcpStageBytes = (kIcpHalf + 128) * 4;  // per warp
+constexpr int kIcpUnits = 143;  // units an image's pixels are summed in (see nui_k_icp.cu)
 constexpr int kSummaryBricks = 32;  // bricks a block of k_brick_summary looks at
 constexpr int kFastWarps = 4;  // warps per block of the tolerance-mode integration
 
@@ -79,14 +80,13 @@ struct IcpLm {
   unsigned icp_iters[kMaxLevels];
 };
 
-// The ICP of one session over many blocks (k_icp_wide): the blocks' sums (depth in 0..28,
+// The ICP of one session over many blocks (k_icp_wide): the units' sums (depth in 0..28,
 // photometric in 32..60) of an even and an odd iteration, the blocks' arrivals in the iterations
 // and the blocks that have left (zero between launches), and whether a wait ran out.
-constexpr int kIcpWideBlocks = 160;  // blocks a session, at most
 constexpr int kIcpWideSessions = 4;  // sessions a launch, at most
 constexpr int kIcpPolls = 1 << 21;   // polls of the arrivals a block makes (each ~0.4 us)
 struct IcpWide {
-  double part[2][kIcpWideBlocks][64];
+  double part[2][kIcpUnits][64];
   unsigned arrived, left, stalled;
 };
 

@@ -380,25 +380,21 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
       : "d"(a), "d"(b));
 }
 
-// What a depth pass reads for every pixel: held in registers through the pass (the barriers
-// of the staging would have it loaded again for each pixel).
-struct IcpView {
-  const float4 *nref, *vref;
-  float fx, fy, cx, cy;      // full-resolution intrinsics
-  float fxi, fyi, cxl, cyl;  // the level's, as level_vertex forms them
-  float fW, fH, thr;
-  int W, N;
-  __device__ __forceinline__ IcpView(const SessionDesc& s, int level)
-      : nref(s.nref), vref(s.vref), fx(s.cam.fx), fy(s.cam.fy), cx(s.cam.cx), cy(s.cam.cy),
-        fxi((float)(1 << level) * s.cam.fx_inv), fyi((float)(1 << level) * s.cam.fy_inv),
-        cxl(s.cam.cx / (float)(1 << level)), cyl(s.cam.cy / (float)(1 << level)), fW((float)s.W), fH((float)s.H),
-        thr(s.dist_thr), W(s.W), N(s.W * s.H) {}
-};
-// The running estimate and the previous camera pose (the reference maps' frame), a row and
-// its translation a float4: R | t, and R_inv | t.
+// What a depth pass reads for every pixel, in shared memory (the pass's registers are all taken:
+// held there, the intrinsics had other values spilled in its loop): the running estimate and the
+// previous camera pose (the reference maps' frame), a row and its translation a float4, R | t and
+// R_inv | t; fx, fy, cx, cy; and a level's 1 / fx, 1 / fy, cx, cy as level_vertex forms them.
 struct IcpPoses {
-  float4 cur[3], prev[3];
+  float4 cur[3], prev[3], cam, lvl[kMaxLevels];
 };
+__device__ __forceinline__ void icp_cameras(IcpPoses& P, const SessionDesc& s) {  // a level a thread
+  const int l = threadIdx.x;
+  if (l == 0) P.cam = make_float4(s.cam.fx, s.cam.fy, s.cam.cx, s.cam.cy);
+  if (l < kMaxLevels) {
+    const float div = (float)(1 << l);
+    P.lvl[l] = make_float4(div * s.cam.fx_inv, div * s.cam.fy_inv, s.cam.cx / div, s.cam.cy / div);
+  }
+}
 // Fills three rows from a matrix and a translation (a row's column a thread, 12 threads).
 __device__ __forceinline__ void icp_pose_rows(float4* rows, const float* R, const float* t) {
   const int k = threadIdx.x >> 2, c = threadIdx.x & 3;
@@ -408,165 +404,333 @@ __device__ __forceinline__ float dot_row(float4 r, float3 v) { return dot3(f3(r.
 
 // The row of one pixel (level pixel (x, y) at depth dep): false without a match, else
 // [n x p, n | n.(q - p), 1].
-__device__ __forceinline__ bool icp_depth_row(const IcpView& c, int x, int y, float dep, const IcpPoses& P,
-                                              float4& ra, float4& rb) {
+__device__ __forceinline__ bool icp_depth_row(const SessionDesc& s, int level, int x, int y, float dep,
+                                              const IcpPoses& P, float4& ra, float4& rb) {
   if (isnan(dep)) return false;
-  const float3 v = f3(dep * (((float)x - c.cxl) * c.fxi), dep * (((float)y - c.cyl) * c.fyi), dep);  // level_vertex
+  const float4 k = P.lvl[level];
+  const float3 v = f3(dep * (((float)x - k.z) * k.x), dep * (((float)y - k.w) * k.y), dep);  // level_vertex
   const float4 r0 = P.cur[0], r1 = P.cur[1], r2 = P.cur[2];
   const float3 pv = f3(dot_row(r0, v) + r0.w, dot_row(r1, v) + r1.w, dot_row(r2, v) + r2.w);
   const float4 q0 = P.prev[0], q1 = P.prev[1], q2 = P.prev[2];
   const float3 pd = f3(pv.x - q0.w, pv.y - q1.w, pv.z - q2.w);
   const float3 pp = f3(dot_row(q0, pd), dot_row(q1, pd), dot_row(q2, pd));
-  const float u = pp.x * c.fx / pp.z + c.cx;
-  const float vv = pp.y * c.fy / pp.z + c.cy;
-  if (!(u >= 0.0f && u < c.fW && vv >= 0.0f && vv < c.fH)) return false;
+  const float4 c = P.cam;
+  const float u = pp.x * c.x / pp.z + c.z;
+  const float vv = pp.y * c.y / pp.z + c.w;
+  const int W = s.W, H = s.H;
+  if (!(u >= 0.0f && u < (float)W && vv >= 0.0f && vv < (float)H)) return false;
   // both maps sampled at once (their eight loads in flight together), then tested: a hole
   // of either makes the distance or the residual NaN
-  const float3 rn = bilinear_holes(c.nref, u, vv, c.W, c.N);
-  const float3 rv = bilinear_holes(c.vref, u, vv, c.W, c.N);
+  const float3 rn = bilinear_holes(s.nref, u, vv, W, W * H);
+  const float3 rv = bilinear_holes(s.vref, u, vv, W, W * H);
   const float3 diff = sub3(rv, pv);
   const float dist = sqrtf(dot3(diff, diff)), res = dot3(rn, diff);
-  if (!(dist < c.thr) || isnan(res)) return false;
+  if (!(dist < s.dist_thr) || isnan(res)) return false;
   const float3 r = cross3(rn, pv);
   ra = make_float4(r.x, r.y, r.z, rn.x);
   rb = make_float4(rn.y, rn.z, res, 1.0f);
   return true;
 }
 
-// How a level's pixels are dealt: runs of T x per pixels, of which this thread's part (a block
-// or a warp of T threads, thread `tid` of it) takes run `rank`, rank + C, ...
-struct IcpDeal {
-  int T, tid, per, rank, C;
+// ---------------------------------------------------------------- the order of the sums
+// The FP64 sums of an image's pixels are formed in an order that its size alone fixes, so a
+// session's poses do not depend on how many blocks track it, on how wide they are or on the other
+// sessions of the launch.  The pixels are cut into runs of 32 (one a lane) and leaves of a few
+// consecutive runs.  Leaves u, u + 143, u + 286, ... are unit u, at most 32 of them (photometric
+// rows: 12, as a leaf ends with 31 exchanges between the lanes, and their blocks have half the
+// warps).  A leaf's rows are summed by one warp, run by run; a unit's leaves by the binary tree
+// that joins those whose place differs in its highest bit first; and the units in fixed groups of
+// nine, these by such a tree.  Blocks take whole units, and whichever stages fall to a thread, a
+// warp or a block, the sums are the same (a leaf that does not exist adds zero, which changes no
+// bit).
+//
+// 143 units are a block on each of 143 of the 148 SMs for one session, on 72 for each of two, on 36
+// for each of four, and twelve each for a cluster of twelve; consecutive leaves in consecutive
+// units keep a block on neighbouring pixels (such a cluster's on 1152 of every 13728 at 640 x 480)
+// and spread every part of the image over all units.  143 is odd: with 144 a unit's photometric
+// leaves lay in the same columns of a 640 x 480 image (sixteen such sessions: 1558 us against 1497).
+// What it costs: with sums that followed the launch's shape a 640 x 480 depth session took 77 us
+// alone and sixteen 234, now 82 and 255; colour-tracked 150 and 1312, now 167 and 1428.
+struct IcpCut {
+  int g, leaves, units;  // runs a leaf; leaves of the image; units that have any
+  __device__ __forceinline__ IcpCut() {}
+  // n pixels in at most `most` leaves of at least `least` runs
+  __device__ __forceinline__ IcpCut(int n, int most, int least) {
+    const int runs = (n + 31) >> 5;
+    g = max(least, (runs + most - 1) / most);
+    leaves = (runs + g - 1) / g;
+    units = min(kIcpUnits, leaves);
+  }
+  __device__ __forceinline__ int of(int u) const { return (leaves - u + kIcpUnits - 1) / kIcpUnits; }  // unit u's leaves
 };
 
-// The depth rows of the level's pixels that fall to this thread's part, their outer products added to the warp's 8 x 8 FP64
-// sums (d0, d1: this lane's two of them).  The 29 sums of a pixel are the upper triangle of
-// the outer product of [row, 1]: JtJ, Jtr, r^2 and the count.  The rows' FP32 values are
-// widened, so every product is exact and only the sums round.
+// The leaves of n consecutive units from u on as tasks, dealt to the block's warps in turn, row by
+// row of the units (leaf j of each, then leaf j + 1), so that a later task has a later leaf.  A
+// task's number is its slot, so there are at most kIcpRoom and, past the end, a block's warps more.
+struct IcpDeal {
+  int n;
+  unsigned recip;  // 2^20 / n and less than one more: exact quotients by n of such numbers
+  __device__ __forceinline__ void form(int n_) { n = n_, recip = (1u << 20) / (unsigned)n_ + 1u; }
+  __device__ __forceinline__ int leaf(int u, int task) const {
+    return (int)((unsigned)task * recip >> 20) * (kIcpUnits - n) + u + task;
+  }
+};
+// What a block does in the passes over one image: its units, as many at a time as have room for
+// their leaves' sums in the slots, and the deals of those and of the rest.  Formed once for all
+// iterations, each of which its divisions would cost a microsecond.
+struct IcpPlan {
+  IcpCut cut;
+  int u0, mine;
+  IcpDeal deal[2];
+  __device__ __forceinline__ static int first(const IcpCut& c, int rank, int parts) { return rank * c.units / parts; }
+  __device__ __forceinline__ void form(const IcpCut& c, int rank, int parts, int room) {
+    const int f = first(c, rank, parts), n = first(c, rank + 1, parts) - f, at_once = max(1, min(n, room / c.of(0)));
+    deal[0].form(at_once);
+    deal[1].form(max(1, n % at_once));
+    cut = c, u0 = f, mine = n;
+  }
+};
+// The plans of a session's levels, and of its photometric rows, a thread each, and whose each unit
+// is (its block, and its place there).
+__device__ __forceinline__ IcpCut icp_cut(const SessionDesc& s, int q) {
+  return q < kMaxLevels ? IcpCut((s.W >> q) * (s.H >> q), 32 * kIcpUnits, 1) : IcpCut(s.W * s.H, 12 * kIcpUnits, 2);
+}
+__device__ __forceinline__ void icp_plans(const SessionDesc& s, IcpPlan* plans, bool color, int rank, int parts, int room) {
+  const int q = (int)threadIdx.x;
+  if (q < s.levels || (q == kMaxLevels && color)) plans[q].form(icp_cut(s, q), rank, parts, room);
+}
+__device__ __forceinline__ void icp_owners(const SessionDesc& s, unsigned short (*owner)[kIcpUnits], bool color, int parts) {
+  for (int i = threadIdx.x; i < (kMaxLevels + 1) * kIcpUnits; i += blockDim.x) {
+    const int q = i / kIcpUnits, u = i % kIcpUnits;
+    if (q >= s.levels && !(q == kMaxLevels && color)) continue;
+    const IcpCut c = icp_cut(s, q);
+    const int r = ((u + 1) * parts - 1) / c.units;
+    if (u < c.units) owner[q][u] = (unsigned short)(r << 8 | (u - IcpPlan::first(c, r, parts)));
+  }
+}
+
+// The terms of the 29 that a lane's two sums of a warp's 8 x 8 are, -1: none.
+__device__ __forceinline__ int icp_lane_term(int i, int j) {
+  if (i < 6) return j >= i && j < 7 ? 7 * i - i * (i - 1) / 2 + j - i : -1;
+  return i == j ? 21 + i : -1;
+}
+
+// The depth rows of the units of a deal, from u0 on, their outer products added to a warp's 8 x 8
+// FP64 sums (d0, d1: this lane's two of them) leaf by leaf.  The 29 sums of a pixel
+// are the upper triangle of the outer product of [row, 1]: JtJ, Jtr, r^2 and the count.  The rows'
+// FP32 values are widened, so every product is exact and only the sums round.
 //
 // The pass waits on its eight map gathers.  The sums of a warp take two doubles a lane instead
 // of 29 a thread (58 registers), which lets 1024 threads of 64 registers share an SM instead of
 // 512 of 128, so twice the warps wait at once (track at 640 x 480: 337 -> 281 us; 39 sessions:
 // 164 -> 147 M warp instructions a launch).
-__device__ __forceinline__ void icp_depth_pass(const SessionDesc& s, int level, const IcpDeal& deal,
-                                               const IcpPoses& P, float* stage, double& d0, double& d1) {
-  const IcpView view(s, level);
+__device__ __forceinline__ void icp_depth_pass(const SessionDesc& s, int level, const IcpCut& cut, const IcpDeal& deal,
+                                               int u0, const IcpPoses& P, float* stage, double* slots) {
   const int w = s.W >> level, n = w * (s.H >> level);
   const float* __restrict__ Dl = s.dlev[level];
-  const int T = deal.T, per = deal.per, C = deal.C, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   const int c = lane >> 2, src = (lane & 3) * 4 + (c < 4 ? c : kIcpHalf + c - 4);
   float4* const sa = reinterpret_cast<float4*>(stage) + lane;
   float4* const sb = reinterpret_cast<float4*>(stage + kIcpHalf) + lane;
-  // the next pixel's depth is in flight while the current one's row forms; a pixel's column
-  // and row advance with its index, by T within a run and by the rest of the other blocks'
-  // runs after it
-  const int jump = T * ((C - 1) * per + 1), ty = T / w, tx = T - ty * w, jy = jump / w, jx = jump - jy * w;
-  int base = deal.rank * T * per, k = 0;
-  int i = base + deal.tid, y = i / w, x = i - y * w;
+  const int terms = (icp_lane_term(c, 2 * (lane & 3)) & 0xff) | icp_lane_term(c, 2 * (lane & 3) + 1) << 8;
+  // a pixel's row: its index over the width, rounded down by a reciprocal of 32 bits that is one
+  // too large at most
+  const unsigned recip = 0xffffffffu / (unsigned)w + 1u;
+  int task = (int)(threadIdx.x >> 5), leaf = deal.leaf(u0, task);
+  int left = cut.g, i = leaf * left * 32 + lane;  // (runs past the image's end have no pixel)
   float dn = i < n ? __ldg(Dl + i) : qnan();
-  while (base < n) {
-    const int cx = x, cy = y;
+  double d0 = 0.0, d1 = 0.0;
+  while (leaf < cut.leaves) {
     const float dep = dn;
-    const bool step = ++k < per;
-    if (!step) {
-      k = 0;
-      base += C * T * per;
+    int y = (int)__umulhi((unsigned)i, recip), x = i - y * w;
+    if (x < 0) x += w, --y;
+    // the next pixel's depth is in flight while the current one's row forms
+    double* const slot = slots + task * kIcpTerms;
+    const bool ends = --left == 0;
+    i += 32;
+    if (ends) {
+      task += (int)(blockDim.x >> 5);
+      leaf = deal.leaf(u0, task);
+      left = cut.g;
+      i = leaf * left * 32 + lane;
     }
-    i += step ? T : jump;
-    x += step ? tx : jx;
-    y += step ? ty : jy;
-    if (x >= w) x -= w, ++y;
     dn = i < n ? __ldg(Dl + i) : qnan();
     float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb = ra;
-    const bool ok = icp_depth_row(view, cx, cy, dep, P, ra, rb);
-    if (!__any_sync(0xffffffffu, ok)) continue;
-    *sa = ra;
-    *sb = rb;
-    __syncwarp();
+    const bool ok = icp_depth_row(s, level, x, y, dep, P, ra, rb);
+    if (__any_sync(0xffffffffu, ok)) {
+      *sa = ra;
+      *sb = rb;
+      __syncwarp();
 #pragma unroll
-    for (int g = 0; g < 8; ++g) {
-      const double x = (double)stage[16 * g + src];
-      dmma(d0, d1, x, x);
+      for (int q = 0; q < 8; ++q) {
+        const double v = (double)stage[16 * q + src];
+        dmma(d0, d1, v, v);
+      }
+      __syncwarp();
     }
-    __syncwarp();
+    if (ends) {
+      if ((terms & 0xff) != 0xff) slot[terms & 0xff] = d0;
+      if (terms >= 0) slot[terms >> 8] = d1;
+      d0 = d1 = 0.0;
+    }
   }
 }
 
-// The photometric rows of the model points that fall to this thread's part, their 28 FP32 terms and
-// the count added to this thread's FP64 sums.
-__device__ __forceinline__ void icp_color_pass(const SessionDesc& s, const IcpDeal& deal, const IcpPoses& P,
-                                               double (&acc)[kIcpTerms]) {
-  const int NM = s.W * s.H, T = deal.T, per = deal.per;
+// The photometric rows of the model points of the units of a deal, their 28 FP32 terms and the
+// count added to a lane's FP64 sums; a leaf's by a reduce-scatter over the warp's lanes,
+// terms padded to 32: at each of five steps a lane keeps half of its values, sends the other half
+// to its partner and adds what it receives, so lane k ends with the leaf's sum of term k after 31
+// exchanges.
+__device__ __forceinline__ void icp_color_pass(const SessionDesc& s, const IcpCut& cut, const IcpDeal& deal, int u0,
+                                               const IcpPoses& P, double* slots) {
+  const int NM = s.W * s.H, lane = threadIdx.x & 31;
   const float4 r0 = P.cur[0], r1 = P.cur[1], r2 = P.cur[2];
   const float R[9] = {r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r2.x, r2.y, r2.z};
   const float3 tc = f3(r0.w, r1.w, r2.w);
 #pragma unroll 1
-  for (int base = deal.rank * T * per; base < NM; base += deal.C * T * per)
+  for (int task = (int)(threadIdx.x >> 5), leaf; (leaf = deal.leaf(u0, task)) < cut.leaves; task += (int)(blockDim.x >> 5)) {
+    double acc[kIcpTerms];
+#pragma unroll
+    for (int q = 0; q < kIcpTerms; ++q) acc[q] = 0.0;
+    const int i0 = leaf * cut.g * 32 + lane, i1 = min(NM, i0 + 32 * cut.g);
 #pragma unroll 1
-    for (int k = 0; k < per; ++k) {
-      const int i = base + k * T + deal.tid;
+    for (int i = i0; i < i1; i += 32) {
       ColorRow row;
-      if (i >= NM || !color_row(s, i, R, tc, row)) continue;
+      if (!color_row(s, i, R, tc, row)) continue;
       row.add_to(acc);
     }
+    double v[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) v[q] = q < kIcpTerms ? acc[q] : 0.0;
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1) {
+      const bool upper = lane & half;
+#pragma unroll
+      for (int j = 0; j < half; ++j) {
+        const double send = upper ? v[j] : v[j + half];
+        const double keep = upper ? v[j + half] : v[j];
+        v[j] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+      }
+    }
+    if (lane < kIcpTerms) slots[task * kIcpTerms + lane] = v[0];
+  }
 }
 
-// Block sums from the warps' sums, each warp's left in its part of the staging memory: the
-// lanes of a warp are dealt over 32 / warps terms (icp_my_term), a lane takes a warp's term (at
-// index `at` of its 64 doubles) and the lanes add up pairwise; every lane of a term's group
-// gets its sum.  (A thread a term, adding the warps one after another, took 0.9 us of 32 warps.)
-// All threads must call it; the block has 8, 16 or 32 warps.
+// The last stages of a tree by a group of lanes, as many as the block has warps (8, 16 or 32), of
+// which there are 32: a group a term (icp_my_term), a lane an entry; every lane gets the sum.
 __device__ __forceinline__ int icp_my_term() { return (int)(threadIdx.x / (blockDim.x >> 5)); }
+__device__ __forceinline__ int icp_my_entry() { return (int)(threadIdx.x & ((blockDim.x >> 5) - 1)); }
 __device__ __forceinline__ double icp_group_sum(double v) {
   for (int off = (int)(blockDim.x >> 6); off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
 }
-__device__ __forceinline__ double icp_warps_sum(const float* stage0, int at) {
-  const int src = (int)(threadIdx.x & ((blockDim.x >> 5) - 1));
-  __syncthreads();
-  const double v = reinterpret_cast<const double*>(stage0 + src * (kIcpStageBytes / 4))[at];
-  __syncthreads();  // the staging memory is used again
-  return icp_group_sum(v);
-}
 
-// The block's sums of one pass, this thread's term (icp_my_term, at `at` of a warp's 64 for the
-// depth rows): of the depth rows, and of the photometric ones.  All threads must call it.
-__device__ __forceinline__ double icp_depth_sums(const SessionDesc& s, int level, const IcpDeal& deal,
-                                                 const IcpPoses& P, float* stage0, int at) {
-  float* const stage = stage0 + (threadIdx.x >> 5) * (kIcpStageBytes / 4);  // this warp's
-  double* const wsum = reinterpret_cast<double*>(stage);
-  const int lane = threadIdx.x & 31;
-  double d0 = 0.0, d1 = 0.0;
-  icp_depth_pass(s, level, deal, P, stage, d0, d1);
-  wsum[2 * lane] = d0;
-  wsum[2 * lane + 1] = d1;
-  return icp_warps_sum(stage0, at);
-}
-// (a warp's sums by a reduce-scatter over its lanes, terms padded to 32: at each of five
-// steps a lane keeps half of its values, sends the other half to its partner and adds what it
-// receives, so lane k ends with the warp's sum of term k after 31 exchanges)
-__device__ __forceinline__ double icp_color_sums(const SessionDesc& s, const IcpDeal& deal, const IcpPoses& P,
-                                                 float* stage0) {
-  double acc[kIcpTerms];
+// Unit sums from the leaves' in the slots, handed to put(unit, term, sum): a term of a unit by a
+// group of as many lanes as the block has warps, or by four, two or one, as they suffice.
+template <class Put>
+__device__ __forceinline__ void icp_unit_sums(const IcpCut& cut, int u0, int kc, const double* slots, Put put) {
+  __syncthreads();
+  if (kc < 3) {
+    const int t = icp_my_term(), e = icp_my_entry(), warps = (int)(blockDim.x >> 5);
+    for (int k = 0; k < kc; ++k) {
+      const int have = t < kIcpTerms ? cut.of(u0 + k) : 0;
+      auto at = [&](int j) { return j < have ? slots[(j * kc + k) * kIcpTerms + t] : 0.0; };
+      double v = at(e);
+      if (warps < 32) v += at(e + 16);
+      if (warps < 16) v += at(e + 8) + at(e + 24);
+      v = icp_group_sum(v);
+      if (e == 0 && t < kIcpTerms) put(u0 + k, t, v);
+    }
+  } else {
+    const bool few = cut.of(0) <= 8;
+    const int log = kc * 128 <= (int)blockDim.x ? 2 : kc * 64 <= (int)blockDim.x ? 1 : 0;
+    for (int i = threadIdx.x; i < kc * 32 << log; i += blockDim.x) {
+      const int o = i & ((1 << log) - 1), t = i >> log & 31, k = i >> log >> 5, have = t < kIcpTerms ? cut.of(u0 + k) : 0;
+      const double* const p = slots + k * kIcpTerms + t;
+      auto eight = [&](int j) {  // leaves j, j + 4, ..., j + 28
+        if (few) return (j < have ? p[j * kc * kIcpTerms] : 0.0) + (j + 4 < have ? p[(j + 4) * kc * kIcpTerms] : 0.0);
+        double v[8];
 #pragma unroll
-  for (int k = 0; k < kIcpTerms; ++k) acc[k] = 0.0;
-  icp_color_pass(s, deal, P, acc);
-  const int lane = threadIdx.x & 31;
-  double v[32];
-#pragma unroll
-  for (int k = 0; k < 32; ++k) v[k] = k < kIcpTerms ? acc[k] : 0.0;
-#pragma unroll
-  for (int half = 16; half > 0; half >>= 1) {
-    const bool upper = lane & half;
-#pragma unroll
-    for (int j = 0; j < half; ++j) {
-      const double send = upper ? v[j] : v[j + half];
-      const double keep = upper ? v[j + half] : v[j];
-      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+        for (int m = 0; m < 8; ++m) v[m] = j + 4 * m < have ? p[(j + 4 * m) * kc * kIcpTerms] : 0.0;
+        return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+      };
+      double a = eight(o);
+      if (log == 2) {
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+      } else {
+        a += eight(o + 2);
+      }
+      if (log > 0) {
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+      } else {
+        const double b = eight(1);
+        a += b + eight(3);
+      }
+      if (o == 0 && t < kIcpTerms) put(u0 + k, t, a);
     }
   }
-  reinterpret_cast<double*>(stage0 + (threadIdx.x >> 5) * (kIcpStageBytes / 4))[lane] = v[0];
-  return icp_warps_sum(stage0, icp_my_term());
+  __syncthreads();  // the slots are used again
+}
+
+// The sums of the block's units of one pass.  All threads must call it; the block has 8, 16 or 32
+// warps (photometric rows: 8 or 16).
+template <class Put>
+__device__ __forceinline__ void icp_depth_sums(const SessionDesc& s, int level, const IcpPlan& plan, const IcpPoses& P,
+                                               float* stage0, double* slots, Put put) {
+  for (int done = 0; done < plan.mine; done += plan.deal[0].n) {
+    const IcpDeal& deal = plan.deal[done + plan.deal[0].n > plan.mine];
+    const int u = plan.u0 + done;
+    icp_depth_pass(s, level, plan.cut, deal, u, P, stage0 + (threadIdx.x >> 5) * (kIcpStageBytes / 4), slots);
+    icp_unit_sums(plan.cut, u, deal.n, slots, put);
+  }
+}
+template <class Put>
+__device__ __forceinline__ void icp_color_sums(const SessionDesc& s, const IcpPlan& plan, const IcpPoses& P, double* slots,
+                                               Put put) {
+  for (int done = 0; done < plan.mine; done += plan.deal[0].n) {
+    const IcpDeal& deal = plan.deal[done + plan.deal[0].n > plan.mine];
+    const int u = plan.u0 + done;
+    icp_color_pass(s, plan.cut, deal, u, P, slots);
+    icp_unit_sums(plan.cut, u, deal.n, slots, put);
+  }
+}
+
+// The image's sums from its units': get(u, t) reads term t of unit u (the photometric terms from 32
+// on).  A warp joins half a group of nine units, a group, or two groups 8 apart (of 32, 16 or 8
+// warps), a lane a term; then as above.  The photometric normal equations and residual enter weighted, the count stays the
+// depth count.  All threads must call it.
+template <bool COLOR, class Get>
+__device__ __forceinline__ void icp_image_sums(const SessionDesc& s, const IcpCut& cut, const IcpCut& ccut, bool photo,
+                                               float* stage0, double* sums, Get get) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5);
+  double* const w = reinterpret_cast<double*>(stage0);
+  auto joined = [&](int units, int t) {
+    auto at = [&](int u) { return u < units && lane < kIcpTerms ? get(u, t) : 0.0; };
+    static_assert(kIcpUnits <= 9 * 16, "the order of the units' sums");
+    auto half0 = [&](int u) {  // units u, u + 16, u + 32, u + 48 and u + 128
+      const double v0 = at(u), v1 = at(u + 16), v2 = at(u + 32), v3 = at(u + 48), v8 = at(u + 128);
+      return ((v0 + v1) + (v2 + v3)) + v8;
+    };
+    auto half1 = [&](int u) {  // the other four of its sixteenth
+      const double v4 = at(u + 64), v5 = at(u + 80), v6 = at(u + 96), v7 = at(u + 112);
+      return (v4 + v5) + (v6 + v7);
+    };
+    if (!COLOR && warps == 32) return warp < 16 ? half0(warp) : half1(warp - 16);
+    double a = half0(warp) + half1(warp);
+    if (warps == 8) a += half0(warp + 8) + half1(warp + 8);
+    return a;
+  };
+  w[33 * warp + lane] = joined(cut.units, lane);
+  if (COLOR && photo) w[33 * (warps + warp) + lane] = joined(ccut.units, 32 + lane);
+  __syncthreads();
+  const int term = icp_my_term(), e = icp_my_entry();
+  double a = icp_group_sum(w[33 * e + term]);
+  if (COLOR && photo) {
+    const double c = icp_group_sum(w[33 * (warps + e) + term]);
+    if (term < kIcpTerms - 1) a += (double)s.photo_w * c;
+  }
+  if (e == 0) sums[term] = a;
+  __syncthreads();  // (the staging memory is used again)
 }
 
 // NuiKinfuOpenCLShiftScene::integrateVolume -> shiftVolume (NuiKinfuOpenCLShiftScene.cpp:
@@ -674,23 +838,23 @@ __global__ void k_track_end(const SessionDesc* __restrict__ descs, int fam, cons
 // All ICP iterations of every level of one frame, one thread-block cluster per session
 // (NuiKinfuOpenCLDepthTracker::IterativeClosestPoint, NuiKinfuOpenCLDepthTracker.cpp:240-504).
 // The C blocks of a cluster (C = 2..16, a launch attribute: the ICP tuning's blocks per
-// session) share the level's pixels (runs of blockDim.x x per pixels); every iteration each
-// block reduces its FP64 sums into its own shared memory, a cluster barrier makes them
-// visible, block 0 adds the blocks' sums in rank order through distributed shared memory and
-// runs the host step (LM accept/reject, FP64 Cholesky, pose update), and a second barrier
-// publishes the new estimate, which every block reads from block 0's shared memory.  The
-// hardware schedules a cluster's blocks together and its barriers need no polling; every
-// block takes the same exits at the same points, since each decision comes from block 0's
-// published state.  One launch per tick replaces one launch per iteration, and sessions
-// whose levels stop early leave their SMs to the others.
+// session) share the level's units; every iteration each block leaves its units' sums in its own
+// shared memory, a cluster barrier makes them visible, block 0 adds them up through distributed
+// shared memory and runs the host step (LM accept/reject, FP64 Cholesky, pose update), and a
+// second barrier publishes the new estimate, which every block reads from block 0's shared
+// memory.  The hardware schedules a cluster's blocks together and its barriers need no polling;
+// every block takes the same exits at the same points, since each decision comes from block 0's
+// published state.  One launch per tick replaces one launch per iteration, and sessions whose
+// levels stop early leave their SMs to the others.
 //
-// The block size is the launch's (256, 512 or 1024 threads, see launch_track): the same code
-// with kIcpStageBytes of dynamic shared memory a warp.  Launches without a colour-tracked
-// session take the variant without the photometric rows (64 registers, up to 1024 threads);
-// the rows' 29 FP64 sums a thread need 128 (up to 512).
+// The block size is the launch's (256, 512 or 1024 threads, see launch_icp_cluster): the same
+// code with kIcpStageBytes of dynamic shared memory a warp, slots for `room` leaves and the sums
+// of the block's units behind them.  Launches without a colour-tracked session take the
+// variant without the photometric rows (64 registers, up to 1024 threads); the rows' 29 FP64
+// sums a thread need 128 (up to 512).
 template <bool COLOR>
 __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
-    k_icp_cluster(const SessionDesc* __restrict__ descs, int fam, int ppt) {
+    k_icp_cluster(const SessionDesc* __restrict__ descs, int fam, int room) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const SessionDesc& s = descs[blockIdx.y];
@@ -699,50 +863,39 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
   const int rank = (int)cluster.block_rank(), C = (int)cluster.num_blocks();
   extern __shared__ __align__(16) float icp_stage[];
   __shared__ IcpPoses P;
-  __shared__ double part[2][32];  // this block's depth / photometric sums
-  __shared__ double sums[kIcpTerms];
+  __shared__ double sums[32];
   __shared__ IcpLm lm;  // block 0: the tracker state during the kernel
   __shared__ IcpStepScratch hw;  // block 0: the LM step's intermediate values
+  __shared__ IcpPlan plans[kMaxLevels + 1];  // of the levels, and of the photometric rows
+  __shared__ unsigned short owner[kMaxLevels + 1][kIcpUnits];  // whose each unit is, and its place there
+  double* const slots = reinterpret_cast<double*>(icp_stage + (blockDim.x >> 5) * (kIcpStageBytes / 4));
+  icp_plans(s, plans, COLOR, rank, C, room);
+  if (rank == 0) icp_owners(s, owner, COLOR, C);
+  // this block's units' sums: depth, then photometric
+  constexpr int kCols = COLOR ? 64 : 32;
+  double* const mine = slots + room * kIcpTerms;
   icp_pose_rows(P.cur, ts->R, ts->t);
   icp_pose_rows(P.prev, ts->xf.R_inv, ts->xf.t);
+  icp_cameras(P, s);
   const int status0 = ts->status;
   if (rank == 0) lm_copy(&lm, ts);
   // every block has read the initial state before block 0 writes any of it
   cluster.sync();
   if (status0 != 0) return;
-  const int term = icp_my_term(), at = icp_term_at(term);
-  const bool writes = term < kIcpTerms && (threadIdx.x & ((blockDim.x >> 5) - 1)) == 0;  // a thread a term
   for (int level = s.levels - 1; level >= 0; --level) {
-    // runs no longer than leave every block one: a level's few runs would otherwise fall
-    // unevenly on the cluster's blocks (19 runs of 1024 pixels for 16 at 160 x 120), and a
-    // pass waits for its slowest block
-    const int per = max(1, min(ppt, (s.W >> level) * (s.H >> level) / (C * (int)blockDim.x)));
-    const IcpDeal deal{(int)blockDim.x, (int)threadIdx.x, per, rank, C};
     const bool photo = COLOR && s.photo_w > 0.f && level == 0;
+    const IcpPlan &plan = plans[level], &cplan = plans[kMaxLevels];
     for (int iter = 0; iter < s.iters[level]; ++iter) {
-      double D = icp_depth_sums(s, level, deal, P, icp_stage, at);
-      if (writes) part[0][term] = D;
-      if (photo) {
-        D = icp_color_sums(s, deal, P, icp_stage);
-        if (writes) part[1][term] = D;
-      }
+      icp_depth_sums(s, level, plan, P, icp_stage, slots, [&](int u, int t, double v) { mine[(u - plan.u0) * kCols + t] = v; });
+      if (photo) icp_color_sums(s, cplan, P, slots, [&](int u, int t, double v) { mine[(u - cplan.u0) * kCols + 32 + t] = v; });
       cluster.sync();  // every block's sums are visible to block 0
-      if (rank == 0 && threadIdx.x < 64) {
-        if (threadIdx.x < kIcpTerms) {
-          // the blocks' sums in rank order; the photometric normal equations and residual
-          // enter weighted, the count stays the depth count
-          double a = 0.0, c = 0.0;
-          for (int r = 0; r < C; ++r) {
-            const double* pr = cluster.map_shared_rank(&part[0][0], r);
-            a += pr[threadIdx.x];
-            if (photo) c += pr[32 + threadIdx.x];
-          }
-          if (photo && threadIdx.x < kIcpTerms - 1) a += (double)s.photo_w * c;
-          sums[threadIdx.x] = a;
-        }
-        icp_step_sync();
+      if (rank == 0) {
         if (threadIdx.x == 0) lm.icp_iters[level] += 1u;
-        icp_host_step(&lm, hw, sums, iter, s.icp_min_count[level]);
+        icp_image_sums<COLOR>(s, plan.cut, cplan.cut, photo, icp_stage, sums, [&](int u, int t) {
+          const unsigned o = owner[t < 32 ? level : kMaxLevels][u];
+          return cluster.map_shared_rank(mine, o >> 8)[(o & 255) * kCols + t];
+        });
+        if (threadIdx.x < 64) icp_host_step(&lm, hw, sums, iter, s.icp_min_count[level]);
       }
       cluster.sync();  // block 0's new estimate is visible to every block
       // (block 0 writes its state again only behind the next iteration's first barrier)
@@ -764,9 +917,9 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
 
 // All ICP iterations of a small batch's sessions, each over its share of the whole device (a
 // block an SM, launched cooperatively: all blocks are resident, so they may wait for one
-// another).  Every iteration a block leaves its sums in the session's part of `work` and counts
-// itself in; when all have, every block adds all the sums, in the same order, and runs the LM
-// step on its own copy of the state, so nothing has to be sent back.  A wait that runs out (it
+// another).  Every iteration a block leaves its units' sums in the session's part of `work` and
+// counts itself in; when all have, every block adds all the sums, in the same order, and runs the
+// LM step on its own copy of the state, so nothing has to be sent back.  A wait that runs out (it
 // cannot with all blocks resident) marks the workspace and loses the frame, as every later launch
 // on the workspace does at once.
 //
@@ -778,7 +931,7 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
 // one 20.
 template <bool COLOR>
 __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
-    k_icp_wide(const SessionDesc* __restrict__ descs, int fam, IcpWide* __restrict__ work, const TrackOut out) {
+    k_icp_wide(const SessionDesc* __restrict__ descs, int fam, int room, IcpWide* __restrict__ work, const TrackOut out) {
   const SessionDesc& s = descs[blockIdx.y];
   if (!in_family(s, fam)) return;  // (this and the next: the same for every block of the session)
   if (s.kind != kTrackFrame) {
@@ -793,32 +946,30 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
   __shared__ IcpLm lm;
   __shared__ IcpStepScratch hw;
   __shared__ int state;  // -1: the wait ran out
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5), B = (int)gridDim.x;
+  const int B = (int)gridDim.x;
   lm_copy(&lm, ts);  // (written again only when every block has counted itself in for the last time)
   icp_pose_rows(P.prev, ts->xf.R_inv, ts->xf.t);
+  icp_cameras(P, s);
   icp_pose_rows(P.cur, ts->R, ts->t);
   if (threadIdx.x == 0) state = *(volatile unsigned*)&f.stalled ? -1 : 0;
+  __shared__ IcpPlan plans[kMaxLevels + 1];  // of the levels, and of the photometric rows
+  icp_plans(s, plans, COLOR, (int)blockIdx.x, B, room);
   __syncthreads();
   if (lm.status != 0) {
     if (blockIdx.x == 0 && threadIdx.x == 0) track_end(s, out);
     return;
   }
-  // runs of a warp, dealt over the blocks first
-  const IcpDeal deal{32, lane, 1, warp * B + (int)blockIdx.x, warps * B};
-  const int term = icp_my_term(), at = icp_term_at(term), src = (int)(threadIdx.x & (warps - 1));
+  double* const slots = reinterpret_cast<double*>(icp_stage + (blockDim.x >> 5) * (kIcpStageBytes / 4));
   unsigned turn = 0;  // iterations of this launch
   bool go = state == 0;
   for (int level = s.levels - 1; level >= 0 && go; --level) {
     const bool photo = COLOR && s.photo_w > 0.f && level == 0;
+    const IcpPlan &plan = plans[level], &cplan = plans[kMaxLevels];
     for (int iter = 0; iter < s.iters[level]; ++iter) {
       // (two sets of sums in turn: a block may be one iteration ahead of one that still reads)
       double(*const part)[64] = f.part[turn & 1];
-      const double D = icp_depth_sums(s, level, deal, P, icp_stage, at);
-      if (term < kIcpTerms && src == 0) part[blockIdx.x][term] = D;
-      if (photo) {
-        const double E = icp_color_sums(s, deal, P, icp_stage);
-        if (term < kIcpTerms && src == 0) part[blockIdx.x][32 + term] = E;
-      }
+      icp_depth_sums(s, level, plan, P, icp_stage, slots, [&](int u, int t, double v) { part[u][t] = v; });
+      if (photo) icp_color_sums(s, cplan, P, slots, [&](int u, int t, double v) { part[u][32 + t] = v; });
       __syncthreads();
       ++turn;
       if (threadIdx.x == 0) {
@@ -838,31 +989,8 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
         go = false;
         break;
       }
-      // the blocks' sums: warp w adds the terms (a lane each) of blocks w, w + warps, ..., then
-      // the warps' sums are added pairwise
-      double a = 0.0, c = 0.0;
-      for (int b0 = warp; b0 < B; b0 += 5 * warps) {
-        double u[5], v[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-          const int b = b0 + k * warps;
-          u[k] = b < B ? __ldcg(&part[b][lane]) : 0.0;
-          v[k] = COLOR && photo && b < B ? __ldcg(&part[b][32 + lane]) : 0.0;
-        }
-#pragma unroll
-        for (int k = 0; k < 5; ++k) a += u[k], c += v[k];
-      }
-      double* const w = reinterpret_cast<double*>(icp_stage);
-      w[33 * warp + lane] = a;
-      if (COLOR) w[33 * (warps + warp) + lane] = c;
-      __syncthreads();
-      a = icp_group_sum(w[33 * src + term]);
-      if (COLOR) c = icp_group_sum(w[33 * (warps + src) + term]);
-      // the photometric normal equations and residual enter weighted, the count stays the depth
-      // count
-      if (src == 0) sums[term] = photo && term < kIcpTerms - 1 ? a + (double)s.photo_w * c : a;
       if (threadIdx.x == 0) lm.icp_iters[level] += 1u;
-      __syncthreads();
+      icp_image_sums<COLOR>(s, plan.cut, cplan.cut, photo, icp_stage, sums, [&](int u, int t) { return __ldcg(&part[u][t]); });
       if (threadIdx.x < 64) icp_host_step(&lm, hw, sums, iter, s.icp_min_count[level]);
       __syncthreads();
       icp_pose_rows(P.cur, lm.R, lm.t);
@@ -887,8 +1015,8 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
 
 template __global__ void k_icp_cluster<false>(const SessionDesc*, int, int);
 template __global__ void k_icp_cluster<true>(const SessionDesc*, int, int);
-template __global__ void k_icp_wide<false>(const SessionDesc*, int, IcpWide*, const TrackOut);
-template __global__ void k_icp_wide<true>(const SessionDesc*, int, IcpWide*, const TrackOut);
+template __global__ void k_icp_wide<false>(const SessionDesc*, int, int, IcpWide*, const TrackOut);
+template __global__ void k_icp_wide<true>(const SessionDesc*, int, int, IcpWide*, const TrackOut);
 
 // Start of an integration the host requests directly (step-wise calls): the gate opens, the
 // counters it reports start over (for a voxel hash, the failures before it are noted) and the

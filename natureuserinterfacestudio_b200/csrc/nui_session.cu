@@ -37,7 +37,7 @@ __global__ void k_vertex_map(const SessionDesc*, int, float4*);
 template <bool COLOR>
 __global__ void k_icp_cluster(const SessionDesc*, int, int);
 template <bool COLOR>
-__global__ void k_icp_wide(const SessionDesc*, int, IcpWide*, const TrackOut);
+__global__ void k_icp_wide(const SessionDesc*, int, int, IcpWide*, const TrackOut);
 __global__ void k_track_end(const SessionDesc*, int, const TrackOut);
 __global__ void k_open_gate(const SessionDesc*);
 __global__ void k_color_level(const SessionDesc, int);
@@ -175,6 +175,8 @@ void noalloc_forget(int device);  // defined with nui_mesh_device_noalloc
 constexpr int kStages = 9;
 constexpr int kEvents = 11;
 constexpr size_t kMaxGraphs = 64;  // captured tick graphs kept per context
+constexpr int kIcpRoom = 288;           // leaf sums an ICP block keeps at most (12 units of 23 at 640 x 480), and
+constexpr int kIcpSmemMax = 136 << 10;  // its dynamic shared memory (a cluster of two blocks takes 131 KB)
 }  // namespace
 
 struct nui_session;
@@ -689,6 +691,13 @@ void launch_shift(const BatchPlan& p, const SessionDesc* d, cudaStream_t st) {
   k_shift_dirty<<<dim3(kShiftBlocks, dense_n(p)), 256, 0, st>>>(d);
 }
 
+// The leaf sums that an ICP block with so many units has room for, and its dynamic shared memory:
+// the warps' staging, those slots, and (clusters) `kept` doubles a unit.
+int icp_room(int units) { return std::min(32 * units, kIcpRoom); }
+size_t icp_smem(int units, int threads, int kept) {
+  return (size_t)(threads / 32) * kIcpStageBytes + (size_t)icp_room(units) * kIcpTerms * 8 + (size_t)units * kept * 8;
+}
+
 // The ICP kernel over n sessions, one cluster of cl blocks each (cl > 8 is beyond the
 // portable cluster size and needs the kernel's opt-in).
 //
@@ -700,18 +709,13 @@ void launch_shift(const BatchPlan& p, const SessionDesc* d, cudaStream_t st) {
 // voxel-hash with colour; six ticks): 47.5 ms with 512 / 256, 49.5 with 512 / 512, 48.0 with
 // 256 / 256.
 void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool color, int fam, cudaStream_t st) {
-  static std::once_flag opt_in;
-  std::call_once(opt_in, [] {
-    cudaFuncSetAttribute(k_icp_cluster<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cudaFuncSetAttribute(k_icp_cluster<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  });
-  const int cl = p.tune.icp_cluster_blocks;
+  const int cl = p.tune.icp_cluster_blocks, units = (int)cdiv(kIcpUnits, cl);
   int threads = (n <= 8 ? 1024 : 512) / (color ? 2 : 1);
   while (threads > 256 && (long)p.maxW * p.maxH < 4L * cl * threads) threads /= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cl, n);
   cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = (size_t)(threads / 32) * kIcpStageBytes;
+  cfg.dynamicSmemBytes = icp_smem(units, threads, color ? 64 : 32);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -720,7 +724,7 @@ void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool co
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, color ? k_icp_cluster<true> : k_icp_cluster<false>, d, fam, p.tune.icp_pixels_per_thread);
+  cudaLaunchKernelEx(&cfg, color ? k_icp_cluster<true> : k_icp_cluster<false>, d, fam, icp_room(units));
 }
 
 // Whether the ICP of n sessions leaves the clusters for the whole device (k_icp_wide, a share of
@@ -732,21 +736,22 @@ void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool co
 // session's share nears a cluster's.
 bool icp_wide(int n, int blocks) { return n <= kIcpWideSessions && blocks >= n; }
 
-// One block an SM, the SMs shared by the sessions.
+// One block an SM, the SMs shared by the sessions; of their blocks as many as shorten the longest
+// share of the units.
 void launch_icp_wide(const SessionDesc* d, int n, bool color, int fam, int blocks, IcpWide* work, const TrackOut& out,
                      cudaStream_t st) {
-  const int threads = color ? 512 : 1024;
+  const int threads = color ? 512 : 1024, units = (int)cdiv(kIcpUnits, blocks / n);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min(blocks / n, kIcpWideBlocks), n);
+  cfg.gridDim = dim3(cdiv(kIcpUnits, units), n);
   cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = (size_t)(threads / 32) * kIcpStageBytes;
+  cfg.dynamicSmemBytes = icp_smem(units, threads, 0);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, color ? k_icp_wide<true> : k_icp_wide<false>, d, fam, work, out);
+  cudaLaunchKernelEx(&cfg, color ? k_icp_wide<true> : k_icp_wide<false>, d, fam, icp_room(units), work, out);
 }
 
 // Colour pyramid (if any session tracks with colour), the ICP iterations of every level,
@@ -884,8 +889,15 @@ nui_status ensure_icp_wide(nui_ctx* ctx) {
   int sms = 0, coop = 0, depth = 0, color = 0;
   NUI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   NUI_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-  NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&depth, k_icp_wide<false>, 1024, 32 * kIcpStageBytes));
-  NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&color, k_icp_wide<true>, 512, 16 * kIcpStageBytes));
+  // clusters above 8 blocks, and more than 48 KB of dynamic shared memory
+  for (const void* k : {(const void*)k_icp_cluster<false>, (const void*)k_icp_cluster<true>}) {
+    NUI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    NUI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kIcpSmemMax));
+  }
+  for (const void* k : {(const void*)k_icp_wide<false>, (const void*)k_icp_wide<true>})
+    NUI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kIcpSmemMax));
+  NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&depth, k_icp_wide<false>, 1024, kIcpSmemMax));
+  NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&color, k_icp_wide<true>, 512, kIcpSmemMax));
   ctx->wide_blocks = coop && depth > 0 && color > 0 ? sms : 0;
   return NUI_OK;
 }
@@ -1368,7 +1380,6 @@ NUI_API nui_status nui_ctx_autotune(nui_ctx* c, const nui_session_cfg* cfgs, int
   // the ICP shapes and ray tiles by the whole tick: with dense and hash sessions the hash
   // sessions' tracking and raycast run on the second stream, beside stages 2-5
   tune_one(&nui_tuning::icp_cluster_blocks, {8, 12, 16}, 6);
-  tune_one(&nui_tuning::icp_pixels_per_thread, {2, 4, 8, 16}, 6);
   if (dense) tune_one(&nui_tuning::raycast_tile_width, {4, 8, 16, 32}, 6);
   if (hash) tune_one(&nui_tuning::hash_raycast_tile_width, {4, 8, 16, 32}, 6);
   float tick_ms = 0.f;
