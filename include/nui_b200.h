@@ -236,6 +236,11 @@ NUI_API nui_status nui_mesh_device_noalloc(nui_session* s, float* d_pos, float* 
  * cudaMalloc / cudaMallocHost / cudaHostAlloc it issues).  No counterpart in the
  * reference; for tests that check an entry point allocates nothing. */
 NUI_API nui_status nui_debug_allocation_count(uint64_t* n);
+/* Makes the next wait between the blocks of a whole-device tracking launch of the context run out
+ * after so many polls (as if a block had not arrived).  For tests of what follows: the frame's
+ * status is NUI_ERR_DEVICE, the session stays on its last frame, and the context tracks by thread
+ * block clusters from then on. */
+NUI_API nui_status nui_debug_stall_icp(nui_ctx* ctx, int polls);
 /* Marching-cubes case index of every cube, (res[0]-1)*(res[1]-1)*(res[2]-1) bytes in the
  * same (y, x, z) order; 0 for cubes skipped because a corner has no weight. */
 NUI_API nui_status nui_mesh_cases(nui_session* s, uint8_t* cases, size_t bytes, uint64_t* nverts);

@@ -45,7 +45,7 @@ struct TrackState {
   float lambda, err_old; // Levenberg-Marquardt state of the level
   float error, count;    // NuiKinfuTracker::getError / getCount
   int level_done;        // the level's iteration loop has stopped early
-  int status;            // 0 ok, 3 tracking lost
+  int status;            // 0 ok, 3 tracking lost, kIcpStalled
   int integrate;         // integration gate of this frame
   int iterations_run;
   float lastR[9], lastT[3];  // pose of the last integration (global translation: local +
@@ -82,12 +82,16 @@ struct IcpLm {
 
 // The ICP of one session over many blocks (k_icp_wide): the units' sums (depth in 0..28,
 // photometric in 32..60) of an even and an odd iteration, the blocks' arrivals in the iterations
-// and the blocks that have left (zero between launches), and whether a wait ran out.
+// and the blocks that have left (zero between launches), whether a wait ran out, and the polls a
+// wait makes (0: kIcpPolls).  Once one has run out, the counts cannot be trusted and every launch
+// ends its session's frame as stalled, until the host has cleared the workspace.
 constexpr int kIcpWideSessions = 4;  // sessions a launch, at most
 constexpr int kIcpPolls = 1 << 21;   // polls of the arrivals a block makes (each ~0.4 us)
+constexpr int kIcpStalled = 5;       // TrackState::status of a frame whose wait ran out
 struct IcpWide {
   double part[2][kIcpUnits][64];
   unsigned arrived, left, stalled;
+  int polls;
 };
 
 // Where a tick's results go (14 floats and 2 ints a slot), and whether a shifting volume's

@@ -920,8 +920,8 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
 // another).  Every iteration a block leaves its units' sums in the session's part of `work` and
 // counts itself in; when all have, every block adds all the sums, in the same order, and runs the
 // LM step on its own copy of the state, so nothing has to be sent back.  A wait that runs out (it
-// cannot with all blocks resident) marks the workspace and loses the frame, as every later launch
-// on the workspace does at once.
+// cannot with all blocks resident) marks the workspace and ends the frame as stalled, and so does
+// every later launch on it at once, until the host has cleared it (icp_recover).
 //
 // What bounds it is latency: an iteration is a pass of a few us, a trip through L2 and the LM
 // step.  A cluster is at most 16 SMs, on which a pass of a colour-tracked 640 x 480 level takes
@@ -945,13 +945,16 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
   __shared__ double sums[32];
   __shared__ IcpLm lm;
   __shared__ IcpStepScratch hw;
-  __shared__ int state;  // -1: the wait ran out
+  __shared__ int state, limit;  // -1: the wait ran out; its polls
   const int B = (int)gridDim.x;
   lm_copy(&lm, ts);  // (written again only when every block has counted itself in for the last time)
   icp_pose_rows(P.prev, ts->xf.R_inv, ts->xf.t);
   icp_cameras(P, s);
   icp_pose_rows(P.cur, ts->R, ts->t);
-  if (threadIdx.x == 0) state = *(volatile unsigned*)&f.stalled ? -1 : 0;
+  if (threadIdx.x == 0) {
+    state = *(volatile unsigned*)&f.stalled ? -1 : 0;
+    limit = f.polls > 0 ? f.polls : kIcpPolls;
+  }
   __shared__ IcpPlan plans[kMaxLevels + 1];  // of the levels, and of the photometric rows
   icp_plans(s, plans, COLOR, (int)blockIdx.x, B, room);
   __syncthreads();
@@ -978,7 +981,7 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&f.arrived) : "memory");
         do {
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(&f.arrived) : "memory");
-        } while (e < turn * (unsigned)B && ++polls < kIcpPolls);
+        } while (e < turn * (unsigned)B && ++polls < limit);
         if (e < turn * (unsigned)B) {
           f.stalled = 1u;
           state = -1;
@@ -1001,7 +1004,7 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
     }
   }
   if (blockIdx.x == 0) {
-    if (threadIdx.x == 0 && state != 0) lm.status = 3;
+    if (threadIdx.x == 0 && state != 0) lm.status = kIcpStalled;
     __syncthreads();
     lm_copy(ts, &lm);
     __syncthreads();

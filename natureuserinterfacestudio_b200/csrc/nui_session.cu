@@ -204,6 +204,7 @@ struct BatchPlan {
   // n - denseHead (0, 0: both families over the whole table)
   int hashTail, denseHead;
   int anyFirst;             // some session of the batch has its first frame (frame-0 maps)
+  int wideBlocks;           // the context's blocks of k_icp_wide
   nui_tuning tune;          // the context's launch shapes
   BatchPlan() { std::memset(this, 0, sizeof(*this)); }
   bool operator<(const BatchPlan& o) const { return std::memcmp(this, &o, sizeof(BatchPlan)) < 0; }
@@ -234,7 +235,7 @@ struct nui_ctx {
   int par = 0;              // the half the next tick uses
   cudaEvent_t ev_tick[2] = {nullptr, nullptr};
   IcpWide* d_icp_wide = nullptr;  // ICP over the whole device: 2 x kIcpWideSessions (a set a stream)
-  int wide_blocks = 0;            // blocks of k_icp_wide the device holds at once, one an SM (0: not to be launched)
+  std::atomic<int> wide_blocks{0};  // blocks of k_icp_wide the device holds at once, one an SM (0: not to be launched)
   unsigned long long* d_count = nullptr;  // counter of the point-cloud fetch
   struct Graph {
     cudaGraphExec_t exec;
@@ -804,16 +805,16 @@ void enqueue_tick(nui_ctx* ctx, const BatchPlan& p, const SessionDesc* d, float*
     if (ev) cudaEventRecord(ctx->ev[9], hs);
     if (ranged) {
       launch_track(p, d + p.denseHead, p.n - p.denseHead, hs, d_pose, d_status, (p.colorIcp & 2) != 0,
-                   ctx->d_icp_wide + kIcpWideSessions, ctx->wide_blocks / 2);
-      launch_track(p, d, p.denseHead, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_icp_wide, ctx->wide_blocks / 2);
+                   ctx->d_icp_wide + kIcpWideSessions, p.wideBlocks / 2);
+      launch_track(p, d, p.denseHead, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_icp_wide, p.wideBlocks / 2);
     } else {
       launch_track(p, d, p.n, hs, d_pose, d_status, (p.colorIcp & 2) != 0, ctx->d_icp_wide + kIcpWideSessions,
-                   ctx->wide_blocks / 2, kFamHash);
-      launch_track(p, d, p.n, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_icp_wide, ctx->wide_blocks / 2,
+                   p.wideBlocks / 2, kFamHash);
+      launch_track(p, d, p.n, st, d_pose, d_status, (p.colorIcp & 1) != 0, ctx->d_icp_wide, p.wideBlocks / 2,
                    kFamDense);
     }
   } else {
-    launch_track(p, d, p.n, st, d_pose, d_status, p.colorIcp != 0, ctx->d_icp_wide, ctx->wide_blocks);
+    launch_track(p, d, p.n, st, d_pose, d_status, p.colorIcp != 0, ctx->d_icp_wide, p.wideBlocks);
   }
   mark(3);
   if (ev) ctx->side_timed = fork;
@@ -902,6 +903,16 @@ nui_status ensure_icp_wide(nui_ctx* ctx) {
   return NUI_OK;
 }
 
+// After a frame whose wait in k_icp_wide ran out: the workspace starts over behind what is queued
+// (a tick in flight ends as stalled too), and the context tracks by clusters from now on, which
+// wait for nothing but their own blocks.
+const char* const kStalledText = "tracking: a wait between blocks ran out; the context tracks by clusters from now on";
+nui_status icp_recover(nui_ctx* ctx) {
+  ctx->wide_blocks = 0;
+  NUI_CUDA(cudaMemsetAsync(ctx->d_icp_wide, 0, sizeof(IcpWide) * 2 * kIcpWideSessions, ctx->stream));
+  return NUI_OK;
+}
+
 nui_status finish_timing(nui_ctx* ctx) {
   if (!ctx->timing) return NUI_OK;
   NUI_CUDA(cudaEventSynchronize(ctx->ev[6]));
@@ -962,6 +973,7 @@ nui_status tick_launch(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
   if (floor) plan_merge(p, *floor);
   p.tune = ctx->tune;
   if ((st = ensure_icp_wide(ctx)) != NUI_OK) return st;
+  p.wideBlocks = ctx->wide_blocks;
   NUI_CUDA(cudaMemcpyAsync(ctx->d_descs, hd, sizeof(SessionDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
   if (use_graph && !ctx->timing) {
     auto it = ctx->graphs.find(p);
@@ -1009,8 +1021,10 @@ nui_status tick_launch(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
 }
 
 // Waits for the tick launched with staging half par and takes its per-session results.
+// stalled (nullable): a session's tracking ran out of a wait; its status is NUI_ERR_DEVICE then, and
+// the results of all are there.
 nui_status tick_finish(nui_ctx* ctx, nui_session* const* ss, int n, const uint16_t* const* raws, nui_status* per,
-                       float* poses, int par) {
+                       float* poses, int par, bool* stalled = nullptr) {
   NUI_CUDA(cudaEventSynchronize(ctx->ev_tick[par]));
   nui_status st = finish_timing(ctx);
   if (st != NUI_OK) return st;
@@ -1022,7 +1036,10 @@ nui_status tick_finish(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
       fail(r, "voxel hash: pool or excess list exhausted (or a corrupted chain); blocks dropped");
     else if (r == NUI_ERR_TRACKING_LOST)
       fail(r, "ICP system is singular");
+    else if (r == NUI_ERR_DEVICE)
+      fail(r, kStalledText);
   };
+  bool stall = false;
   for (int i = 0; i < n; ++i) {
     nui_session* s = ss[i];
     if (!s || !raws[i]) {
@@ -1039,10 +1056,11 @@ nui_status tick_finish(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
       if (poses) std::memcpy(poses + 12 * i, h_pose + 14 * i, 12 * sizeof(float));
       continue;
     }
-    nui_status r = status == 0 ? NUI_OK : NUI_ERR_TRACKING_LOST;
+    nui_status r = status == 0 ? NUI_OK : status == kIcpStalled ? NUI_ERR_DEVICE : NUI_ERR_TRACKING_LOST;
     if (per) per[i] = r;
     if (r != NUI_OK) {
-      agg = NUI_ERR_TRACKING_LOST;
+      stall |= r == NUI_ERR_DEVICE;
+      agg = stall ? NUI_ERR_DEVICE : r;
       note(agg);
       // the device state stays on the previous frame, which the frame count follows; the
       // flag is cleared in stream order (every tick also clears it when it starts), so
@@ -1052,6 +1070,11 @@ nui_status tick_finish(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
     }
     if (poses) std::memcpy(poses + 12 * i, h_pose + 14 * i, 12 * sizeof(float));
   }
+  if (stall) {
+    st = icp_recover(ctx);
+    if (st != NUI_OK) return st;
+  }
+  if (stalled) *stalled = stall;
   return agg;
 }
 
@@ -1249,6 +1272,20 @@ NUI_API nui_status nui_ctx_synchronize(nui_ctx* c) {
 NUI_API nui_status nui_ctx_enable_timing(nui_ctx* c, int enable) {
   if (!c) return fail(NUI_ERR_INVALID_ARG, "null context");
   c->timing = enable != 0;
+  return NUI_OK;
+}
+
+NUI_API nui_status nui_debug_stall_icp(nui_ctx* c, int polls) {
+  if (!c || polls <= 0) return fail(NUI_ERR_INVALID_ARG, "bad argument");
+  const nui_status st = ensure_icp_wide(c);
+  if (st != NUI_OK) return st;
+  // one arrival short: the count wraps to zero with the first block
+  const unsigned missing = ~0u;
+  for (int i = 0; i < 2 * kIcpWideSessions; ++i) {
+    NUI_CUDA(cudaMemcpyAsync(&c->d_icp_wide[i].arrived, &missing, sizeof(missing), cudaMemcpyHostToDevice, c->stream));
+    NUI_CUDA(cudaMemcpyAsync(&c->d_icp_wide[i].polls, &polls, sizeof(polls), cudaMemcpyHostToDevice, c->stream));
+  }
+  NUI_CUDA(cudaStreamSynchronize(c->stream));
   return NUI_OK;
 }
 
@@ -1976,6 +2013,10 @@ NUI_API nui_status nui_track(nui_session* s, float* err, int* count) {
   if (t.status != 0) {
     int zero = 0;
     cudaMemcpy(&s->ts->status, &zero, sizeof(int), cudaMemcpyHostToDevice);
+    if (t.status == kIcpStalled) {
+      st = icp_recover(s->ctx);
+      return st != NUI_OK ? st : fail(NUI_ERR_DEVICE, kStalledText);
+    }
     return fail(NUI_ERR_TRACKING_LOST, "ICP system is singular");
   }
   return NUI_OK;
@@ -2597,8 +2638,9 @@ nui_status server_collect(nui_server* v) {
   const int n = (int)v->bsess.size();
   std::vector<nui_status> per(n);
   std::vector<float> poses(12 * (size_t)n);
-  nui_status st = tick_finish(v->ctx, v->bsess.data(), n, v->braw.data(), per.data(), poses.data(), v->bpar);
-  if (st != NUI_OK && st != NUI_ERR_TRACKING_LOST && st != NUI_ERR_HASH_FULL) return st;
+  bool stalled = false;
+  nui_status st = tick_finish(v->ctx, v->bsess.data(), n, v->braw.data(), per.data(), poses.data(), v->bpar, &stalled);
+  if (st != NUI_OK && st != NUI_ERR_TRACKING_LOST && st != NUI_ERR_HASH_FULL && !stalled) return st;
   for (int i = 0; i < n; ++i) {
     if (!v->bsess[i] || !v->braw[i]) continue;
     nui_server_result r;
