@@ -236,6 +236,8 @@ struct nui_ctx {
   cudaEvent_t ev_tick[2] = {nullptr, nullptr};
   IcpWide* d_icp_wide = nullptr;  // ICP over the whole device: 2 x kIcpWideSessions (a set a stream)
   std::atomic<int> wide_blocks{0};  // blocks of k_icp_wide the device holds at once, one an SM (0: not to be launched)
+  std::mutex icp_mu;                // the first tracking sets the three up, whichever thread it is on
+  std::atomic<bool> icp_ready{false};
   unsigned long long* d_count = nullptr;  // counter of the point-cloud fetch
   struct Graph {
     cudaGraphExec_t exec;
@@ -879,27 +881,38 @@ nui_status ensure_cap(nui_ctx* ctx, int n) {
   return NUI_OK;
 }
 
-// The workspace of k_icp_wide, at the context's first tracking, and the blocks that are
-// sure to be resident together: one an SM, if the device launches cooperatively and an SM holds
-// a block of either variant.
-nui_status ensure_icp_wide(nui_ctx* ctx) {
-  if (ctx->d_icp_wide) return NUI_OK;
-  const size_t bytes = sizeof(IcpWide) * 2 * kIcpWideSessions;
-  NUI_CUDA(counted_pool_alloc((void**)&ctx->d_icp_wide, bytes, ctx->pool, ctx->stream));
-  NUI_CUDA(cudaMemsetAsync(ctx->d_icp_wide, 0, bytes, ctx->stream));
-  int sms = 0, coop = 0, depth = 0, color = 0;
-  NUI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-  NUI_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
-  // clusters above 8 blocks, and more than 48 KB of dynamic shared memory
+// What the tracking launches need, at the context's first tracking: the kernels' opt-ins (clusters
+// above 8 blocks, more than 48 KB of dynamic shared memory), the blocks of k_icp_wide that are sure
+// to be resident together -- one an SM, if the device launches cooperatively and an SM holds a
+// block of either variant -- and its workspace.  Without room for that the context tracks by
+// clusters.  Sessions of a context may be called from several threads.
+nui_status ensure_icp(nui_ctx* ctx) {
+  if (ctx->icp_ready.load(std::memory_order_acquire)) return NUI_OK;
+  std::lock_guard<std::mutex> lock(ctx->icp_mu);
+  if (ctx->icp_ready.load(std::memory_order_relaxed)) return NUI_OK;
   for (const void* k : {(const void*)k_icp_cluster<false>, (const void*)k_icp_cluster<true>}) {
     NUI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     NUI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kIcpSmemMax));
   }
   for (const void* k : {(const void*)k_icp_wide<false>, (const void*)k_icp_wide<true>})
     NUI_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kIcpSmemMax));
+  int sms = 0, coop = 0, depth = 0, color = 0;
+  NUI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+  NUI_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
   NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&depth, k_icp_wide<false>, 1024, kIcpSmemMax));
   NUI_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&color, k_icp_wide<true>, 512, kIcpSmemMax));
-  ctx->wide_blocks = coop && depth > 0 && color > 0 ? sms : 0;
+  if (coop && depth > 0 && color > 0) {
+    const size_t bytes = sizeof(IcpWide) * 2 * kIcpWideSessions;
+    IcpWide* work = nullptr;
+    if (counted_pool_alloc((void**)&work, bytes, ctx->pool, ctx->stream) == cudaSuccess) {
+      ctx->d_icp_wide = work;
+      NUI_CUDA(cudaMemsetAsync(work, 0, bytes, ctx->stream));
+      ctx->wide_blocks = sms;
+    } else {
+      cudaGetLastError();
+    }
+  }
+  ctx->icp_ready.store(true, std::memory_order_release);
   return NUI_OK;
 }
 
@@ -972,7 +985,7 @@ nui_status tick_launch(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
   }
   if (floor) plan_merge(p, *floor);
   p.tune = ctx->tune;
-  if ((st = ensure_icp_wide(ctx)) != NUI_OK) return st;
+  if ((st = ensure_icp(ctx)) != NUI_OK) return st;
   p.wideBlocks = ctx->wide_blocks;
   NUI_CUDA(cudaMemcpyAsync(ctx->d_descs, hd, sizeof(SessionDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
   if (use_graph && !ctx->timing) {
@@ -1277,8 +1290,9 @@ NUI_API nui_status nui_ctx_enable_timing(nui_ctx* c, int enable) {
 
 NUI_API nui_status nui_debug_stall_icp(nui_ctx* c, int polls) {
   if (!c || polls <= 0) return fail(NUI_ERR_INVALID_ARG, "bad argument");
-  const nui_status st = ensure_icp_wide(c);
+  const nui_status st = ensure_icp(c);
   if (st != NUI_OK) return st;
+  if (!c->d_icp_wide) return fail(NUI_ERR_UNSUPPORTED, "the context tracks by clusters");
   // one arrival short: the count wraps to zero with the first block
   const unsigned missing = ~0u;
   for (int i = 0; i < 2 * kIcpWideSessions; ++i) {
@@ -1946,9 +1960,10 @@ nui_status run_stage(nui_session* s, int what, bool sync = true) {
     for (int l = 1; l < p.maxLevels; ++l)
       k_pyramid<<<dim3(cdiv((long)(p.maxW >> l) * (p.maxH >> l), 256), 1), 256, 0, st>>>(dd, l);
   } else if (what == 1) {
-    const nui_status fs = ensure_icp_wide(ctx);
+    const nui_status fs = ensure_icp(ctx);
     if (fs != NUI_OK) return fs;
-    launch_track(p, dd, p.n, st, ctx->d_pose, ctx->d_status, p.colorIcp != 0, ctx->d_icp_wide, ctx->wide_blocks, kFamAll, false);
+    // (the result is read from the session's state: the context's arrays are its ticks')
+    launch_track(p, dd, p.n, st, nullptr, nullptr, p.colorIcp != 0, ctx->d_icp_wide, ctx->wide_blocks, kFamAll, false);
   } else if (what == 2) {
     k_open_gate<<<1, 32, 0, st>>>(dd);
     launch_shift(p, dd, st);
@@ -1999,11 +2014,9 @@ NUI_API nui_status nui_feedback_update(nui_session* s) {
 
 NUI_API nui_status nui_track(nui_session* s, float* err, int* count) {
   if (!s) return fail(NUI_ERR_INVALID_ARG, "null session");
-  nui_status st = ensure_cap(s->ctx, 1);
-  if (st != NUI_OK) return st;
   // the track stage must run with the integration threshold of the session, and must
   // not integrate: the tracking only decides the gate
-  st = run_stage(s, 1, false);
+  nui_status st = run_stage(s, 1, false);
   if (st != NUI_OK) return st;
   TrackState t;
   NUI_CUDA(cudaMemcpyAsync(&t, s->ts, sizeof(t), cudaMemcpyDeviceToHost, s->ctx->stream));

@@ -2,6 +2,7 @@
 and without the photometric rows, block sizes by image size -- the same poses by
 every route, at the edges of the rules -- and the shared-reciprocal quotients of the
 photometric rows against the division they replace."""
+import ctypes as C
 import random
 import threading
 from fractions import Fraction
@@ -91,6 +92,52 @@ def test_contexts_on_threads_track_at_once():
         for lap in o:
             for (ok, p), (ok0, p0) in zip(lap, alone[0]):
                 assert ok == ok0 and np.array_equal(p, p0)
+
+
+@pytest.mark.gpu
+def test_first_trackings_of_a_context_on_threads(gpu_ctx):
+    """Sessions of one context may be called from several threads, its first trackings too: the
+    workspace is allocated once, and every thread tracks to the poses of a context that one uses."""
+    W, H, N = 160, 120, 6
+    cfg, seq = cfg_for(W=W, H=H, res=(64, 64, 64), trunc=0.1, iters=(4, 3, 3)), frames(2, W=W, H=H, seed=5)
+
+    def count():
+        n = C.c_uint64()
+        L.check(L.lib().nui_debug_allocation_count(C.byref(n)))
+        return n.value
+
+    def track(s, bar, out):
+        s.upload(seq[0][0])
+        s.feedback_update()
+        s.upload(seq[1][0])
+        if bar:
+            bar.wait()
+        s.track()
+        out.append(s.get_pose())
+
+    want, allocations = [], []
+    for threads in (1, N, N, N, N):
+        ctx = L.Context(0)
+        ss = [L.Session(ctx, cfg) for _ in range(N)]
+        L.check(L.lib().nui_ctx_synchronize(ctx.h))
+        n0, out, bar = count(), [], threading.Barrier(N) if threads > 1 else None
+        if threads == 1:
+            for s in ss:
+                track(s, None, out)
+        else:
+            ts = [threading.Thread(target=track, args=(s, bar, out)) for s in ss]
+            for t in ts:
+                t.start()
+            for t in ts:
+                t.join()
+        assert len(out) == N
+        want = want or out[0]
+        assert all(np.array_equal(a, b) for p in out for a, b in zip(p, want))
+        allocations.append(count() - n0)
+        for s in ss:
+            s.close()
+        ctx.close()
+    assert len(set(allocations)) == 1, allocations
 
 
 def _f32(x):
