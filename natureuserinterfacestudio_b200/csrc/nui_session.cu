@@ -205,6 +205,7 @@ struct BatchPlan {
   int hashTail, denseHead;
   int anyFirst;             // some session of the batch has its first frame (frame-0 maps)
   int wideBlocks;           // the context's blocks of k_icp_wide
+  int icpFit[2];            // clusters of the widest blocks that the device holds at once: depth, colour
   nui_tuning tune;          // the context's launch shapes
   BatchPlan() { std::memset(this, 0, sizeof(*this)); }
   bool operator<(const BatchPlan& o) const { return std::memcmp(this, &o, sizeof(BatchPlan)) < 0; }
@@ -236,8 +237,13 @@ struct nui_ctx {
   cudaEvent_t ev_tick[2] = {nullptr, nullptr};
   IcpWide* d_icp_wide = nullptr;  // ICP over the whole device: 2 x kIcpWideSessions (a set a stream)
   std::atomic<int> wide_blocks{0};  // blocks of k_icp_wide the device holds at once, one an SM (0: not to be launched)
-  std::mutex icp_mu;                // the first tracking sets the three up, whichever thread it is on
+  std::mutex icp_mu;                // the first tracking sets these up, whichever thread it is on
   std::atomic<bool> icp_ready{false};
+  std::atomic<int> icp_fit[2][17];  // per colour and cluster size, -1: not asked yet
+  nui_ctx() {
+    for (auto& c : icp_fit)
+      for (auto& n : c) n = -1;
+  }
   unsigned long long* d_count = nullptr;  // counter of the point-cloud fetch
   struct Graph {
     cudaGraphExec_t exec;
@@ -704,16 +710,16 @@ size_t icp_smem(int units, int threads, int kept) {
 // The ICP kernel over n sessions, one cluster of cl blocks each (cl > 8 is beyond the
 // portable cluster size and needs the kernel's opt-in).
 //
-// Block size: the clusters of up to eight sessions may fill their SMs (a block an SM, a cluster
-// a GPC); those of more share them.  Small images keep four pixels or more of the finest level
-// a thread, where a wider block only has more warps to reduce.  The colour variant holds twice
-// the registers, so half the threads.  Measured, one 640 x 480 session (the whole step-wise
-// track): 292 us with 1024 threads, 313 with 512, 381 with 256; 64 sessions (39 dense, 25
-// voxel-hash with colour; six ticks): 47.5 ms with 512 / 256, 49.5 with 512 / 512, 48.0 with
-// 256 / 256.
+// Block size: clusters fill their SMs (a block an SM) while the device holds all of them at once,
+// else they share them.  A 1024-thread block's registers are an SM's, so 12 of them want 12 whole
+// SMs of a GPC.  Small images keep four pixels or more of the finest level a thread, where a wider
+// block only has more warps to reduce.  The colour variant holds twice the registers, so half the
+// threads.  The device holds seven such clusters of 12; the tracking stage of n sessions at 7, 8 and
+// 9: 640 x 480 depth 153, 220, 224 us, with colour 680, 1193, 1233, 320 x 240 depth 118, 141, 142,
+// with colour 264, 429, 428 (eight with the widest blocks, in two waves: 286, 1288, 218 and 501).
 void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool color, int fam, cudaStream_t st) {
   const int cl = p.tune.icp_cluster_blocks, units = (int)cdiv(kIcpUnits, cl);
-  int threads = (n <= 8 ? 1024 : 512) / (color ? 2 : 1);
+  int threads = (n <= p.icpFit[color] ? 1024 : 512) / (color ? 2 : 1);
   while (threads > 256 && (long)p.maxW * p.maxH < 4L * cl * threads) threads /= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cl, n);
@@ -916,6 +922,35 @@ nui_status ensure_icp(nui_ctx* ctx) {
   return NUI_OK;
 }
 
+// How many clusters of the plan's size, of the widest blocks, the device holds at once.
+void icp_fit(nui_ctx* ctx, BatchPlan& p) {
+  const int cl = p.tune.icp_cluster_blocks, units = (int)cdiv(kIcpUnits, cl);
+  for (int color = 0; color < 2; ++color) {
+    std::atomic<int>& known = ctx->icp_fit[color][cl];
+    if (known < 0) {
+      const int threads = color ? 512 : 1024;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(cl);
+      cfg.blockDim = dim3(threads);
+      cfg.dynamicSmemBytes = icp_smem(units, threads, color ? 64 : 32);
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = cl;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, color ? k_icp_cluster<true> : k_icp_cluster<false>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      known = n;
+    }
+    p.icpFit[color] = known;
+  }
+}
+
 // After a frame whose wait in k_icp_wide ran out: the workspace starts over behind what is queued
 // (a tick in flight ends as stalled too), and the context tracks by clusters from now on, which
 // wait for nothing but their own blocks.
@@ -987,6 +1022,7 @@ nui_status tick_launch(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
   p.tune = ctx->tune;
   if ((st = ensure_icp(ctx)) != NUI_OK) return st;
   p.wideBlocks = ctx->wide_blocks;
+  icp_fit(ctx, p);
   NUI_CUDA(cudaMemcpyAsync(ctx->d_descs, hd, sizeof(SessionDesc) * n, cudaMemcpyHostToDevice, ctx->stream));
   if (use_graph && !ctx->timing) {
     auto it = ctx->graphs.find(p);
@@ -1962,6 +1998,7 @@ nui_status run_stage(nui_session* s, int what, bool sync = true) {
   } else if (what == 1) {
     const nui_status fs = ensure_icp(ctx);
     if (fs != NUI_OK) return fs;
+    icp_fit(ctx, p);
     // (the result is read from the session's state: the context's arrays are its ticks')
     launch_track(p, dd, p.n, st, nullptr, nullptr, p.colorIcp != 0, ctx->d_icp_wide, ctx->wide_blocks, kFamAll, false);
   } else if (what == 2) {
