@@ -737,19 +737,35 @@ void launch_icp_cluster(const BatchPlan& p, const SessionDesc* d, int n, bool co
 }
 
 // Whether the ICP of n sessions leaves the clusters for the whole device (k_icp_wide, a share of
-// `blocks` blocks a session): for few sessions, of any size, as even small levels gain from
-// one warp a scheduler more than a wait through L2 costs over a cluster's barrier.  Measured, one
-// session, clusters (level 0 of large images over the device by a launch an iteration) and
-// k_icp_wide: track at 640 x 480 253 -> 194 us, 320 x 240 218 -> 181, 188 x 132 172 -> 162, with
-// colour 352 x 208 333 -> 261; locate on a voxel hash with colour 875 -> 750.  Beyond four, a
-// session's share nears a cluster's.
+// its blocks a session): for up to four, of any size.  Measured, the tracking stage of 1, 2, 3 and 4
+// sessions by k_icp_wide on all SMs, and of as many and of five by clusters: 640 x 480 82, 88, 90,
+// 97 us and 144 to 149, with colour 167, 215, 258, 290 and 589 to 631, 320 x 240 91, 94, 92, 94 and
+// 115 to 117, with colour 130, 146, 157, 166 and 256 to 262.  The workspace is four sessions'; more
+// have not been measured by this route.
 bool icp_wide(int n, int blocks) { return n <= kIcpWideSessions && blocks >= n; }
 
-// One block an SM, the SMs shared by the sessions; of their blocks as many as shorten the longest
-// share of the units.
-void launch_icp_wide(const SessionDesc* d, int n, bool color, int fam, int blocks, IcpWide* work, const TrackOut& out,
-                     cudaStream_t st) {
-  const int threads = color ? 512 : 1024, units = (int)cdiv(kIcpUnits, blocks / n);
+// The blocks of a launch of k_icp_wide, one an SM.  A block fills its SM and several contexts may
+// track at once, so a launch takes no more SMs than the images need: all of them from half a million
+// pixels on (photometric rows count fourfold), 108 (with colour 72) from 128 K, else 48.  Measured,
+// the stage of one context and frames/s of eight on threads, with all SMs, 72 and 48 in a launch
+// (and before there was one, by 6-SM clusters of narrow blocks):
+//   640 x 480, one session  82, 88, 89 us    9.1, 12.9, 15.3 k (194 us, 11.8 k)
+//     three                 90, 104, 127     15.8, 19.4, 20.6  (196, 17.2); with 108: 95, 17.1
+//   320 x 240, one          92, 92, 93       10.0, 17.0, 22.0  (129, 18.9)
+//     three                 100, 104, 113    24.8, 37.5, 44.1  (144, 40.9)
+//   160 x 120, four         125, 126, 125    32.6, 54.3, 69.2  (132, 67.4)
+//   colour 640 x 480, one   167, 207, 247    5.5, 7.9, 9.2     (932, 5.5)
+//     three                 257, 366, 491    9.3, 11.3, 11.3   (945, 9.5)
+//   colour 320 x 240, one   132, 140, 152    7.6, 12.6, 15.7   (331, 11.8)
+//     four                  167, 210, 249    21.4, 28.7, 32.9  (329, 29.6)
+int icp_wide_total(long pixels, bool color, int blocks) {
+  const long work = pixels * (color ? 4 : 1);
+  return work >= 1L << 19 ? blocks : std::min(blocks, work >= 1L << 17 ? (color ? 72 : 108) : 48);
+}
+void launch_icp_wide(const SessionDesc* d, int n, long pixels, bool color, int fam, int blocks, IcpWide* work,
+                     const TrackOut& out, cudaStream_t st) {
+  // of the blocks of a session's share as many as shorten the longest one's units
+  const int threads = color ? 512 : 1024, units = (int)cdiv(kIcpUnits, icp_wide_total(pixels, color, blocks) / n);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cdiv(kIcpUnits, units), n);
   cfg.blockDim = dim3(threads);
@@ -774,7 +790,7 @@ void launch_track(const BatchPlan& p, const SessionDesc* d, int n, cudaStream_t 
   // every level and iteration of every session in one launch, and the tracking's end
   const TrackOut out{d_pose, d_status, tick ? 1 : 0};
   if (icp_wide(n, wide_blocks)) {
-    launch_icp_wide(d, n, color, fam, wide_blocks, work, out, st);
+    launch_icp_wide(d, n, (long)p.maxW * p.maxH, color, fam, wide_blocks, work, out, st);
   } else {
     launch_icp_cluster(p, d, n, color, fam, st);
     k_track_end<<<n, 32, 0, st>>>(d, fam, out);
