@@ -484,6 +484,20 @@ void fill_desc(const nui_session* s, SessionDesc& d, int kind, const uint16_t* r
   }
 }
 
+// Restores the caller's current device when the entry point returns.
+struct DeviceGuard {
+  int prev = -1;
+  DeviceGuard() {
+    if (cudaGetDevice(&prev) != cudaSuccess) {
+      prev = -1;
+      cudaGetLastError();
+    }
+  }
+  ~DeviceGuard() {
+    if (prev >= 0) cudaSetDevice(prev);
+  }
+};
+
 // Puts the descriptor into the session's one-entry table in stream order; a table that holds it
 // already is left alone (a pageable copy costs a step-wise call ~6 us).
 cudaError_t upload_desc1(nui_session* s, const SessionDesc& d) {
@@ -1728,6 +1742,8 @@ NUI_API nui_status nui_set_pose(nui_session* s, const float* pose12) {
     m.R_inv[i] = (float)(inv[i] / det);
   }
   for (int i = 0; i < 3; ++i) m.t[i] = pose12[9 + i];
+  DeviceGuard guard;  // (a launch, unlike a copy, needs the stream's device to be current)
+  NUI_CUDA(cudaSetDevice(s->ctx->device));
   k_set_pose<<<1, 32, 0, s->ctx->stream>>>(s->ts, m);
   NUI_CUDA(cudaGetLastError());
   return NUI_OK;
@@ -1855,6 +1871,8 @@ NUI_API nui_status nui_session_restore(nui_session* s, const void* host, size_t 
     BatchPlan p1;
     p1.n = 1;
     plan_add(p1, s);
+    DeviceGuard guard;
+    NUI_CUDA(cudaSetDevice(s->ctx->device));
     launch_distances(p1, s->d_desc1, s->ctx->stream, 1);
     NUI_CUDA(cudaGetLastError());
     NUI_CUDA(cudaStreamSynchronize(s->ctx->stream));
@@ -2539,20 +2557,6 @@ static __device__ __align__(256) unsigned char g_mesh_scratch[kNoAllocCols * 4 +
 constexpr int kMaxDevices = 64;
 unsigned char* g_mesh_scratch_addr[kMaxDevices] = {};
 std::mutex g_mesh_scratch_mu;
-
-// Restores the caller's current device when the entry point returns.
-struct DeviceGuard {
-  int prev = -1;
-  DeviceGuard() {
-    if (cudaGetDevice(&prev) != cudaSuccess) {
-      prev = -1;
-      cudaGetLastError();
-    }
-  }
-  ~DeviceGuard() {
-    if (prev >= 0) cudaSetDevice(prev);
-  }
-};
 
 // Device address of the scratch array on `device` (current); looked up on the first call
 // after the library loads or after a context is created on the device (nui_ctx_create

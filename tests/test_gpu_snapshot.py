@@ -44,3 +44,24 @@ def test_restored_session_continues_identically(gpu_ctx, name, cfg, color):
         other.restore(snap)
     for s in (a, b, other):
         s.close()
+
+
+def test_pose_and_restore_while_another_device_is_current(gpu_ctx):
+    """nui_set_pose and nui_session_restore work on the session's device whatever the calling
+    thread's current one is, and leave that as it was."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices")
+    cfg = cfg_for(W=320, H=240, res=(64, 64, 64), trunc=0.1)
+    d, _, R, t = frames(1, W=320, H=240, seed=5)[0]
+    s = L.Session(gpu_ctx, cfg)
+    assert s.process(d)[0]
+    snap = s.snapshot()
+    with torch.cuda.device(1):
+        s.set_pose(R, t)
+        r2, t2 = s.get_pose()
+        s.restore(snap)
+        assert torch.cuda.current_device() == 1
+    assert np.array_equal(r2, np.asarray(R, np.float32)) and np.array_equal(t2, np.asarray(t, np.float32))
+    assert np.array_equal(s.snapshot(), snap)
+    s.close()
