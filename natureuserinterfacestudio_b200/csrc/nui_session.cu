@@ -500,7 +500,7 @@ struct DeviceGuard {
 
 // Puts the descriptor into the session's one-entry table in stream order; a table that holds it
 // already is left alone (a pageable copy costs a step-wise call ~6 us).
-cudaError_t upload_desc1(nui_session* s, const SessionDesc& d) {
+[[nodiscard]] cudaError_t upload_desc1(nui_session* s, const SessionDesc& d) {
   if (s->desc1_set && std::memcmp(&s->h_desc1, &d, sizeof(d)) == 0) return cudaSuccess;
   s->desc1_set = false;
   std::memcpy(&s->h_desc1, &d, sizeof(d));
@@ -2142,11 +2142,11 @@ NUI_API nui_status nui_debug_download(nui_session* s, int what, int level, void*
     case 2: {  // vertex map of a level, rebuilt from its depth
       need = Nl * 16;
       if (bytes < need) return fail(NUI_ERR_INVALID_ARG, "buffer too small");
-      void* tmp = nullptr;
-      NUI_CUDA(counted_malloc(&tmp, need));
       SessionDesc d;
       fill_desc(s, d, kInactive, nullptr, nullptr);
-      upload_desc1(s, d);
+      NUI_CUDA(upload_desc1(s, d));
+      void* tmp = nullptr;
+      NUI_CUDA(counted_malloc(&tmp, need));
       k_vertex_map<<<dim3(cdiv((long)Nl, 256), 1), 256, 0, s->ctx->stream>>>(s->d_desc1, level, (float4*)tmp);
       cudaError_t e = cudaMemcpyAsync(host, tmp, need, cudaMemcpyDeviceToHost, s->ctx->stream);
       cudaStreamSynchronize(s->ctx->stream);
@@ -2190,11 +2190,11 @@ NUI_API nui_status nui_debug_download(nui_session* s, int what, int level, void*
       if (!s->hash) return fail(NUI_ERR_INVALID_ARG, "not a hash session");
       need = (size_t)c.hash_pool_blocks * 512 * 6;
       if (bytes < need) return fail(NUI_ERR_INVALID_ARG, "buffer too small");
-      void* tmp = nullptr;
-      NUI_CUDA(counted_malloc(&tmp, need));
       SessionDesc d;
       fill_desc(s, d, kInactive, nullptr, nullptr);
-      upload_desc1(s, d);
+      NUI_CUDA(upload_desc1(s, d));
+      void* tmp = nullptr;
+      NUI_CUDA(counted_malloc(&tmp, need));
       k_hash_export_voxels<<<1184, 256, 0, s->ctx->stream>>>(s->d_desc1, (uint8_t*)tmp);
       cudaError_t e = cudaMemcpyAsync(host, tmp, need, cudaMemcpyDeviceToHost, s->ctx->stream);
       cudaStreamSynchronize(s->ctx->stream);
@@ -2207,11 +2207,11 @@ NUI_API nui_status nui_debug_download(nui_session* s, int what, int level, void*
       need = nv * 4;
       if (bytes < need) return fail(NUI_ERR_INVALID_ARG, "buffer too small");
       if (what == 9 && !s->cvol) return fail(NUI_ERR_INVALID_ARG, "no colour volume");
-      void* tmp = nullptr;
-      NUI_CUDA(counted_malloc(&tmp, need));
       SessionDesc d;
       fill_desc(s, d, kInactive, nullptr, nullptr);
-      upload_desc1(s, d);
+      NUI_CUDA(upload_desc1(s, d));
+      void* tmp = nullptr;
+      NUI_CUDA(counted_malloc(&tmp, need));
       short2* vo = what == 5 ? (short2*)tmp : nullptr;
       uchar4* co = what == 9 ? (uchar4*)tmp : nullptr;
       switch (c.tsdf_format) {
@@ -2251,11 +2251,11 @@ NUI_API nui_status nui_debug_upload_volume(nui_session* s, const int16_t* ref) {
   if (s && s->hash) return fail(NUI_ERR_UNSUPPORTED, "dense volumes only");
   if (!s || !ref) return fail(NUI_ERR_INVALID_ARG, "null argument");
   const size_t nv = (size_t)s->cfg.res[0] * s->cfg.res[1] * s->cfg.res[2];
-  void* tmp = nullptr;
-  NUI_CUDA(counted_malloc(&tmp, nv * 4));
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
-  upload_desc1(s, d);
+  NUI_CUDA(upload_desc1(s, d));
+  void* tmp = nullptr;
+  NUI_CUDA(counted_malloc(&tmp, nv * 4));
   cudaMemcpyAsync(tmp, ref, nv * 4, cudaMemcpyHostToDevice, s->ctx->stream);
   k_occ_clear<<<256, 256, 0, s->ctx->stream>>>(s->d_desc1);
   switch (s->cfg.tsdf_format) {
