@@ -1515,8 +1515,8 @@ __global__ void k_hash_export_voxels(const SessionDesc* __restrict__ descs, uint
 // 64z), triangles in table order.  No weight test: the reference reads sdf alone.
 namespace nui {
 __constant__ uint64_t c_htri[256];
-void hash_mc_upload_tables(cudaStream_t st, const uint64_t* table) {
-  cudaMemcpyToSymbolAsync(c_htri, table, 256 * sizeof(uint64_t), 0, cudaMemcpyHostToDevice, st);
+cudaError_t hash_mc_upload_tables(cudaStream_t st, const uint64_t* table) {
+  return cudaMemcpyToSymbolAsync(c_htri, table, 256 * sizeof(uint64_t), 0, cudaMemcpyHostToDevice, st);
 }
 
 template <int HF>

@@ -29,8 +29,8 @@ namespace nui {
 constexpr int kMcThreads = 256;
 __constant__ uint64_t c_tri[256];
 
-void mc_upload_tables(cudaStream_t st) {
-  cudaMemcpyToSymbolAsync(c_tri, NUI_MC_TRI_PACKED, sizeof(NUI_MC_TRI_PACKED), 0, cudaMemcpyHostToDevice, st);
+cudaError_t mc_upload_tables(cudaStream_t st) {
+  return cudaMemcpyToSymbolAsync(c_tri, NUI_MC_TRI_PACKED, sizeof(NUI_MC_TRI_PACKED), 0, cudaMemcpyHostToDevice, st);
 }
 
 // Bit 0: the voxel has a weight; bit 1: its tsdf is negative.

@@ -2392,7 +2392,7 @@ struct DevBuf {
 };
 }  // namespace
 namespace nui {
-void hash_mc_upload_tables(cudaStream_t st, const uint64_t* table);
+cudaError_t hash_mc_upload_tables(cudaStream_t st, const uint64_t* table);
 template <int F>
 __global__ void k_hash_mesh_count(const SessionDesc*, unsigned*);
 __global__ void k_hash_mesh_scan(const unsigned*, unsigned long long*, int);
@@ -2413,7 +2413,7 @@ nui_status nui_hash_mesh_impl(nui_session* s, float* pos, float* col, uint64_t c
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
   NUI_CUDA(upload_desc1(s, d));
-  if (!s->ctx->hash_mc_tables) hash_mc_upload_tables(st, NUI_MC_TRI_PACKED);
+  if (!s->ctx->hash_mc_tables) NUI_CUDA(hash_mc_upload_tables(st, NUI_MC_TRI_PACKED));
   s->ctx->hash_mc_tables = true;
   DevBuf cnt, off, dp, dc;
   NUI_CUDA(counted_malloc(&cnt.p, (size_t)nvis * 4));
@@ -2446,7 +2446,7 @@ nui_status nui_hash_mesh_impl(nui_session* s, float* pos, float* col, uint64_t c
 }
 }  // namespace
 namespace nui {
-void mc_upload_tables(cudaStream_t st);
+cudaError_t mc_upload_tables(cudaStream_t st);
 template <int F>
 __global__ void k_mc_count(const SessionDesc*, int, unsigned int*, unsigned long long*, uint8_t*);
 __global__ void k_mc_scan(unsigned long long*, int);
@@ -2485,7 +2485,7 @@ nui_status mc_prepare(nui_session* s, DevBuf& cc, DevBuf& bt, uint8_t* d_cases, 
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
   NUI_CUDA(upload_desc1(s, d));
-  if (!s->ctx->mc_tables) mc_upload_tables(st);
+  if (!s->ctx->mc_tables) NUI_CUDA(mc_upload_tables(st));
   s->ctx->mc_tables = true;
   const unsigned nb = mc_blocks(c);
   NUI_CUDA(counted_malloc(&cc.p, sizeof(unsigned) * (size_t)(c.res[0] - 1) * (c.res[1] - 1)));
@@ -2620,7 +2620,7 @@ extern "C" NUI_API nui_status nui_mesh_device_noalloc(nui_session* s, float* d_p
   SessionDesc d;
   fill_desc(s, d, kInactive, nullptr, nullptr);
   NUI_CUDA(upload_desc1(s, d));
-  if (!s->ctx->mc_tables) mc_upload_tables(st);
+  if (!s->ctx->mc_tables) NUI_CUDA(mc_upload_tables(st));
   s->ctx->mc_tables = true;
   switch (c.tsdf_format) {
     case 0: mc_count<0>(s, cc, bt, nullptr); break;
