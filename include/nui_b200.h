@@ -370,12 +370,12 @@ NUI_API nui_status nui_ctx_set_tuning(nui_ctx* ctx, const nui_tuning* t);
 /* Autotuner: creates n scratch sessions of cfgs (device memory for all n at once), runs
  * `frames` frames of each through batch ticks (frame f of session i: depth_mm[i * frames
  * + f], host u16; bgra likewise or NULL), then times every candidate of each parameter in
- * turn (coordinate descent: integration, ICP, dense raycast, hash raycast; parameters no
- * session uses are skipped) as the median device time over `repeats` ticks of the
- * integration stage (integration) or of the whole graphed tick (the others); a setting
- * keeps its current value unless a candidate is at least 2 % faster,
- * keeps the fastest in the context, frees the scratch sessions and reports the choice
- * (out) and the whole-tick median with it (out_tick_ms, nullable).  Takes the context's
+ * turn (coordinate descent: ICP clusters, dense raycast, hash raycast; parameters no
+ * session uses are skipped) as the median device time over `repeats` of the whole graphed
+ * tick; the clusters are timed as clusters also with few enough sessions that a tick of
+ * them alone has none.  A setting keeps its current value unless a candidate is at least
+ * 2 % faster.  Keeps the fastest in the context, frees the scratch sessions and reports the
+ * choice (out) and the whole-tick median with it (out_tick_ms, nullable).  Takes the context's
  * stream for the whole call. */
 NUI_API nui_status nui_ctx_autotune(nui_ctx* ctx, const nui_session_cfg* cfgs, int n,
                                     const uint16_t* const* depth_mm, const uint8_t* const* bgra, int frames,

@@ -1496,7 +1496,13 @@ NUI_API nui_status nui_ctx_autotune(nui_ctx* c, const nui_session_cfg* cfgs, int
   };
   // the ICP shapes and ray tiles by the whole tick: with dense and hash sessions the hash
   // sessions' tracking and raycast run on the second stream, beside stages 2-5
-  tune_one(&nui_tuning::icp_cluster_blocks, {8, 12, 16}, 6);
+  {
+    // up to four sessions would be tracked over the whole device, which has no clusters to size,
+    // while the context may serve many more of these kinds
+    const int wide = c->wide_blocks.exchange(0);
+    tune_one(&nui_tuning::icp_cluster_blocks, {8, 12, 16}, 6);
+    c->wide_blocks = wide;
+  }
   if (dense) tune_one(&nui_tuning::raycast_tile_width, {4, 8, 16, 32}, 6);
   if (hash) tune_one(&nui_tuning::hash_raycast_tile_width, {4, 8, 16, 32}, 6);
   float tick_ms = 0.f;
