@@ -1050,6 +1050,7 @@ nui_status tick_launch(nui_ctx* ctx, nui_session* const* ss, int n, const uint16
   }
   if (floor) plan_merge(p, *floor);
   p.tune = ctx->tune;
+  p.tune.integrate_threads_log2 = p.tune.icp_pixels_per_thread = 0;  // (without effect: one graph whatever they are)
   if ((st = ensure_icp(ctx)) != NUI_OK) return st;
   p.wideBlocks = ctx->wide_blocks;
   icp_fit(ctx, p);
