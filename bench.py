@@ -877,11 +877,14 @@ def run_configs(args):
 
 
 def cpu_baseline_or_reason(args, **kw):
-    """The CPU baseline, or why there is none (the reference's kernels are built from its tree)."""
+    """The CPU baseline, or why its kernels cannot be loaded (they are built from the reference's
+    tree).  What goes wrong in the run itself is raised."""
+    from oracle import oracle
     try:
-        return cpu_baseline(args, **kw)
+        oracle.ref()
     except (RuntimeError, OSError) as e:
-        return {"unavailable": str(e).splitlines()[0]}
+        return {"unavailable": (str(e) or repr(e)).splitlines()[0]}
+    return cpu_baseline(args, **kw)
 
 
 def run_reference(args, rank, world):
