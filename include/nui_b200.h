@@ -241,6 +241,9 @@ NUI_API nui_status nui_debug_allocation_count(uint64_t* n);
  * status is NUI_ERR_DEVICE, the session stays on its last frame, and the context tracks by thread
  * block clusters from then on. */
 NUI_API nui_status nui_debug_stall_icp(nui_ctx* ctx, int polls);
+/* The quotients a[i] / b[i] as the photometric rows form theirs (device pointers), for the test
+ * that compares them with the division. */
+NUI_API nui_status nui_debug_quotients(nui_ctx* ctx, const float* d_a, const float* d_b, float* d_q, int n);
 /* Marching-cubes case index of every cube, (res[0]-1)*(res[1]-1)*(res[2]-1) bytes in the
  * same (y, x, z) order; 0 for cubes skipped because a corner has no weight. */
 NUI_API nui_status nui_mesh_cases(nui_session* s, uint8_t* cases, size_t bytes, uint64_t* nverts);

@@ -101,6 +101,7 @@ _SIGS = {
     "nui_mesh_device_noalloc": (C.c_int, [_P, _P, _P, C.c_uint64, _P]),
     "nui_debug_allocation_count": (C.c_int, [_P]),
     "nui_debug_stall_icp": (C.c_int, [_P, C.c_int]),
+    "nui_debug_quotients": (C.c_int, [_P, _P, _P, _P, C.c_int]),
     "nui_k_color_pyramid": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, _P, _P, _P]),
     "nui_server_create": (C.c_int, [_P, C.c_size_t, C.c_int, _P]),
     "nui_server_destroy": (C.c_int, [_P]),

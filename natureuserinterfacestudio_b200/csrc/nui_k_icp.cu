@@ -41,12 +41,19 @@ __device__ __forceinline__ float3 bilinear_holes(const float4* __restrict__ src,
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): a
 // quotient within one ulp plus its exactly computed remainder times r rounds correctly.  The
 // first remainder step brings a r within one ulp, the second rounds.  Exact while nothing
-// under- or overflows: b in 2^-40 .. 2^40, a zero or in 2^-80 .. 2^80 in magnitude.
+// under- or overflows: b in 2^-40 .. 2^40, a zero or in 2^-80 .. 2^80 in magnitude; a smaller a
+// gives a quotient within two ulps.
 __device__ __forceinline__ float div_shared(float a, float b, float r) {
   float q = a * r;
   q = __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
   return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
 }
+// The quotients of a test.
+__global__ void k_div_shared(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ q, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) q[i] = div_shared(a[i], b[i], 1.0f / b[i]);
+}
+
 // ---------------------------------------------------------------- photometric rows
 // One model point of the colour tracker's term (color_icp_block_kernel, colorIcp.cl:
 // 119-178, in the tracker's convention), at the finest level: the world point m of the
@@ -112,7 +119,8 @@ __device__ __forceinline__ bool color_row(const SessionDesc& s, int i, const flo
     }
   };
   // the twelve quotients by zz share its reciprocal for points between a micrometre and 10^6 m
-  // away along every axis that counts: the numerators are then far inside div_shared's range
+  // away along every axis that counts: the numerators are then below the end of div_shared's range.
+  // One that cancels to less than 2^-80 may end two ulps off (a derivative below 2^-28).
   const float far = fmaxf(fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(m.x), fabsf(m.y))), fmaxf(fabsf(m.z), p.z));
   if (zz > 1e-12f && far < 1e6f) {
     const float rzz = 1.0f / zz;

@@ -39,6 +39,7 @@ __global__ void k_icp_cluster(const SessionDesc*, int, int);
 template <bool COLOR>
 __global__ void k_icp_wide(const SessionDesc*, int, int, IcpWide*, const TrackOut);
 __global__ void k_track_end(const SessionDesc*, int, const TrackOut);
+__global__ void k_div_shared(const float*, const float*, float*, int);
 __global__ void k_open_gate(const SessionDesc*);
 __global__ void k_color_level(const SessionDesc, int);
 __global__ void k_color_grad_one(const SessionDesc);
@@ -1366,6 +1367,14 @@ NUI_API nui_status nui_debug_stall_icp(nui_ctx* c, int polls) {
     NUI_CUDA(cudaMemcpyAsync(&c->d_icp_wide[i].arrived, &missing, sizeof(missing), cudaMemcpyHostToDevice, c->stream));
     NUI_CUDA(cudaMemcpyAsync(&c->d_icp_wide[i].polls, &polls, sizeof(polls), cudaMemcpyHostToDevice, c->stream));
   }
+  NUI_CUDA(cudaStreamSynchronize(c->stream));
+  return NUI_OK;
+}
+
+NUI_API nui_status nui_debug_quotients(nui_ctx* c, const float* d_a, const float* d_b, float* d_q, int n) {
+  if (!c || !d_a || !d_b || !d_q || n <= 0) return fail(NUI_ERR_INVALID_ARG, "bad argument");
+  k_div_shared<<<cdiv(n, 256), 256, 0, c->stream>>>(d_a, d_b, d_q, n);
+  NUI_CUDA(cudaGetLastError());
   NUI_CUDA(cudaStreamSynchronize(c->stream));
   return NUI_OK;
 }

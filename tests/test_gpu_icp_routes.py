@@ -171,3 +171,36 @@ def test_shared_reciprocal_quotient_is_the_division():
         for _ in range(2):
             q = _f32(q + _f32(a - q * b) * r)
         assert q == _f32(a / b), (a, b)
+
+
+def _quotients(ctx, a, b):
+    torch = pytest.importorskip("torch")
+    ta, tb = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    q = torch.empty_like(ta)
+    torch.cuda.synchronize()
+    L.check(L.lib().nui_debug_quotients(ctx.h, ta.data_ptr(), tb.data_ptr(), q.data_ptr(), a.size))
+    return q.cpu().numpy()
+
+
+def _random(rng, n, lo, hi):
+    """Floats of 2^lo .. 2^(hi + 1), a third of them with mantissas at the ends of the binade."""
+    m = rng.integers(1 << 23, 1 << 24, n)
+    k = rng.integers(0, 6, n)
+    m = np.where(k == 0, (1 << 23) + rng.integers(0, 4, n), np.where(k == 1, (1 << 24) - 1 - rng.integers(0, 4, n), m))
+    return np.ldexp(m.astype(np.float64), rng.integers(lo, hi + 1, n) - 23).astype(np.float32)
+
+
+@pytest.mark.gpu
+def test_device_quotients_are_the_division(gpu_ctx):
+    """The rows' quotients over the whole range they claim (numerators of 2^-80 .. 2^80 and zero,
+    denominators of 2^-40 .. 2^40), bit for bit; below it, where a numerator cancels, two ulps."""
+    rng, n = np.random.default_rng(11), 1 << 20
+    b = _random(rng, n, -40, 39)
+    a = _random(rng, n, -80, 79) * rng.choice(np.array([-1, 1], np.float32), n)
+    a[:64] = 0
+    want = (a.astype(np.float64) / b.astype(np.float64)).astype(np.float32)  # (53 bits: no double rounding)
+    assert np.array_equal(_quotients(gpu_ctx, a, b), want)
+    a = _random(rng, n, -126, -81) * rng.choice(np.array([-1, 1], np.float32), n)
+    exact = a.astype(np.float64) / b.astype(np.float64)
+    ulp = np.maximum(np.spacing(np.abs(exact).astype(np.float32)).astype(np.float64), 2.0 ** -149)
+    assert np.max(np.abs(_quotients(gpu_ctx, a, b).astype(np.float64) - exact) / ulp) <= 2.0
