@@ -588,9 +588,9 @@ def ate_vs_plain(L, ctx, seqs, gts, nframes, nstreams):
     dense TSDF / int16 hash, one stream at a time).  Reported per stream: the RMS distance
     between the two trajectories' camera positions, and each one's ATE against the true
     trajectory (RMS position error after both start at the first frame's pose).  The plain
-    path also runs a second time with other ICP launch shapes (8-block clusters, 8 pixels a
-    thread), which change nothing but the FP64 rounding of the ICP sums: the spread between
-    the two plain runs is how far rounding alone moves a trajectory of that stream."""
+    path also runs a second time with all streams in one tick and other ICP launch shapes
+    (8-block clusters): the order of the ICP's sums follows from the image size alone, so the
+    two plain runs are the same trajectories."""
     nseq = len(seqs)
     cfg16 = stream_cfgs(L, nstreams, L.TSDF_F16_U8, L.TSDF_F16_U8)
     cfg32 = stream_cfgs(L, nstreams, L.TSDF_F32, L.TSDF_I16)
@@ -615,14 +615,13 @@ def ate_vs_plain(L, ctx, seqs, gts, nframes, nstreams):
             p32[i, k] = b[i].process(fr[i], co[i])[1][9:]
     for s in a + b:
         s.close()
-    # the plain path again with other ICP launch shapes
-    ctx.set_tuning(L.Tuning(**dict(tune0, icp_cluster_blocks=8, icp_pixels_per_thread=8)))
+    # the plain path again, batched and with other ICP launch shapes
+    ctx.set_tuning(L.Tuning(**dict(tune0, icp_cluster_blocks=8)))
     b = [L.Session(ctx, c) for c in cfg32]
     p32b = np.zeros((nstreams, nframes, 3))
     for k in range(nframes):
-        fr, co = frames(k)
-        for i in range(nstreams):
-            p32b[i, k] = b[i].process(fr[i], co[i])[1][9:]
+        _, poses = ctx.batch_tick(b, *frames(k))
+        p32b[:, k] = poses[:, 9:]
     for s in b:
         s.close()
     ctx.set_tuning(L.Tuning(**tune0))
@@ -932,8 +931,9 @@ def main():
     ap.add_argument("--config-cpu-frames", dest="config_cpu_frames", type=int, default=4)
     ap.add_argument("--room-frames", dest="room_frames", type=int, default=300)
     ap.add_argument("--tuning", default="",
-                    help="launch shapes to use instead of autotuning: integration threads log2, ICP pixels "
-                         "per thread, dense and hash ray tile widths, ICP blocks per session (e.g. 16,8,8,4,8)")
+                    help="launch shapes to use instead of autotuning: integration threads log2 and ICP pixels per "
+                         "thread (both without effect), dense and hash ray tile widths, ICP blocks per session "
+                         "(e.g. 18,4,8,4,8)")
     args = ap.parse_args()
     args.warmup = max(3, args.warmup)
     if args.configs:

@@ -440,7 +440,7 @@ NUI_API nui_status nui_session_work_counters(nui_session* s, uint64_t* out);
 
 /* ---------------------------------------------------------------- kernel-level calls
  * One entry point per reference kernel launch on the hot path, on device pointers,
- * launched on the context's stream (asynchronous).  Vertex/normal maps are float4 per
+ * run on the context's stream and complete when the call returns.  Vertex/normal maps are float4 per
  * pixel (xyz, w = 0); depth maps float; volumes in the session layout are reached
  * through sessions only. */
 /* depth_passing_filter_kernel + bilateral_filter_depth_kernel + depth2vertex_kernel +

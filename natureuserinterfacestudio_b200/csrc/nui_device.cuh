@@ -69,9 +69,9 @@ struct TrackState {
   unsigned int fast_count, fast_done;
 };
 
-// The tracker state the host step reads and writes: kept in block 0's shared memory for
-// the whole ICP kernel (so that the single thread's step makes no global-memory round
-// trips), copied in at the start and back at the end.
+// The tracker state the host step reads and writes: kept in shared memory for the whole ICP kernel
+// (so that the step makes no global-memory round trips), of a cluster's first block or of every
+// block of k_icp_wide, copied in at the start and back at the end by the first.
 struct IcpLm {
   float R[9], t[3], Rg[9], tg[3];
   double good[27];

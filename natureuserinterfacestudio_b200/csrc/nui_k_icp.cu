@@ -1,14 +1,14 @@
-// Point-to-plane ICP: every iteration of every level in one launch, one thread-block
-// cluster per session, no host round trip.
+// Point-to-plane ICP: every iteration of every level in one launch, no host round trip; up to four
+// sessions over the whole device (k_icp_wide), more by a thread-block cluster each (k_icp_cluster).
 //
 // Per pixel (icp_block_kernel, icp.cl:222-292): rebuild the level's vertex from its depth,
 // transform it by the running estimate, project into the previous camera with
 // full-resolution intrinsics, bilinearly sample the world reference normal and vertex
 // (icp.cl:192-220; a tap NaN -> no match), and if |q - p| < distThres form the row
 // [n x p, n | n.(q - p)].  A warp adds the outer products of its pixels' rows in FP64 on the
-// tensor path (exact products of the FP32 row values); blocks add their warps' sums, the
-// cluster's first block the blocks' (distributed shared memory, fixed order), and it runs the
-// host step of
+// tensor path (exact products of the FP32 row values), and the warps' sums are joined in an
+// order that the image size fixes, by every block of k_icp_wide or the first of a cluster, which
+// run the host step of
 // NuiKinfuOpenCLDepthTracker::IterativeClosestPoint (NuiKinfuOpenCLDepthTracker.cpp:324-496):
 // Levenberg-Marquardt accept/reject, FP64 determinant check and Cholesky solve, ZYX Euler
 // increment composed in FP64.  The next iteration reads the updated estimate.
@@ -934,9 +934,10 @@ __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
 // What bounds it is latency: an iteration is a pass of a few us, a trip through L2 and the LM
 // step.  A cluster is at most 16 SMs, on which a pass of a colour-tracked 640 x 480 level takes
 // 120 us; a launch an iteration costs 2 us even after the level has ended (a level that starts
-// close to its end runs one iteration of the ten).  At 640 x 480 a depth iteration takes 12 us
-// (pass 3.3, waiting 1.0, sums 1.5, LM step 3.9; 7 us at the coarser levels) and a photometric
-// one 20.
+// close to its end runs one iteration of the ten).  A 640 x 480 depth session's iterations, over
+// its levels and on 72 SMs, take 12.4 us (pass and unit sums 5.1, arriving and waiting 2.0, the
+// image's sums 1.0, LM step 4.3; on 143 the pass is 3.9), with photometric rows 16.1 (pass 3.7,
+// those and the wait 6.9).
 template <bool COLOR>
 __global__ void __launch_bounds__(COLOR ? 512 : 1024, 1)
     k_icp_wide(const SessionDesc* __restrict__ descs, int fam, int room, IcpWide* __restrict__ work, const TrackOut out) {

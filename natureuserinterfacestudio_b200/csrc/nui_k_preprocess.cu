@@ -25,15 +25,12 @@ constexpr int kPreSW = kPreTX + 2 * kMaxRadius, kPreSH = kPreTY + 2 * kMaxRadius
 // The bilateral sum of one pixel: taps in row-major window order, each weighted by its
 // spatial weight times exp(-diff^2 sigma) when it is positive and within the depth
 // threshold of the centre c (NaN taps fail both tests).  t points at the window's corner
-// in the staged tile, g at the spatial weights.  KR > 0 unrolls a window of that radius;
-// FAST takes nui_expf_neg, valid when thr^2 sigma <= 87.
-template <int KR, bool FAST>
+// in the staged tile, g at the spatial weights.  FAST takes nui_expf_neg, valid when
+// thr^2 sigma <= 87.
+template <bool FAST>
 __device__ __forceinline__ float bilateral_px(const float* t, const float* g, int R, float c, float thr, float sig) {
-  if (KR > 0) R = KR;
   float sd = 0.f, swt = 0.f;
-#pragma unroll
   for (int dy = 0; dy <= 2 * R; ++dy) {
-#pragma unroll
     for (int dx = 0; dx <= 2 * R; ++dx) {
       const float nr = t[dy * kPreSW + dx];
       const float diff = fabsf(c - nr);
@@ -72,8 +69,9 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
   return r;
 }
-// A product that an addition follows: the assembler joins a packed multiply and a packed add
-// into one fused operation whatever their rounding qualifiers, a scalar multiply it leaves.
+// A product that an addition follows, by scalar multiplications: with a packed one the sums had the
+// bits of a single rounding of product and addition, and the filtered depths were not the
+// reference's (tests/test_gpu_preprocess_edges.py).
 __device__ __forceinline__ F2 mul2_apart(F2 a, F2 b) {
   float a0, a1, b0, b1;
   unpack2(a, a0, a1);
@@ -222,8 +220,8 @@ __device__ __forceinline__ void preprocess_block(const SessionDesc& s) {
     for (int k = 0; k < 2; ++k) {
       if (isnan(cs[k])) continue;
       const float* t = &tile[ly0 + k][threadIdx.x];
-      if (fast) outs[k] = bilateral_px<0, true>(t, &gw[0][0], R, cs[k], thr, sig);
-      else outs[k] = bilateral_px<0, false>(t, &gw[0][0], R, cs[k], thr, sig);
+      if (fast) outs[k] = bilateral_px<true>(t, &gw[0][0], R, cs[k], thr, sig);
+      else outs[k] = bilateral_px<false>(t, &gw[0][0], R, cs[k], thr, sig);
     }
   }
   float m = 0.f;  // largest ray-length depth of this thread's two pixels

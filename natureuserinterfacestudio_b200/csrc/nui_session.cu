@@ -5,8 +5,9 @@
 // One frame of a session (NuiKinfuTrackingEngine::RunTracking, NuiKinfuTrackingEngine.cpp:68-142)
 // is this fixed sequence of launches, each covering every session of the batch
 // (blockIdx.y = session):
-//   k_preprocess, k_pyramid x (levels-1), k_feedback, k_icp x sum(iterations),
-//   k_track_end, k_integrate<fmt>, k_raycast<fmt>
+//   k_preprocess, k_pyramid x (levels-1), k_feedback, the ICP (k_icp_wide, or k_icp_cluster and
+//   k_track_end), k_integrate<fmt> (the FP16 formats: k_integrate_cull, k_integrate_fast), the
+//   brick summaries and distances, k_raycast<fmt> and its refinement
 // Which session does what in a tick (first frame / tracking / inactive) is data in the
 // session table, so the same sequence serves every tick and is captured once.
 #include <cuda_runtime.h>
